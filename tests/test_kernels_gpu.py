@@ -320,6 +320,45 @@ def test_paged_attention_generic(dtype, nh, nkv, d, ps, window):
     assert rel_err(got, want) < 5e-2, "the far key that stands out was not seen"
 
 
+@pytest.mark.parametrize("nh,nkv,d,dv,window,keep", [(8, 4, 128, 128, None, 0), (3, 3, 4, 12, None, 0), (12, 2, 64, 64, 40, 0),
+                                                     (16, 1, 32, 32, 33, 5), (32, 1, 20, 128, None, 0), (24, 8, 100, 60, 7, 70)])
+def test_paged_attention_float32_tiles(nh, nkv, d, dv, window, keep):
+    """The form for 32-bit heads of a multiple of four numbers: tiles over several requests, single tokens by
+    themselves, groups of 1 to 32 heads, and the same bits for a token whichever way its step was cut.  A product of two
+    sums of n terms: within n 2^-23 of the largest value."""
+    from inferrs_b200 import kernels as K
+    ps, lens, new = 16, [300, 17, 64, 1, 129], [40, 17, 1, 1, 33]
+    table, positions, row_request, k_pages, v_pages = _paged_setup(torch.float32, nkv, max(d, dv), ps, lens, new, 20)
+    k_pages, v_pages = k_pages[..., :d].contiguous(), v_pages[..., :dv].contiguous()
+    n = sum(new)
+    q = rand((n, nh, d), torch.float32, 23)
+    opt = dict(keep_first=keep, sinks=rand((nh,), torch.float32, 24), cap=9.0) if keep else {}
+    out = torch.full((n, nh * dv), float("nan"), device=dev())
+    K.paged_attention_generic(q, k_pages, v_pages, table, row_request, positions, d ** -0.5, window, out, **opt)
+    dq, dk, dvv = q.double().cpu(), k_pages.double().cpu(), v_pages.double().cpu()
+    R_out = torch.empty((n, nh * dv), dtype=torch.float64)
+    for r in range(n):
+        pos, req = int(positions[r]), int(row_request[r])
+        lo = max(0, pos - window + 1) if window else 0
+        js = [j for j in range(pos + 1) if j >= lo or j < keep]
+        pages, slots = table[req, [j // ps for j in js]].cpu().long(), torch.tensor([j % ps for j in js])
+        for h in range(nh):
+            kv = h // (nh // nkv)
+            s = dk[pages, kv, slots] @ dq[r, h] * d ** -0.5
+            if keep:
+                s = torch.cat([9.0 * torch.tanh(s / 9.0), opt["sinks"][h:h + 1].double().cpu()])
+            p = torch.softmax(s, 0)[:len(js)]
+            R_out[r, h * dv:(h + 1) * dv] = p @ dvv[pages, kv, slots]
+    err = (out.double().cpu() - R_out).abs().max().item()
+    assert err <= (max(lens) + d) * 2.0 ** -23 * float(v_pages.abs().max())
+    one = torch.full((n, nh * dv), float("nan"), device=dev())
+    for r in range(n):                                  # every token in a step of its own
+        req = int(row_request[r])
+        K.paged_attention_generic(q[r:r + 1], k_pages, v_pages, table[req:req + 1], torch.zeros_like(row_request[:1]),
+                                  positions[r:r + 1], d ** -0.5, window, one[r:r + 1], **opt)
+    assert torch.equal(one, out)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n,m,k", [(70, 130, 100), (1, 517, 96), (64, 64, 16), (129, 65, 33)])
 def test_gemm_tn_simt(dtype, n, m, k):
@@ -344,6 +383,38 @@ def test_gemm_rows_do_not_depend_on_the_batch():
     one = torch.empty((1, 200), dtype=torch.float32, device=dev())
     K.gemm_tn_simt(x[77:78].contiguous(), w, one, torch.float32)
     assert torch.equal(one[0], full[77])
+
+
+@pytest.mark.parametrize("m,k", [(33, 4), (1030, 260), (2100, 1156), (32800, 132)])
+def test_gemm_rows_are_one_chain_in_every_kernel(m, k):
+    """Every number of rows gives the bits of a row alone: the kernels for few rows at each of their row limits and
+    numbers of features (below 2,048, below 32,768, above), both tiles, and the form for rows that do not start on 16 bytes.
+    Against 64 bits a chain of k fused multiply-adds is off by at most k 2^-24 sum |x w|."""
+    from inferrs_b200 import kernels as K
+    x, w = rand((130, k), torch.float32, 42), rand((m, k), torch.float32, 43)
+    want = x.double() @ w.double().t()
+    bound = k * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    first = None
+    for n in (130, 1, 4, 5, 8, 9, 16, 17, 32, 33, 64, 65):
+        out = torch.full((n, m), float("nan"), device=dev())
+        K.gemm_tn_simt(x[:n], w, out, torch.float32)
+        assert bool(((out.double() - want[:n]).abs() <= bound[:n]).all())
+        first = out if first is None else first
+        assert torch.equal(out, first[:n]), n
+    odd = torch.empty(130 * k + 1, device=dev())[1:].view(130, k).copy_(x)       # starts on 4 bytes only
+    out = torch.full((130, m), float("nan"), device=dev())
+    K.gemm_tn_simt(odd, w, out, torch.float32)
+    assert torch.equal(out, first)
+
+
+def test_gemm_batched_float32_strides():
+    from inferrs_b200 import kernels as K
+    for n in (3, 40):
+        x, w = rand((n, 4 * 36), torch.float32, 44), rand((4, 50, 36), torch.float32, 45)
+        out = torch.empty((n, 4 * 50), device=dev())
+        K.batched_linear(x.view(n, 4, 36).transpose(0, 1), w, out.view(n, 4, 50).transpose(0, 1), torch.float32)
+        want = torch.einsum("nbk,bmk->nbm", x.double().view(n, 4, 36), w.double()).reshape(n, 200)
+        assert rel_err(out, want) < 36 * 2.0 ** -24 * 4
 
 
 def test_gemm_bf16_library():
