@@ -41,8 +41,8 @@ _SIGNATURES = {
                               c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                               c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
     "ib_paged_attention_generic": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
-                                   c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_void_p, c_int,
-                                   *_SCORE_OPTIONS, c_void_p],
+                                   c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_int, c_void_p,
+                                   c_int, *_SCORE_OPTIONS, c_void_p],
     "ib_gemm_tn_simt": [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_long, c_long,
                         c_long, c_void_p],
     "ib_paged_attention_mma": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
@@ -845,7 +845,8 @@ def paged_attention_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: tor
                           f"joint queries)")
     _check(_core(act).ib_paged_attention_generic(
         _p(q), _p(k_pages), _p(v_pages), _p(block_table), block_table.shape[1], page_size, n_pages, _p(row_request),
-        _p(positions), n, nh, nkv, d, dv, float(scale), int(window) if window else 0, _p(out), int(bool(joint)),
+        _p(positions), n, block_table.shape[0], nh, nkv, d, dv, float(scale), int(window) if window else 0, _p(out),
+        int(bool(joint)),
         _p(dist_bias), 0 if dist_bias is None else dist_bias.shape[1], *opt.args(), out_ld, _stream()),
         "paged_attention_generic")
 
