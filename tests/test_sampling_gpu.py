@@ -75,6 +75,60 @@ def test_a_row_shared_by_one_to_eight_ctas_gives_the_same_token(vocab):
         K.sample(logits, temperature, top_k, top_p, min_p, uniform, got, cluster=3)
 
 
+@pytest.mark.parametrize("vocab", [7, 514, 2047, 32001])
+def test_top_k_over_two_passes(vocab):
+    """The kernel for rows with top-k: its largest k and the one beyond, k of one and of nearly the vocabulary, ties around
+    the k-th place (few: all gathered; more than its list holds: the general kernel's), infinities and NaN among the
+    logits, rows that do not start on 16 bytes, one to eight CTAs a row."""
+    import kernel_refs as R
+    from inferrs_b200 import kernels as K
+    rows = 12
+    logits = _logits(rows, vocab, seed=29)
+    logits[1] = (logits[1] * 2).round() / 2                     # many equal values
+    logits[2] = (logits[2] * 64).round() / 64                   # a few
+    logits[3, ::3] = float("-inf")
+    logits[4, 1::2] = float("nan")
+    logits[5] = float("-inf")
+    logits[5, vocab // 2] = -3.0                                # one candidate, fewer than k
+    logits = logits.cuda()
+    temperature = torch.tensor([0.7] * 10 + [0.0, 1.7]).cuda()
+    top_k = torch.tensor([1, 40, 40, 50, 30, 20, 512, 513, max(1, vocab - 1), 2, 5, 64], dtype=torch.int32).cuda()
+    top_p = torch.tensor([0.9, 1.0, 0.8, 0.9, 0.95, 0.9, 1.0, 0.7, 1.0, 0.01, 0.9, 0.5]).cuda()
+    min_p = torch.tensor([0.0] * 8 + [0.05, 0.0, 0.0, 0.3]).cuda()
+    clean = [r for r in range(rows) if r != 4]                  # the plain statement sorts no NaN
+    odd = torch.empty(rows * vocab + 1, device="cuda")[1:].view(rows, vocab).copy_(logits)
+    for draw in (0.0, 0.37, 0.85, 0.999999):
+        uniform = torch.full((rows,), draw).cuda()
+        want = torch.empty(rows, dtype=torch.int32, device="cuda")
+        R.sample(logits[clean], temperature[clean], top_k[clean], top_p[clean], min_p[clean], uniform[clean], want[:rows - 1])
+        first = None
+        for cluster in (1, 2, 4, 8, 0):
+            for x in (logits, odd):
+                got = torch.full((rows,), -5, dtype=torch.int32, device="cuda")
+                K.sample(x, temperature, top_k, top_p, min_p, uniform, got, cluster=cluster)
+                assert [got.tolist()[r] for r in clean] == want[:rows - 1].tolist(), (cluster, draw)
+                first = got.tolist() if first is None else first
+                assert got.tolist() == first
+        assert first[4] % 2 == 0                                # never a NaN
+
+
+def test_penalties_of_long_windows():
+    """A window longer than the kernel keeps in shared memory, and one just within it."""
+    from inferrs_b200 import kernels as K
+    for n in (4096, 4099):
+        prev = torch.randint(0, 700, (2, n), generator=torch.Generator().manual_seed(n), dtype=torch.int32).cuda()
+        n_prev = torch.tensor([n, n - 3], dtype=torch.int32).cuda()
+        one, logits = torch.ones(2).cuda(), _logits(2, 1000, seed=3).cuda()
+        want = logits.clone()
+        K.penalties(logits, prev, n_prev, one * 1.2, one * 0.01, one * 0.3)
+        for r in range(2):
+            seen, count = prev[r, :n_prev[r]].long().unique(return_counts=True)
+            v = want[r, seen]
+            want[r, seen] = torch.where(v >= 0, v / 1.2, v * 1.2) - 0.01 * count - 0.3
+        # four roundings of 32 bits on values below 64
+        assert (logits - want).abs().max().item() < 4 * 2.0 ** -24 * 64
+
+
 def test_penalties_and_mixed_rows():
     from inferrs_b200.sampling.sampler import Sampler
     vocab, rows = 2000, 6
