@@ -67,6 +67,8 @@ def host_library():
         i, p, l = ctypes.c_int, ctypes.c_void_p, ctypes.c_int64
         lib.ibh_cache_new.argtypes = [i, p, p, p, i, i]
         lib.ibh_cache_new.restype = p
+        lib.ibh_uniforms.argtypes = [p, p, i, p]
+        lib.ibh_uniforms.restype = None
         lib.ibh_cache_delete.argtypes = [p]
         lib.ibh_cache_delete.restype = None
         lib.ibh_sched_new.argtypes = [p, i, i, i, i, p, i]

@@ -228,6 +228,27 @@ struct Cache {
 
 #define IBH_EXPORT extern "C" __attribute__((visibility("default")))
 
+// The random number in [0, 1) of a request's seed and step for n requests: the reference's stateless generator
+// (inferrs/src/sampler.rs:370-397), 64-bit arithmetic that wraps around.
+static inline uint64_t splitmix(uint64_t x) {
+    x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
+    x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
+    return x ^ (x >> 31);
+}
+
+IBH_EXPORT void ibh_uniforms(const uint64_t* seeds, const uint64_t* steps, int n, float* out) {
+    const uint64_t golden = 0x9E3779B97F4A7C15ull;
+    for (int i = 0; i < n; ++i) {
+        uint64_t x = splitmix(seeds[i] + golden);
+        x = splitmix(x + (steps[i] + 1) * golden);
+        if (x == 0) x = 0x1234567890ABCDEFull;
+        x ^= x << 13;
+        x ^= x >> 7;
+        x ^= x << 17;
+        out[i] = (float)((double)((x * 0x2545F4914F6CDD1Dull) >> 32) / 4294967296.0);
+    }
+}
+
 // windows[g] < 0: group g keeps all keys; keeps[g] of a sequence's first keys stay visible beside a window.  Returns
 // nullptr for sizes that make no sense.
 IBH_EXPORT void* ibh_cache_new(int n_groups, const int* windows, const int* keeps, const int* n_pages, int page_size,

@@ -6,7 +6,8 @@ to the host is one token id per row.
 """
 from __future__ import annotations
 
-from typing import List, Sequence
+from array import array
+from typing import Sequence
 
 import numpy as np
 import torch
@@ -75,37 +76,55 @@ class Sampler:
         pend = [int(pending)] * r if isinstance(pending, int) else [int(x) for x in pending]
         if len(pend) != r or any(x not in (0, 1) for x in pend):
             raise ValueError("pending: 0 or 1, one for all rows or one per row")
-        length = [(h.n_tokens if hasattr(h, "n_tokens") else len(h)) + x for h, x in zip(histories, pend)]
-        penalised = [p.has_penalty for p in params]
+        length = [h.n_tokens if hasattr(h, "n_tokens") else len(h) for h in histories]
+        if any(pend):
+            length = [n + x for n, x in zip(length, pend)]
+        # rows that share an options object share its numbers (looked up within this call only)
+        options, kinds = {}, []
+        for p in params:
+            if id(p) not in options:
+                on = p.has_penalty
+                options[id(p)] = (len(options), p.repeat_last_n if on else 0,
+                                  (p.temperature, p.top_p, p.min_p, p.repetition_penalty if on else 1.0,
+                                   p.frequency_penalty if on else 0.0, p.presence_penalty if on else 0.0), p.top_k)
+            kinds.append(options[id(p)])
         width = 0
-        if any(penalised):
+        if any(last for _, last, _, _ in options.values()):
             if any(pend) and pending_ids is None and pending_from is None:
                 raise ValueError("penalties need the whole history: the one pending token must be given on the device")
-            width = max(1, max(min(p.repeat_last_n, n) if on else 0 for p, n, on in zip(params, length, penalised)))
+            width = max(1, max(min(k[1], n) for k, n in zip(kinds, length)))
         # the block: seven rows of floats (as their bits), two of ints, the penalties' windows, the pending tokens' places
         look_up = width > 0 and any(pend) and pending_ids is None
         words = np.empty((9 * r + r * width + (r if look_up else 0),), dtype=np.int32)
         floats = words[:7 * r].view(np.float32).reshape(7, r)
-        floats[0] = [p.temperature for p in params]
-        floats[1] = [p.top_p for p in params]
-        floats[2] = [p.min_p for p in params]
+        rows = list(options.values())
+        which = [k[0] for k in kinds] if len(rows) > 1 else 0
+        numbers = np.array([k[2] for k in rows], dtype=np.float32).T
+        floats[:3] = numbers[:3, which].reshape(3, -1)
         floats[3] = uniforms_for(seeds, length)
-        floats[4] = [p.repetition_penalty if on else 1.0 for p, on in zip(params, penalised)]
-        floats[5] = [p.frequency_penalty if on else 0.0 for p, on in zip(params, penalised)]
-        floats[6] = [p.presence_penalty if on else 0.0 for p, on in zip(params, penalised)]
-        words[7 * r:8 * r] = [p.top_k for p in params]
+        floats[4:] = numbers[3:, which].reshape(3, -1)
+        words[7 * r:8 * r] = np.array([k[3] for k in rows], dtype=np.int32)[which]
         n_prev = words[8 * r:9 * r]
         n_prev[:] = 0
         if width:
-            prev = words[9 * r:9 * r + r * width].reshape(r, width)
-            prev[:] = -1
-            for i, (p, h) in enumerate(zip(params, histories)):
-                if penalised[i]:
-                    # the window's order does not matter: the pending token, if any, takes the first place
-                    known = p.repeat_last_n - pend[i]
-                    tail = (h.tail(known) if hasattr(h, "tail") else list(h[-known:])) if known > 0 else []
-                    prev[i, pend[i]:pend[i] + len(tail)] = tail
-                    n_prev[i] = len(tail) + pend[i]
+            # the windows, row by row: -1 in the place of the pending token, the history's tail, -1 up to the width.  The
+            # window's order does not matter: the pending token, if any, takes the first place.
+            windows, counts, blank = array("i"), [], array("i", [-1]) * width
+            for k, h, x in zip(kinds, histories, pend):
+                known, n = k[1] - x, 0
+                if k[1]:
+                    if x:
+                        windows.append(-1)
+                    if known > 0:
+                        tail = h.tail(known) if hasattr(h, "tail") else h[-known:]
+                        windows.fromlist(tail if isinstance(tail, list) else list(tail))
+                        n = len(tail)
+                    n += x
+                counts.append(n)
+                if n < width:
+                    windows.extend(blank[:width - n])
+            words[9 * r:9 * r + r * width] = np.frombuffer(windows, dtype=np.int32)
+            n_prev[:] = counts
         if look_up:
             words[9 * r + r * width:] = list(pending_from[1])
         dev = self._upload(words)

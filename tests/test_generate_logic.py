@@ -30,6 +30,15 @@ def test_uniform_matches_the_plain_generator():
         assert abs(uniform_for(seed, step) - float(plain_sampler.rand_f32(seed, step))) < 1e-7
 
 
+def test_uniforms_of_many_rows_have_the_same_bits():
+    import numpy as np
+    from inferrs_b200.sampling.params import uniforms_for
+    seeds = [0, 4, 2 ** 63 - 1, 2 ** 64 - 1, 2 ** 70 + 5, -1, -12345] + random_tokens(50, 10 ** 9, seed=3)
+    steps = [0, 17, 5000, 1, 2 ** 31, 7, 0] + random_tokens(50, 10 ** 5, seed=4)
+    want = np.array([uniform_for(a, b) for a, b in zip(seeds, steps)], dtype=np.float32)
+    assert np.array_equal(uniforms_for(seeds, steps), want) and uniforms_for([], []).shape == (0,)
+
+
 @pytest.mark.parametrize("name", ["A", "B"])
 def test_greedy_generation(model_dirs, monkeypatch, name):
     kernel_refs.install(monkeypatch)
