@@ -3,11 +3,10 @@
 // The work of one CTA is one key/value head of one request and one slice of its keys.  A producer warp
 // brings the slice's keys and values page by page with TMA into a ring of 128-byte-swizzled 64-key tiles
 // (no address arithmetic in the compute warps); four compute warps take 16 keys each of every tile:
-// scores with mma.sync (the G query heads of the group are the rows of a 16-row tile), online softmax in
-// float32, P V with mma.sync.  The warps' partial results are merged through shared memory, and the
-// slices' results through float32 scratch: every CTA adds one to a counter of its (request, head group),
-// and the CTA that finds it was the last one merges all slices and writes the output, so no second
-// kernel is needed.  How many slices are used is decided from the request's real length (at least `min_tiles`
+// scores with mma.sync, online softmax in float32, P V with mma.sync (see Share).  The warps' partial results
+// are merged through shared memory, and the slices' results through float32 scratch: every CTA adds one to
+// a counter of its (request, head group), and the CTA that finds it was the last one merges all slices and
+// writes the output, so no second kernel is needed.  How many slices are used is decided from the request's real length (at least `min_tiles`
 // tiles per slice); CTAs of unused slices leave at once.
 #include <cuda.h>
 
@@ -47,6 +46,12 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const unsigned (&a)[4], 
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// a transposed 8 x 8 matrix of 16-bit numbers (a lane: row lane / 4, columns 2 (lane % 4) and the next)
+__device__ __forceinline__ unsigned movmatrix(unsigned a) {
+    unsigned d;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+    return d;
+}
 // byte offset of 16-byte chunk c (0..15 over the 128 dims) of key row `row` in a tile of two swizzled halves
 __device__ __forceinline__ unsigned tile_off(int row, int c) {
     return (unsigned)((c >> 3) * HALF_BYTES + row * 128 + (((c & 7) ^ (row & 7)) << 4));
@@ -69,9 +74,276 @@ struct Params {
     IbScoreOptions opt;
 };
 
+// One warp's share of a row: 16 keys of every tile against the group's query heads; scores, softmax in float32, values.
+//
+// Up to eight heads (FEW): keys are the products' 16 rows and the heads their eight columns (S^T = K Q^T, O^T = V^T P^T), so
+// that no row of a product is padding; the probabilities are turned round by movmatrix between the two.  Against the form
+// below, half the products, half the accumulators and, where no maximum moves, no rescaling: a warp's tile takes
+// about half the instructions, which with its dependent steps is what a CTA's pace is bound by.
+template <bool OPTIONS, bool FEW>
+struct Share {
+    float o[D / 16][4];                     // [16 dimensions: gid, gid + 8][heads 2 tig, 2 tig + 1]
+    float m[2], l[2];                       // of heads 2 tig and 2 tig + 1 (l: of this lane's keys until close())
+    unsigned qf[D / 16][2];
+    float scale[2], slope[2];
+
+    __device__ __forceinline__ static int head(int lane, int h) { return 2 * (lane & 3) + h; }
+
+    // `sq`: [8 or more heads][128], zeros behind the group's
+    __device__ __forceinline__ void begin(const __nv_bfloat16* sq, int lane, const Params& P, int head0, int G) {
+#pragma unroll
+        for (int n = 0; n < D / 16; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.0f;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ks += 2)
+            ldmatrix_x4(qf[ks][0], qf[ks][1], qf[ks + 1][0], qf[ks + 1][1],
+                        smem_u32(sq + (lane & 7) * D + (2 * ks + (lane >> 3)) * 8));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            m[h] = -INFINITY;
+            l[h] = 0.0f;
+            scale[h] = P.scale_log2;
+            slope[h] = 0.0f;
+            if (OPTIONS && head(lane, h) < G) {
+                if (P.opt.head_scale) scale[h] *= P.opt.head_scale[head0 + head(lane, h)];
+                if (P.opt.slopes) slope[h] = P.opt.slopes[head0 + head(lane, h)] * P.slope_factor;
+            }
+        }
+    }
+
+    __device__ __forceinline__ void step(unsigned tk, unsigned tv, int warp, int lane, int tile_key, int lo, int pos, int keep,
+                                         const Params& P, int G) {
+        const int key0 = warp * 16, gid = lane >> 2;
+        float sc[2][4];                     // two chains of products, added below
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sc[0][e] = sc[1][e] = 0.0f;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+            unsigned a[4];
+            ldmatrix_x4(a[0], a[1], a[2], a[3], tk + tile_off(key0 + (lane & 15), 2 * ks + (lane >> 4)));
+            mma16816(sc[ks & 1], a, qf[ks][0], qf[ks][1]);
+        }
+        float top[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {       // key gid + 8 (e >> 1), head 2 tig + (e & 1)
+            const int j = tile_key + key0 + gid + 8 * (e >> 1);
+            float x = (sc[0][e] + sc[1][e]) * scale[e & 1];
+            if (OPTIONS) {
+                x -= slope[e & 1] * (float)(pos - j);
+                if (P.opt.cap > 0.0f) x = ib_capped_log2(x, P.cap_c);
+            }
+            sc[0][e] = ib_visible(j, lo, pos, keep) ? x : -INFINITY;
+            top[e & 1] = fmaxf(top[e & 1], sc[0][e]);
+        }
+        float corr[2], safe[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int w = 4; w < 32; w <<= 1) top[h] = fmaxf(top[h], __shfl_xor_sync(0xffffffffu, top[h], w));
+            const float m_new = fmaxf(m[h], top[h]);
+            safe[h] = m_new == -INFINITY ? 0.0f : m_new;
+            corr[h] = m[h] == -INFINITY ? 0.0f : exp2f(m[h] - safe[h]);
+            m[h] = m_new;
+        }
+        if (__any_sync(0xffffffffu, corr[0] != 1.0f || corr[1] != 1.0f)) {
+            l[0] *= corr[0];
+            l[1] *= corr[1];
+#pragma unroll
+            for (int n = 0; n < D / 16; ++n) {
+                o[n][0] *= corr[0]; o[n][1] *= corr[1];
+                o[n][2] *= corr[0]; o[n][3] *= corr[1];
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            sc[0][e] = exp2f(sc[0][e] - safe[e & 1]);
+            l[e & 1] += sc[0][e];
+        }
+        const unsigned b0 = movmatrix(pack_bf16(sc[0][0], sc[0][1])), b1 = movmatrix(pack_bf16(sc[0][2], sc[0][3]));
+#pragma unroll
+        for (int n = 0; n < D / 16; ++n) {
+            unsigned a[4];
+            ldmatrix_x4_trans(a[0], a[1], a[2], a[3],
+                              tv + tile_off(key0 + (lane & 7) + 8 * (lane >> 4), 2 * n + ((lane >> 3) & 1)));
+            mma16816(o[n], a, b0, b1);
+        }
+    }
+
+    __device__ __forceinline__ void close(int lane, int warp, int G, float* sm, float* sl) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int w = 4; w < 32; w <<= 1) l[h] += __shfl_xor_sync(0xffffffffu, l[h], w);
+            if (lane < 4 && head(lane, h) < G) { sm[warp * 16 + head(lane, h)] = m[h]; sl[warp * 16 + head(lane, h)] = l[h]; }
+        }
+    }
+
+    // dimensions d0 .. d0 + dims - 1 of every head to `so`, a head's row ld numbers behind the one before it
+    __device__ __forceinline__ void put(float* so, int ld, int d0, int dims, int lane, int G) const {
+#pragma unroll
+        for (int n = 0; n < D / 16; ++n)
+            if (n * 16 >= d0 && n * 16 < d0 + dims)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (head(lane, e & 1) < G) so[head(lane, e & 1) * ld + n * 16 - d0 + (lane >> 2) + 8 * (e >> 1)] = o[n][e];
+    }
+};
+
+// Up to sixteen heads: they are the products' rows (gid and gid + 8 of this lane).
+template <bool OPTIONS>
+struct Share<OPTIONS, false> {
+    float o[D / 8][4], m_r[2], l_r[2], scale_r[2], slope_r[2];
+    unsigned qf[D / 16][4];
+
+    __device__ __forceinline__ void begin(const __nv_bfloat16* sq, int lane, const Params& P, int head0, int G) {
+#pragma unroll
+        for (int n = 0; n < D / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.0f;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+            const int r = (lane & 7) + 8 * ((lane >> 3) & 1), c = 2 * ks + (lane >> 4);
+            ldmatrix_x4(qf[ks][0], qf[ks][1], qf[ks][2], qf[ks][3], smem_u32(sq + r * D + c * 8));
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int head = (lane >> 2) + 8 * h;
+            m_r[h] = -INFINITY;
+            l_r[h] = 0.0f;
+            scale_r[h] = P.scale_log2;
+            slope_r[h] = 0.0f;
+            if (OPTIONS && head < G) {
+                if (P.opt.head_scale) scale_r[h] *= P.opt.head_scale[head0 + head];
+                if (P.opt.slopes) slope_r[h] = P.opt.slopes[head0 + head] * P.slope_factor;
+            }
+        }
+    }
+
+    __device__ __forceinline__ void step(unsigned tk, unsigned tv, int warp, int lane, int tile_key, int lo, int pos, int keep,
+                                         const Params& P, int G) {
+        const int tig = lane & 3;
+        const bool row_ok[2] = {(lane >> 2) < G, (lane >> 2) + 8 < G};
+        const int key0 = warp * 16;                      // this warp's 16 keys of the tile
+        float sc[2][4];
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sc[n][e] = 0.0f;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+            unsigned b0, b1, b2, b3;
+            const int kr = key0 + (lane & 7) + 8 * (lane >> 4);
+            const int c = 2 * ks + ((lane >> 3) & 1);
+            ldmatrix_x4(b0, b1, b2, b3, tk + tile_off(kr, c));
+            mma16816(sc[0], qf[ks], b0, b1);
+            mma16816(sc[1], qf[ks], b2, b3);
+        }
+        float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int h = e >> 1;
+                const int j = tile_key + key0 + n * 8 + 2 * tig + (e & 1);
+                const bool vis = row_ok[h] && ib_visible(j, lo, pos, keep);
+                float x = sc[n][e] * scale_r[h];
+                if (OPTIONS) {
+                    x -= slope_r[h] * (float)(pos - j);
+                    if (P.opt.cap > 0.0f) x = ib_capped_log2(x, P.cap_c);
+                }
+                sc[n][e] = vis ? x : -INFINITY;
+                mx[h] = fmaxf(mx[h], sc[n][e]);
+            }
+        float corr[2], msafe[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
+            mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
+            const float m_new = fmaxf(m_r[h], mx[h]);
+            msafe[h] = m_new == -INFINITY ? 0.0f : m_new;
+            corr[h] = m_r[h] == -INFINITY ? 0.0f : exp2f(m_r[h] - msafe[h]);
+            m_r[h] = m_new;
+            l_r[h] *= corr[h];
+        }
+#pragma unroll
+        for (int n = 0; n < D / 8; ++n) {
+            o[n][0] *= corr[0]; o[n][1] *= corr[0];
+            o[n][2] *= corr[1]; o[n][3] *= corr[1];
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float p = exp2f(sc[n][e] - msafe[e >> 1]);
+                sc[n][e] = p;
+                l_r[e >> 1] += p;
+            }
+        unsigned a[4];
+        a[0] = pack_bf16(sc[0][0], sc[0][1]);
+        a[1] = pack_bf16(sc[0][2], sc[0][3]);
+        a[2] = pack_bf16(sc[1][0], sc[1][1]);
+        a[3] = pack_bf16(sc[1][2], sc[1][3]);
+#pragma unroll
+        for (int dn = 0; dn < D / 16; ++dn) {
+            unsigned b0, b1, b2, b3;
+            const int kr = key0 + (lane & 7) + 8 * ((lane >> 3) & 1);
+            const int c = 2 * dn + (lane >> 4);
+            ldmatrix_x4_trans(b0, b1, b2, b3, tv + tile_off(kr, c));
+            mma16816(o[2 * dn], a, b0, b1);
+            mma16816(o[2 * dn + 1], a, b2, b3);
+        }
+    }
+
+    __device__ __forceinline__ void close(int lane, int warp, int G, float* sm, float* sl) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            l_r[h] += __shfl_xor_sync(0xffffffffu, l_r[h], 1);
+            l_r[h] += __shfl_xor_sync(0xffffffffu, l_r[h], 2);
+            const int head = (lane >> 2) + 8 * h;
+            if ((lane & 3) == 0 && head < G) { sm[warp * 16 + head] = m_r[h]; sl[warp * 16 + head] = l_r[h]; }
+        }
+    }
+
+    __device__ __forceinline__ void put(float* so, int ld, int d0, int dims, int lane, int G) const {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int head = (lane >> 2) + 8 * h;
+            if (head >= G) continue;
+#pragma unroll
+            for (int n = 0; n < D / 8; ++n)
+                if (n * 8 >= d0 && n * 8 < d0 + dims)
+                    *reinterpret_cast<float2*>(so + head * ld + n * 8 - d0 + 2 * (lane & 3)) = make_float2(o[n][2 * h], o[n][2 * h + 1]);
+        }
+    }
+};
+
+// Four numbers of a row's end: the sink joins the row's sum L (M its maximum), then the gate.
+template <bool OPTIONS>
+__device__ __forceinline__ void store_row(const Params& P, __nv_bfloat16* out_row, int row, int head, int e, float4 acc,
+                                          float M, float L) {
+    __nv_bfloat162 lo2, hi2;
+    if (OPTIONS) {
+        float f = 1.0f;
+        if (P.opt.sinks) {
+            const float sink = P.opt.sinks[head] * 1.4426950408889634f;
+            const float m_new = fmaxf(M, sink);
+            f = M == -INFINITY ? 0.0f : exp2f(M - m_new);
+            L = L * f + exp2f(sink - m_new);
+        }
+        f = L > 0.0f ? f / L * ib_head_gate(P.opt, row, head) : 0.0f;
+        lo2 = __floats2bfloat162_rn(acc.x * f, acc.y * f);
+        hi2 = __floats2bfloat162_rn(acc.z * f, acc.w * f);
+    } else {
+        if (!(L > 0.0f)) { acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f); L = 1.0f; }
+        lo2 = __floats2bfloat162_rn(acc.x / L, acc.y / L);
+        hi2 = __floats2bfloat162_rn(acc.z / L, acc.w / L);
+    }
+    uint2 w;
+    w.x = *reinterpret_cast<unsigned*>(&lo2);
+    w.y = *reinterpret_cast<unsigned*>(&hi2);
+    *reinterpret_cast<uint2*>(out_row + head * D + e) = w;
+}
+
 // OPTIONS: a factor, a slope and a sink per head, a cap on the scores, a sequence's first keys beside the window, a
 // gate per head.
-template <bool OPTIONS>
+template <bool OPTIONS, bool FEW>
 __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constant__ CUtensorMap map_k,
                                                             const __grid_constant__ CUtensorMap map_v, const Params P) {
     extern __shared__ unsigned char raw_smem[];
@@ -131,9 +403,7 @@ __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constan
         asm volatile("bar.sync 1, 128;" ::: "memory");
     }
 
-    float o[D / 8][4];
-    float m_r[2] = {-INFINITY, -INFINITY}, l_r[2] = {0.0f, 0.0f};
-    const int gid = lane >> 2, tig = lane & 3;
+    Share<OPTIONS, FEW> mine;
 
     if (warp == 4) {
         // producer: lane p brings page p of every tile (K and V, two 64-column halves each)
@@ -177,159 +447,31 @@ __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constan
         }
         if (!waited) asm volatile("griddepcontrol.wait;" ::: "memory");   // the loop never reached it
     } else {
-#pragma unroll
-        for (int n = 0; n < D / 8; ++n)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) o[n][i] = 0.0f;
-        // query fragments: rows gid and gid + 8 of the 16-row tile
-        unsigned qf[D / 16][4];
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-            const int r = (lane & 7) + 8 * ((lane >> 3) & 1);
-            const int c = 2 * ks + (lane >> 4);
-            ldmatrix_x4(qf[ks][0], qf[ks][1], qf[ks][2], qf[ks][3], smem_u32(sq + r * D + c * 8));
-        }
-        const bool row_ok[2] = {gid < G, gid + 8 < G};
-        float scale_r[2] = {P.scale_log2, P.scale_log2}, slope_r[2] = {0.0f, 0.0f};
-        if (OPTIONS) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (!row_ok[h]) continue;
-                const int head = kvh * G + gid + 8 * h;
-                if (P.opt.head_scale) scale_r[h] *= P.opt.head_scale[head];
-                if (P.opt.slopes) slope_r[h] = P.opt.slopes[head] * P.slope_factor;
-            }
-        }
+        mine.begin(sq, lane, P, kvh * G, G);
         for (int i = 0; i < n_tiles; ++i) {
             const int s = i % STAGES;
             if (ok && !mbar_wait(full0 + 8 * s, (i / STAGES) & 1, 2)) ok = false;
-            const unsigned tk = smem_u32(sk + s * TILE_BYTES), tv = smem_u32(sv + s * TILE_BYTES);
-            const int key0 = warp * 16;                      // this warp's 16 keys of the tile
-            float sc[2][4];
-#pragma unroll
-            for (int n = 0; n < 2; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) sc[n][e] = 0.0f;
-#pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks) {
-                unsigned b0, b1, b2, b3;
-                const int kr = key0 + (lane & 7) + 8 * (lane >> 4);
-                const int c = 2 * ks + ((lane >> 3) & 1);
-                ldmatrix_x4(b0, b1, b2, b3, tk + tile_off(kr, c));
-                mma16816(sc[0], qf[ks], b0, b1);
-                mma16816(sc[1], qf[ks], b2, b3);
-            }
-            const int tile_key = ib_nth_tile(i_begin + i, n_kept, t_first) * KEYS;
-            float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-            for (int n = 0; n < 2; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int h = e >> 1;
-                    const int j = tile_key + key0 + n * 8 + 2 * tig + (e & 1);
-                    const bool vis = row_ok[h] && ib_visible(j, lo, pos, keep);
-                    float x = sc[n][e] * scale_r[h];
-                    if (OPTIONS) {
-                        x -= slope_r[h] * (float)(pos - j);
-                        if (P.opt.cap > 0.0f) x = ib_capped_log2(x, P.cap_c);
-                    }
-                    sc[n][e] = vis ? x : -INFINITY;
-                    mx[h] = fmaxf(mx[h], sc[n][e]);
-                }
-            float corr[2], msafe[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
-                mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
-                const float m_new = fmaxf(m_r[h], mx[h]);
-                msafe[h] = m_new == -INFINITY ? 0.0f : m_new;
-                corr[h] = m_r[h] == -INFINITY ? 0.0f : exp2f(m_r[h] - msafe[h]);
-                m_r[h] = m_new;
-                l_r[h] *= corr[h];
-            }
-#pragma unroll
-            for (int n = 0; n < D / 8; ++n) {
-                o[n][0] *= corr[0]; o[n][1] *= corr[0];
-                o[n][2] *= corr[1]; o[n][3] *= corr[1];
-            }
-#pragma unroll
-            for (int n = 0; n < 2; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float p = exp2f(sc[n][e] - msafe[e >> 1]);
-                    sc[n][e] = p;
-                    l_r[e >> 1] += p;
-                }
-            unsigned a[4];
-            a[0] = pack_bf16(sc[0][0], sc[0][1]);
-            a[1] = pack_bf16(sc[0][2], sc[0][3]);
-            a[2] = pack_bf16(sc[1][0], sc[1][1]);
-            a[3] = pack_bf16(sc[1][2], sc[1][3]);
-#pragma unroll
-            for (int dn = 0; dn < D / 16; ++dn) {
-                unsigned b0, b1, b2, b3;
-                const int kr = key0 + (lane & 7) + 8 * ((lane >> 3) & 1);
-                const int c = 2 * dn + (lane >> 4);
-                ldmatrix_x4_trans(b0, b1, b2, b3, tv + tile_off(kr, c));
-                mma16816(o[2 * dn], a, b0, b1);
-                mma16816(o[2 * dn + 1], a, b2, b3);
-            }
+            mine.step(smem_u32(sk + s * TILE_BYTES), smem_u32(sv + s * TILE_BYTES), warp, lane,
+                      ib_nth_tile(i_begin + i, n_kept, t_first) * KEYS, lo, pos, keep, P, G);
             __syncwarp();
             if (lane == 0) mbar_arrive(empty0 + 8 * s);      // this warp has read the stage
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            l_r[h] += __shfl_xor_sync(0xffffffffu, l_r[h], 1);
-            l_r[h] += __shfl_xor_sync(0xffffffffu, l_r[h], 2);
         }
     }
 
     // merge the four warps' partial results (different keys, same rows); the rings are idle by now
     __syncthreads();
-    float* so = reinterpret_cast<float*>(sk);                // [4 warps][16 rows][128]
-    float* sm = so + 4 * 16 * D;                              // [4][16]
+    constexpr int LD = D + 4;                                // (lanes of other heads meet other banks)
+    float* so = reinterpret_cast<float*>(sk);                // [4 warps][16 rows][LD]
+    float* sm = so + 4 * 16 * LD;                             // [4][16]
     float* sl = sm + 4 * 16;                                  // [4][16]
     if (warp < 4) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int r = gid + 8 * h;
-            if (r >= G) continue;                             // rows beyond the group's heads hold nothing
-            if (tig == 0) { sm[warp * 16 + r] = m_r[h]; sl[warp * 16 + r] = l_r[h]; }
-#pragma unroll
-            for (int n = 0; n < D / 8; ++n) {
-                *reinterpret_cast<float2*>(so + (warp * 16 + r) * D + n * 8 + 2 * tig) = make_float2(o[n][2 * h], o[n][2 * h + 1]);
-            }
-        }
+        mine.close(lane, warp, G, sm, sl);
+        mine.put(so + warp * 16 * LD, LD, 0, D, lane, G);
     }
     __syncthreads();
     __nv_bfloat16* const out_row = P.out + row * P.opt.out_ld;
-    // a row's end: the sink joins the row's sum L (M its maximum), then the gate; returns the factor on the output
-    auto finish = [&](int g, float M, float L) -> float {
-        const int head = kvh * G + g;
-        float f = 1.0f;
-        if (P.opt.sinks) {
-            const float sink = P.opt.sinks[head] * 1.4426950408889634f;
-            const float m_new = fmaxf(M, sink);
-            f = M == -INFINITY ? 0.0f : exp2f(M - m_new);
-            L = L * f + exp2f(sink - m_new);
-        }
-        return L > 0.0f ? f / L * ib_head_gate(P.opt, row, head) : 0.0f;
-    };
     auto store4 = [&](int g, int e, float4 acc, float M, float L) {
-        __nv_bfloat162 lo2, hi2;
-        if (OPTIONS) {
-            const float f = finish(g, M, L);
-            lo2 = __floats2bfloat162_rn(acc.x * f, acc.y * f);
-            hi2 = __floats2bfloat162_rn(acc.z * f, acc.w * f);
-        } else {
-            if (!(L > 0.0f)) { acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f); L = 1.0f; }
-            lo2 = __floats2bfloat162_rn(acc.x / L, acc.y / L);
-            hi2 = __floats2bfloat162_rn(acc.z / L, acc.w / L);
-        }
-        uint2 w;
-        w.x = *reinterpret_cast<unsigned*>(&lo2);
-        w.y = *reinterpret_cast<unsigned*>(&hi2);
-        *reinterpret_cast<uint2*>(out_row + (kvh * G + g) * D + e) = w;
+        store_row<OPTIONS>(P, out_row, row, kvh * G + g, e, acc, M, L);
     };
     const long part0 = (long)place * P.n_heads + kvh * G;     // of the slices' scratch
     for (int idx = threadIdx.x; idx < G * (D / 4); idx += THREADS) {   // four elements per thread: one pass
@@ -343,7 +485,7 @@ __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constan
 #pragma unroll
             for (int w = 0; w < 4; ++w) {
                 const float f = exp2f(sm[w * 16 + g] - M);
-                const float4 v = *reinterpret_cast<const float4*>(so + (w * 16 + g) * D + e);
+                const float4 v = *reinterpret_cast<const float4*>(so + (w * 16 + g) * LD + e);
                 acc.x += f * v.x; acc.y += f * v.y; acc.z += f * v.z; acc.w += f * v.w;
                 L += f * sl[w * 16 + g];
             }
@@ -459,15 +601,19 @@ IB_EXPORT int ib_paged_attention_decode(const void* q, const void* k_pages, cons
     P.cap_c = cap * 1.4426950408889634f;
     P.opt = {head_scale, slopes, sinks, cap, keep_first, (const act_t*)gate, gate_ld, out_ld};
     const size_t smem = 2 * dec::STAGES * dec::TILE_BYTES + 16 * dec::D * 2 + (2 * dec::STAGES + 1) * 8 + 1024;
-    static IbDeviceSet configured, configured_options;   // the attribute is kept per device
     const dim3 grid(n_rows, n_kv_heads, max_splits);
-    if (head_scale != nullptr || slopes != nullptr || sinks != nullptr || cap > 0.0f || gate != nullptr || keep_first > 0) {
-        if (const int e = ib_allow_dynamic_smem(configured_options, dec::decode_kernel<true>, smem)) return e;
-        ib_launch(dec::decode_kernel<true>, grid, dec::THREADS, smem, stream, mk, mv, P);
-    } else {
-        if (const int e = ib_allow_dynamic_smem(configured, dec::decode_kernel<false>, smem)) return e;
-        ib_launch(dec::decode_kernel<false>, grid, dec::THREADS, smem, stream, mk, mv, P);
-    }
+    const bool options = head_scale != nullptr || slopes != nullptr || sinks != nullptr || cap > 0.0f || gate != nullptr || keep_first > 0;
+#define IB_DECODE(OPTIONS, FEW)                                                                                \
+    do {                                                                                                       \
+        static IbDeviceSet configured; /* the attribute is kept per device */                                  \
+        if (const int e = ib_allow_dynamic_smem(configured, dec::decode_kernel<OPTIONS, FEW>, smem)) return e; \
+        ib_launch(dec::decode_kernel<OPTIONS, FEW>, grid, dec::THREADS, smem, stream, mk, mv, P);              \
+    } while (0)
+    if (options && G <= 8) IB_DECODE(true, true);
+    else if (options) IB_DECODE(true, false);
+    else if (G <= 8) IB_DECODE(false, true);
+    else IB_DECODE(false, false);
+#undef IB_DECODE
     return ib_launch_status();
 }
 

@@ -616,6 +616,23 @@ def test_paged_attention_decode(nh, nkv, ps, window, max_splits):
     assert rel_err(got, want) < 5e-2, "the far key that stands out was not seen"
 
 
+@pytest.mark.parametrize("nh,nkv", [(1, 1), (7, 1), (8, 1), (9, 1), (16, 2), (15, 5)])
+@pytest.mark.parametrize("splits", [1, 5])
+def test_decode_attention_at_the_edge_of_its_two_forms(nh, nkv, splits):
+    """Up to eight heads a group are the columns of the products, more are their rows; keys around a tile's and a warp's
+    edge.  bfloat16 probabilities and outputs: within 2e-2 of the float32 reference, as above."""
+    from inferrs_b200 import kernels as K
+    lens = [1, 15, 16, 17, 63, 64, 65, 129, 700]
+    table, positions, row_request, k_pages, v_pages = _paged_setup(torch.bfloat16, nkv, 128, 16, lens, [1] * len(lens), 61)
+    q = rand((len(lens), nh, 128), torch.bfloat16, 62)
+    out = torch.full((len(lens), nh * 128), float("nan"), dtype=torch.bfloat16, device=dev())
+    ref = torch.empty_like(out)
+    K.paged_attention_decode(q, k_pages, v_pages, table, positions, 128 ** -0.5, None, out, splits, min_tiles=2)
+    assert K.attention_decode_error() == 0
+    R.paged_attention_generic(q, k_pages, v_pages, table, row_request, positions, 128 ** -0.5, None, ref)
+    assert rel_err(out, ref) < 2e-2
+
+
 def test_how_the_decode_kernel_is_cut_follows_the_waves_of_ctas():
     """Host arithmetic only: the slices per request for numbers of (request, head group) pairs around one and two
     waves of resident CTAs."""
