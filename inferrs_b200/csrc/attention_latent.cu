@@ -167,18 +167,24 @@ latent_attention_kernel(const QT* __restrict__ q, long q_row, long q_head, const
     }
 }
 
-// Joins the slices of one (row, head): a warp each.  A lane owns up to two slices' weights exp(m_s - m) (at most 64
-// slices); the sums then run over the slices in ascending order with loads that carry no condition (a slice without
-// keys has left zeros and the weight 0), so they are all under way together.
-__global__ void latent_attention_join_kernel(const float* __restrict__ ws_acc, const float* __restrict__ ws_ml,
-                                             int n_rows, int n_heads, int R, int n_slices, act_t* __restrict__ out,
-                                             long o_row, long o_head) {
+// Joins the slices of one (row, head): a thread per number, so that the few rows of a decode step have all their loads
+// under way at once.  A lane owns up to two slices' weights exp(m_s - m) (at most 64 slices), every warp all of them; the
+// sums then run over the slices in ascending order, a group of slices' numbers asked for before its weights are used
+// and without a condition (a slice without keys has left zeros and the weight 0).
+#define LJ_THREADS 128
+#define LJ_GROUP 16
+
+__global__ void __launch_bounds__(LJ_THREADS) latent_attention_join_kernel(
+    const float* __restrict__ ws_acc, const float* __restrict__ ws_ml, int n_heads, int R, int n_slices,
+    act_t* __restrict__ out, long o_row, long o_head) {
     ib_grid_dependency_sync();
-    const int lane = threadIdx.x & 31;
-    const long item = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (item >= (long)n_rows * n_heads) return;
-    const int row = (int)(item / n_heads), h = (int)(item % n_heads);
+    const int lane = threadIdx.x & 31, e = blockIdx.y * LJ_THREADS + threadIdx.x;
+    const long item = blockIdx.x;
     const float* ml = ws_ml + item * n_slices * 2;
+    const float* acc = ws_acc + item * n_slices * R + min(e, R - 1);
+    float part[LJ_GROUP];
+#pragma unroll
+    for (int j = 0; j < LJ_GROUP; ++j) part[j] = acc[(long)min(j, n_slices - 1) * R];
     float ms[2], ls[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
@@ -193,22 +199,18 @@ __global__ void latent_attention_join_kernel(const float* __restrict__ ws_acc, c
     for (int k = 0; k < 2; ++k) w[k] = (ms[k] == -INFINITY) ? 0.0f : expf(ms[k] - m);
     const float l = ib_warp_sum(ls[0] * w[0] + ls[1] * w[1]);
     const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-    const float* acc = ws_acc + item * n_slices * R;
-    act_t* dst = out + (long)row * o_row + (long)h * o_head;
-    // all of a slice's numbers for this lane are asked for together (up to 16 loads under way), slice after slice
-    float v[16];
+    float v = 0.0f;
+    for (int s0 = 0; s0 < n_slices; s0 += LJ_GROUP) {
 #pragma unroll
-    for (int k = 0; k < 16; ++k) v[k] = 0.0f;
-#pragma unroll 2
-    for (int s = 0; s < n_slices; ++s) {
-        const float ws = __shfl_sync(0xffffffffu, s < 32 ? w[0] : w[1], s & 31);
-        const float* a = acc + (long)s * R;
+        for (int j = 0; j < LJ_GROUP; ++j) {
+            const int s = s0 + j;
+            const float ws = __shfl_sync(0xffffffffu, s < 32 ? w[0] : w[1], s & 31);    // beyond the slices: 0
+            v = s < n_slices ? fmaf(part[j], ws, v) : v;
+        }
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = fmaf(a[min(lane + 32 * k, R - 1)], ws, v[k]);
+        for (int j = 0; j < LJ_GROUP; ++j) part[j] = acc[(long)min(s0 + LJ_GROUP + j, n_slices - 1) * R];
     }
-#pragma unroll
-    for (int k = 0; k < 16; ++k)
-        if (lane + 32 * k < R) dst[lane + 32 * k] = ib_from_float<act_t>(v[k] * inv);
+    if (e < R) out[(item / n_heads) * o_row + (item % n_heads) * o_head + e] = ib_from_float<act_t>(v * inv);
 }
 
 #if IB_ACT_BF16
@@ -608,10 +610,8 @@ IB_EXPORT int ib_latent_attention(const void* q, int q_is_f32, long q_row, long 
         }
         if (e != IB_ERR_UNSUPPORTED) {
             if (e != IB_OK || n_slices == 1) return e;
-            const int jw = 4;
-            const long n_items = (long)n_rows * n_heads;
-            ib_launch(latent_attention_join_kernel, (unsigned)((n_items + jw - 1) / jw), 32 * jw, 0, stream, ws_acc, ws_ml,
-                      n_rows, n_heads, R, n_slices, (act_t*)out, o_row, o_head);
+            ib_launch(latent_attention_join_kernel, dim3((unsigned)((long)n_rows * n_heads), (R + LJ_THREADS - 1) / LJ_THREADS), LJ_THREADS, 0,
+                      stream, ws_acc, ws_ml, n_heads, R, n_slices, (act_t*)out, o_row, o_head);
             return ib_launch_status();
         }
         e = IB_OK;
@@ -631,9 +631,7 @@ IB_EXPORT int ib_latent_attention(const void* q, int q_is_f32, long q_row, long 
 #undef IB_LAT_R
 #undef IB_LAT
     if (e != IB_OK || n_slices == 1) return e;
-    const int warps = 4;
-    const long items = (long)n_rows * n_heads;
-    ib_launch(latent_attention_join_kernel, (unsigned)((items + warps - 1) / warps), 32 * warps, 0, stream, ws_acc, ws_ml,
-              n_rows, n_heads, R, n_slices, (act_t*)out, o_row, o_head);
+    ib_launch(latent_attention_join_kernel, dim3((unsigned)((long)n_rows * n_heads), (R + LJ_THREADS - 1) / LJ_THREADS), LJ_THREADS, 0, stream,
+              ws_acc, ws_ml, n_heads, R, n_slices, (act_t*)out, o_row, o_head);
     return ib_launch_status();
 }
