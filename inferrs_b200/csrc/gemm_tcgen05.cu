@@ -583,10 +583,14 @@ static int choose_splits(int n_tok, int n_out, int num_kb, int bn, int split_k) 
     int splits = split_k;
     if (splits <= 0) {
         const long tiles = (long)((n_out + tc::BM - 1) / tc::BM) * ((n_tok + bn - 1) / bn);
-        // few tiles over a long K (the down projection of a decode step): eight parts, of which each CTA has a
-        // larger share on its way before the kernel before it has finished; over a short K eight cost more
-        // in the cluster's summing than they gain
-        splits = tiles >= 120 ? 1 : tiles >= 60 ? 2 : (tiles < 40 && num_kb >= 128) ? 8 : 4;
+        // Few tiles: parts until the CTAs' rings hold most of W before the kernel before them has finished; a ring is
+        // 80 KB, so that is what a CTA has on its way by then.  Eight parts over a long K (the down projection of a
+        // decode step), and over a shorter one too where the tiles are so few that four parts would leave most SMs
+        // without a CTA (1,024 features over 2,048 and 3,072: a decode step of one request 1,133 -> 1,083 us with 64
+        // CTAs in place of 32); 32 tiles over 4,096 are as fast with four (985 us a step of 8 requests, 995 with eight).
+        // Sixty to seventy tiles: four parts still fit as one wave of two CTAs an SM (8,192 features over 2,048, in a
+        // model of four layers: 2 % of the step).
+        splits = tiles >= 120 ? 1 : tiles > 71 ? 2 : tiles >= 60 ? 4 : (tiles < 40 && num_kb >= 128) || (tiles < 20 && num_kb >= 32) ? 8 : 4;
     }
     if (bn == 256) splits = 1;
     while (splits > 1 && (num_kb + splits - 1) / splits * (splits - 1) >= num_kb) splits >>= 1;  // no empty part
