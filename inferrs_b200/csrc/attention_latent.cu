@@ -252,8 +252,9 @@ __host__ __device__ constexpr int lm_swizzle(int rk) { return rk % 64 == 0 ? 7 :
 // (tile_req[i] < 0: no tile); the two tokens' queries meet every tile of latents together, so a prompt's latents
 // cross from L2 half as often and every B operand serves twice as many products.  One slice then.
 // ROT: cached vectors and queries have rot.width (a multiple of 16) more numbers, which join the scores alone.
-template <int NT, int TT, bool ROT>
-__global__ void __launch_bounds__(128)
+// WARPS: 4, or 8 for two tokens: four warps then score one token each, and a warp sums an eighth of R.
+template <int NT, int TT, bool ROT, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, WARPS == 8 ? 2 : 1)
 latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, long q_head,
                             const __nv_bfloat16* __restrict__ plane, const int* __restrict__ block_table, int max_pages,
                             int page_size, int n_pages, const int* __restrict__ row_request,
@@ -262,6 +263,8 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
                             int window, int n_slices, __nv_bfloat16* __restrict__ out, long o_row, long o_head,
                             float* __restrict__ ws_acc, float* __restrict__ ws_ml, const LatentRot rot) {
     constexpr int R = 32 * NT, MR = TT * LM_ROWS;
+    constexpr int TS = TT * 4 / WARPS;                   // tokens that a warp scores
+    constexpr int NW = NT * 4 / WARPS;                   // n-tiles of 8 columns that it sums
     const int RK = ROT ? R + rot.width : R;              // numbers of a cached vector
     const int sw = ROT ? lm_swizzle(RK) : 0;             // rows without padding, their 16-byte places exchanged
     const int LDC = RK + (sw ? 0 : LM_PAD), LDP = LM_KEYS + (sw ? 0 : LM_PAD);
@@ -277,6 +280,7 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
     ib_grid_dependency_sync();
     const int slice = blockIdx.z, head0 = blockIdx.y * LM_ROWS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int kw = warp & 3, ts0 = (warp >> 2) * TS;     // this warp's 16 keys of a tile, its first token
     int row, req, n_tok = 1;
     if (TT == 1) {
         row = blockIdx.x;
@@ -312,9 +316,10 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
             q_s[at(m, LDC, (R + e) & ~7) + (e & 7)] = __float2bfloat16_rn(ok ? latent_rot_value<__nv_bfloat16>(rot, row + tok, h, e, pos0 + tok) : 0.0f);
         }
     }
-    // two threads per key: the page is looked up once per key and tile, each thread copies half of the latent
+    // two or four threads per key: each looks the page up and copies its share of the latent
     auto load_tile = [&](int t) {
-        const int jj = threadIdx.x >> 1, half = threadIdx.x & 1;
+        constexpr int PER = WARPS / 2;                   // threads per key
+        const int jj = threadIdx.x / PER, half = threadIdx.x % PER;
         const int j = first + t * LM_KEYS + jj;
         const __nv_bfloat16* src = plane;
         int bytes = 0;
@@ -326,19 +331,19 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
             }
         }
 #pragma unroll
-        for (int ch = half; ch < R / 8; ch += 2) lm_cp_async16(c_s + at(jj, LDC, ch * 8), bytes ? src + ch * 8 : src, bytes);
+        for (int ch = half; ch < R / 8; ch += PER) lm_cp_async16(c_s + at(jj, LDC, ch * 8), bytes ? src + ch * 8 : src, bytes);
         if constexpr (ROT)
-            for (int ch = R / 8 + half; ch < RK / 8; ch += 2) lm_cp_async16(c_s + at(jj, LDC, ch * 8), bytes ? src + ch * 8 : src, bytes);
+            for (int ch = R / 8 + half; ch < RK / 8; ch += PER) lm_cp_async16(c_s + at(jj, LDC, ch * 8), bytes ? src + ch * 8 : src, bytes);
     };
     if (t0 < t1) load_tile(t0);
     asm volatile("cp.async.commit_group;" ::: "memory");
 
-    float o[TT][NT][4];
+    float o[TT][NW][4];
     float m_run[TT][2], l_run[TT][2];                 // rows lane/4 and lane/4 + 8 of every token
 #pragma unroll
     for (int tk = 0; tk < TT; ++tk) {
 #pragma unroll
-        for (int i = 0; i < NT; ++i) o[tk][i][0] = o[tk][i][1] = o[tk][i][2] = o[tk][i][3] = 0.0f;
+        for (int i = 0; i < NW; ++i) o[tk][i][0] = o[tk][i][1] = o[tk][i][2] = o[tk][i][3] = 0.0f;
         m_run[tk][0] = m_run[tk][1] = -INFINITY;
         l_run[tk][0] = l_run[tk][1] = 0.0f;
     }
@@ -348,11 +353,11 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
         const __nv_bfloat16* ct = c_s;
-        // ---- scores of this warp's 16 keys, for every token -------------------------------------------------
+        // ---- scores of this warp's 16 keys, for its tokens -------------------------------------------------
         // (two sets of accumulators take turns, so that a product does not wait for the one before it)
-        float sc[TT][2][4], sd[TT][2][4];
+        float sc[TS][2][4], sd[TS][2][4];
 #pragma unroll
-        for (int tk = 0; tk < TT; ++tk)
+        for (int tk = 0; tk < TS; ++tk)
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 sc[tk][i][0] = sc[tk][i][1] = sc[tk][i][2] = sc[tk][i][3] = 0.0f;
@@ -360,11 +365,11 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
             }
         auto score_step = [&](int ks, bool second) {
             uint32_t b0, b1, b2, b3;
-            lm_ldmatrix_x4(b0, b1, b2, b3, ct + at(warp * 16 + (lane & 7) + (lane >> 4) * 8, LDC, ks * 16 + ((lane >> 3) & 1) * 8));
+            lm_ldmatrix_x4(b0, b1, b2, b3, ct + at(kw * 16 + (lane & 7) + (lane >> 4) * 8, LDC, ks * 16 + ((lane >> 3) & 1) * 8));
 #pragma unroll
-            for (int tk = 0; tk < TT; ++tk) {
+            for (int tk = 0; tk < TS; ++tk) {
                 uint32_t a0, a1, a2, a3;
-                lm_ldmatrix_x4(a0, a1, a2, a3, q_s + at(tk * LM_ROWS + (lane & 15), LDC, ks * 16 + (lane >> 4) * 8));
+                lm_ldmatrix_x4(a0, a1, a2, a3, q_s + at((ts0 + tk) * LM_ROWS + (lane & 15), LDC, ks * 16 + (lane >> 4) * 8));
                 if (second) {
                     lm_mma(sd[tk][0], a0, a1, a2, a3, b0, b1);
                     lm_mma(sd[tk][1], a0, a1, a2, a3, b2, b3);
@@ -378,11 +383,12 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
         for (int ks = 0; ks < R / 16; ++ks) score_step(ks, ks & 1);
         if constexpr (ROT)
             for (int ks = R / 16; ks < RK / 16; ++ks) score_step(ks, false);
-        const int j_base = first + t * LM_KEYS + warp * 16 + 2 * (lane & 3);
+        const int j_base = first + t * LM_KEYS + kw * 16 + 2 * (lane & 3);
 #pragma unroll
-        for (int tk = 0; tk < TT; ++tk) {
-            const int lo = lo0 + (window > 0 && pos0 + tk - window + 1 > 0 ? (pos0 + tk - window + 1) - lo0 : 0);
-            const int hi = tk < n_tok ? pos0 + tk : -1;             // a token that does not exist sees nothing
+        for (int tk = 0; tk < TS; ++tk) {
+            const int tok = ts0 + tk;
+            const int lo = lo0 + (window > 0 && pos0 + tok - window + 1 > 0 ? (pos0 + tok - window + 1) - lo0 : 0);
+            const int hi = tok < n_tok ? pos0 + tok : -1;             // a token that does not exist sees nothing
             float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
             for (int i = 0; i < 2; ++i)
@@ -399,35 +405,41 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
                 mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], 2));
             }
             if ((lane & 3) == 0) {
-                pmax[warp * MR + tk * LM_ROWS + r_lo] = mx[0];
-                pmax[warp * MR + tk * LM_ROWS + r_hi] = mx[1];
+                pmax[kw * MR + tok * LM_ROWS + r_lo] = mx[0];
+                pmax[kw * MR + tok * LM_ROWS + r_hi] = mx[1];
             }
         }
         __syncthreads();
         float corr[TT][2];
 #pragma unroll
         for (int tk = 0; tk < TT; ++tk) {
-            float m_new[2];
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
                 const int rr = tk * LM_ROWS + (k ? r_hi : r_lo);
                 const float tm = fmaxf(fmaxf(pmax[rr], pmax[MR + rr]), fmaxf(pmax[2 * MR + rr], pmax[3 * MR + rr]));
-                m_new[k] = fmaxf(m_run[tk][k], tm);
-                corr[tk][k] = (m_run[tk][k] == -INFINITY) ? 0.0f : expf(m_run[tk][k] - m_new[k]);
-                m_run[tk][k] = m_new[k];
+                const float m_new = fmaxf(m_run[tk][k], tm);
+                corr[tk][k] = (m_run[tk][k] == -INFINITY) ? 0.0f : expf(m_run[tk][k] - m_new);
+                m_run[tk][k] = m_new;
             }
+        }
+#pragma unroll
+        for (int tk = 0; tk < TS; ++tk) {
+            const int tok = ts0 + tk;
+            float top[2];                             // the token's maxima (ts0 is 0 or 1: no index into registers)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) top[k] = (TS == TT || ts0 == 0) ? m_run[tk][k] : m_run[TT - 1][k];
             float sm[2] = {0.0f, 0.0f};
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 float p[4];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    p[c] = (sc[tk][i][c] == -INFINITY) ? 0.0f : expf(sc[tk][i][c] - m_new[c >> 1]);
+                    p[c] = (sc[tk][i][c] == -INFINITY) ? 0.0f : expf(sc[tk][i][c] - top[c >> 1]);
                     sm[c >> 1] += p[c];
                 }
-                const int col = warp * 16 + i * 8, in8 = 2 * (lane & 3);
-                *reinterpret_cast<__nv_bfloat162*>(p_s + at(tk * LM_ROWS + r_lo, LDP, col) + in8) = __floats2bfloat162_rn(p[0], p[1]);
-                *reinterpret_cast<__nv_bfloat162*>(p_s + at(tk * LM_ROWS + r_hi, LDP, col) + in8) = __floats2bfloat162_rn(p[2], p[3]);
+                const int col = kw * 16 + i * 8, in8 = 2 * (lane & 3);
+                *reinterpret_cast<__nv_bfloat162*>(p_s + at(tok * LM_ROWS + r_lo, LDP, col) + in8) = __floats2bfloat162_rn(p[0], p[1]);
+                *reinterpret_cast<__nv_bfloat162*>(p_s + at(tok * LM_ROWS + r_hi, LDP, col) + in8) = __floats2bfloat162_rn(p[2], p[3]);
             }
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
@@ -435,8 +447,8 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
                 sm[k] += __shfl_xor_sync(0xffffffffu, sm[k], 2);
             }
             if ((lane & 3) == 0) {
-                psum[warp * MR + tk * LM_ROWS + r_lo] = sm[0];
-                psum[warp * MR + tk * LM_ROWS + r_hi] = sm[1];
+                psum[kw * MR + tok * LM_ROWS + r_lo] = sm[0];
+                psum[kw * MR + tok * LM_ROWS + r_hi] = sm[1];
             }
         }
         __syncthreads();
@@ -448,12 +460,12 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
                 l_run[tk][k] = l_run[tk][k] * corr[tk][k] + ((psum[rr] + psum[MR + rr]) + (psum[2 * MR + rr] + psum[3 * MR + rr]));
             }
 #pragma unroll
-            for (int i = 0; i < NT; ++i) {
+            for (int i = 0; i < NW; ++i) {
                 o[tk][i][0] *= corr[tk][0]; o[tk][i][1] *= corr[tk][0];
                 o[tk][i][2] *= corr[tk][1]; o[tk][i][3] *= corr[tk][1];
             }
         }
-        // ---- this warp's quarter of the sums over all 64 keys, for every token -------------------------------
+        // ---- this warp's share of the sums over all 64 keys, for every token -------------------------------
 #pragma unroll
         for (int kk = 0; kk < LM_KEYS / 16; ++kk) {
             uint32_t a[TT][4];
@@ -461,13 +473,13 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
             for (int tk = 0; tk < TT; ++tk)
                 lm_ldmatrix_x4(a[tk][0], a[tk][1], a[tk][2], a[tk][3], p_s + at(tk * LM_ROWS + (lane & 15), LDP, kk * 16 + (lane >> 4) * 8));
 #pragma unroll
-            for (int i = 0; i < NT; i += 2) {
+            for (int i = 0; i < NW; i += 2) {
                 uint32_t b0, b1, b2, b3;
-                lm_ldmatrix_x4_trans(b0, b1, b2, b3, ct + at(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, LDC, warp * (R / 4) + i * 8 + (lane >> 4) * 8));
+                lm_ldmatrix_x4_trans(b0, b1, b2, b3, ct + at(kk * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, LDC, warp * (R / WARPS) + i * 8 + (lane >> 4) * 8));
 #pragma unroll
                 for (int tk = 0; tk < TT; ++tk) {
                     lm_mma(o[tk][i], a[tk][0], a[tk][1], a[tk][2], a[tk][3], b0, b1);
-                    if (i + 1 < NT) lm_mma(o[tk][i + 1], a[tk][0], a[tk][1], a[tk][2], a[tk][3], b2, b3);   // an odd last tile: the other half read padding
+                    if (i + 1 < NW) lm_mma(o[tk][i + 1], a[tk][0], a[tk][1], a[tk][2], a[tk][3], b2, b3);   // an odd last tile: the other half read padding
                 }
             }
         }
@@ -486,16 +498,16 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
             if (h >= n_heads) continue;
             if (n_slices == 1) {
                 const float inv = l_run[tk][k] > 0.0f ? 1.0f / l_run[tk][k] : 0.0f;
-                __nv_bfloat16* dst = out + (long)(row + tk) * o_row + (long)h * o_head + warp * (R / 4) + 2 * (lane & 3);
+                __nv_bfloat16* dst = out + (long)(row + tk) * o_row + (long)h * o_head + warp * (R / WARPS) + 2 * (lane & 3);
 #pragma unroll
-                for (int i = 0; i < NT; ++i)
+                for (int i = 0; i < NW; ++i)
                     *reinterpret_cast<__nv_bfloat162*>(dst + i * 8) =
                         __floats2bfloat162_rn(o[tk][i][2 * k] * inv, o[tk][i][2 * k + 1] * inv);
             } else {
                 const long item = ((long)(row + tk) * n_heads + h) * n_slices + slice;
-                float* dst = ws_acc + item * R + warp * (R / 4) + 2 * (lane & 3);
+                float* dst = ws_acc + item * R + warp * (R / WARPS) + 2 * (lane & 3);
 #pragma unroll
-                for (int i = 0; i < NT; ++i) {
+                for (int i = 0; i < NW; ++i) {
                     dst[i * 8] = o[tk][i][2 * k];
                     dst[i * 8 + 1] = o[tk][i][2 * k + 1];
                 }
@@ -517,19 +529,20 @@ static int launch_latent_mma(const void* q, long q_row, long q_head, const void*
                              const int* tile_req, const int* tile_row0, const int* q_start, int n_blocks, int n_heads,
                              float scale, int window, int n_slices, void* out, long o_row, long o_head, float* ws_acc,
                              float* ws_ml, const LatentRot& rot, cudaStream_t stream) {
-    constexpr int R = 32 * NT, MR = TT * LM_ROWS;
+    // Eight warps a block where two tokens meet and an eighth of R is whole pairs of n-tiles: see WARPS_TIMES
+    constexpr int R = 32 * NT, MR = TT * LM_ROWS, WARPS = TT == 2 && NT % 4 == 0 ? 8 : 4;
     auto smem_for = [](int width, int pad) {
         return (size_t)((MR + LM_KEYS) * (R + width + pad) + MR * (LM_KEYS + pad)) * 2 + 8 * MR * sizeof(float);
     };
     const size_t smem = ROT ? smem_for(rot.width, lm_swizzle(R + rot.width) ? 0 : LM_PAD) : smem_for(0, LM_PAD);
     const size_t smem_most = smem_for(ROT ? LM_MOST_ROT : 0, LM_PAD);     // the permission is given once per device, for the most
     if (smem_most > 48 * 1024) {
-        const int e = ib_allow_dynamic_smem(latent_mma_smem_set[ROT][TT - 1][NT], latent_attention_mma_kernel<NT, TT, ROT>,
+        const int e = ib_allow_dynamic_smem(latent_mma_smem_set[ROT][TT - 1][NT], latent_attention_mma_kernel<NT, TT, ROT, WARPS>,
                                             smem_most);
         if (e != IB_OK) return e;
     }
     const dim3 grid(n_blocks, (n_heads + LM_ROWS - 1) / LM_ROWS, n_slices);
-    ib_launch(latent_attention_mma_kernel<NT, TT, ROT>, grid, 128, smem, stream, (const __nv_bfloat16*)q, q_row, q_head,
+    ib_launch(latent_attention_mma_kernel<NT, TT, ROT, WARPS>, grid, 32 * WARPS, smem, stream, (const __nv_bfloat16*)q, q_row, q_head,
               (const __nv_bfloat16*)plane, block_table, max_pages, page_size, n_pages, row_request, positions, tile_req,
               tile_row0, q_start, n_heads, scale, window, n_slices, (__nv_bfloat16*)out, o_row, o_head, ws_acc, ws_ml, rot);
     return ib_launch_status();
