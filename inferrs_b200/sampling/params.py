@@ -80,14 +80,18 @@ def uniform_for(seed: int, step: int) -> float:
 
 
 def uniforms_for(seeds, steps):
-    """:func:`uniform_for` for many (seed, step) pairs at once, with the same bits, in native code.  Returns float32 [n]."""
+    """:func:`uniform_for` for many (seed, step) pairs at once, with the same bits, in native code.  One seed or one step
+    goes with every entry of the other list.  Returns float32 [n]."""
     import numpy as np
 
     from ..cache.manager import host_library
 
-    words = array("Q", [int(s) & _M64 for s in seeds])
-    words.extend([int(n) & _M64 for n in steps])
-    n = len(words) // 2
+    a, b = [int(s) & _M64 for s in seeds], [int(n) & _M64 for n in steps]
+    if len(a) != len(b):
+        if len(a) != 1 and len(b) != 1:
+            raise ValueError(f"{len(a)} seeds for {len(b)} steps")
+        a, b = (a * len(b), b) if len(a) == 1 else (a, b * len(a))
+    words, n = array("Q", a + b), len(a)
     out = np.empty((n,), dtype=np.float32)
     at = words.buffer_info()[0]
     host_library().ibh_uniforms(at, at + 8 * n, n, out.__array_interface__["data"][0])

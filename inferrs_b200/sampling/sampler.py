@@ -62,6 +62,8 @@ class Sampler:
         where nothing is pending) has it for the penalties' window.  Instead of ``pending_ids``, ``pending_from`` =
         (ids, places) names a tensor of token ids on the device and, per row, the place of the row's pending token
         in it (any valid place where nothing is pending): the look-up then goes to the device with everything else.
+        One options object, one seed or one history counts for every row; windows are those of the rows that have
+        both an options object and a history of their own.
 
         Everything the two kernels need per row goes to the device as one block of words in one copy that the
         host does not wait for, so a step can be prepared while the one before it still runs.
@@ -76,9 +78,9 @@ class Sampler:
         pend = [int(pending)] * r if isinstance(pending, int) else [int(x) for x in pending]
         if len(pend) != r or any(x not in (0, 1) for x in pend):
             raise ValueError("pending: 0 or 1, one for all rows or one per row")
-        length = [h.n_tokens if hasattr(h, "n_tokens") else len(h) for h in histories]
-        if any(pend):
-            length = [n + x for n, x in zip(length, pend)]
+        if len(params) not in (1, r):
+            raise ValueError(f"options of {len(params)} rows for {r}")
+        length = [(h.n_tokens if hasattr(h, "n_tokens") else len(h)) + x for h, x in zip(histories, pend)]
         # rows that share an options object share its numbers (looked up within this call only)
         options, kinds = {}, []
         for p in params:
@@ -123,8 +125,10 @@ class Sampler:
                 counts.append(n)
                 if n < width:
                     windows.extend(blank[:width - n])
-            words[9 * r:9 * r + r * width] = np.frombuffer(windows, dtype=np.int32)
-            n_prev[:] = counts
+            prev = words[9 * r:9 * r + r * width]
+            prev[:len(windows)] = windows
+            prev[len(windows):] = -1
+            n_prev[:len(counts)] = counts
         if look_up:
             words[9 * r + r * width:] = list(pending_from[1])
         dev = self._upload(words)

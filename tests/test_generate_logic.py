@@ -39,6 +39,38 @@ def test_uniforms_of_many_rows_have_the_same_bits():
     assert np.array_equal(uniforms_for(seeds, steps), want) and uniforms_for([], []).shape == (0,)
 
 
+def _sampler_words(monkeypatch, params, seeds, histories, rows):
+    """What a sampling call hands to its kernels: (temperatures, uniforms, windows)."""
+    from inferrs_b200 import kernels
+    from inferrs_b200.sampling.sampler import Sampler
+    got = {"windows": []}
+    monkeypatch.setattr(kernels, "sample", lambda l, t, k, p, m, u, out, act, **kw: got.update(t=t.tolist(), u=u.tolist()))
+    monkeypatch.setattr(kernels, "penalties", lambda l, prev, n, *rest: got.update(
+        windows=[sorted(row[:k]) for row, k in zip(prev.tolist(), n.tolist())]))
+    Sampler(torch.device("cpu")).sample(torch.zeros(rows, 9), params, seeds, histories)
+    return got["t"], got["u"], got["windows"]
+
+
+def test_sampling_with_lists_of_other_lengths(monkeypatch):
+    """One options object, seed or history counts for every row; any other length that is not the rows' is refused."""
+    import numpy as np
+    plain, window = SamplingParams(repetition_penalty=1.0), SamplingParams(repeat_last_n=3)
+    u = lambda seed, step: float(np.float32(uniform_for(seed, step)))   # noqa: E731
+    assert _sampler_words(monkeypatch, [plain] * 2, [4], [[1], [1, 2]], 2)[1] == [u(4, 1), u(4, 2)]
+    assert _sampler_words(monkeypatch, [plain] * 3, [1, 2, 3], [[1, 2]], 3)[1] == [u(1, 2), u(2, 2), u(3, 2)]
+    t, got, _ = _sampler_words(monkeypatch, [plain], [7, 8], [[1], [2]], 2)
+    assert t == [t[0]] * 2 and got == [u(7, 1), u(8, 1)]
+    # windows: of the rows with an options object and a history of their own; histories beyond the rows are not looked at
+    assert _sampler_words(monkeypatch, [window], [1] * 3, [[1, 2, 3, 4]] * 3, 3)[2] == [[2, 3, 4], [], []]
+    assert _sampler_words(monkeypatch, [window] * 3, [1] * 3, [[5]], 3)[2] == [[5], [], []]
+    assert _sampler_words(monkeypatch, [window] * 2, [1] * 2, [[1], [2], [3]], 2)[2] == [[1], [2]]
+    for params, seeds, histories in (([plain] * 4, [4, 5, 6], [[1]] * 5), ([plain] * 2, [1] * 4, [[1]] * 4),
+                                     ([window] * 5, [1] * 4, [[1]] * 4), ([plain] * 4, [1] * 4, [[1]] * 3),
+                                     ([plain] * 4, [], [[1]] * 4), ([plain] * 4, [1, 2], [[1]])):
+        with pytest.raises(ValueError):
+            _sampler_words(monkeypatch, params, seeds, histories, 4)
+
+
 @pytest.mark.parametrize("name", ["A", "B"])
 def test_greedy_generation(model_dirs, monkeypatch, name):
     kernel_refs.install(monkeypatch)
