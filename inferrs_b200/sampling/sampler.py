@@ -119,7 +119,11 @@ class Sampler:
                         windows.append(-1)
                     if known > 0:
                         tail = h.tail(known) if hasattr(h, "tail") else h[-known:]
-                        windows.fromlist(tail if isinstance(tail, list) else list(tail))
+                        tail = tail if isinstance(tail, list) else list(tail)
+                        try:
+                            windows.fromlist(tail)
+                        except TypeError:               # ids held as floating-point numbers
+                            windows.fromlist([int(t) for t in tail])
                         n = len(tail)
                     n += x
                 counts.append(n)

@@ -71,6 +71,14 @@ def test_sampling_with_lists_of_other_lengths(monkeypatch):
             _sampler_words(monkeypatch, params, seeds, histories, 4)
 
 
+def test_windows_from_histories_of_every_kind(monkeypatch):
+    import numpy as np
+    for history in ([4, 6], (4, 6), torch.tensor([4, 6]), np.array([4, 6]), [4.0, 6.0], np.array([4.0, 6.0]),
+                    torch.tensor([4.0, 6.0]), range(4, 8, 2)):
+        words = _sampler_words(monkeypatch, [SamplingParams()] * 2, [1, 2], [history, [1]], 2)
+        assert words[2] == [[4, 6], [1]]
+
+
 @pytest.mark.parametrize("name", ["A", "B"])
 def test_greedy_generation(model_dirs, monkeypatch, name):
     kernel_refs.install(monkeypatch)
