@@ -81,40 +81,48 @@ class Sampler:
         if len(params) not in (1, r):
             raise ValueError(f"options of {len(params)} rows for {r}")
         length = [(h.n_tokens if hasattr(h, "n_tokens") else len(h)) + x for h, x in zip(histories, pend)]
-        # rows that share an options object share its numbers (looked up within this call only)
-        options, kinds = {}, []
-        for p in params:
-            if id(p) not in options:
-                on = p.has_penalty
-                options[id(p)] = (len(options), p.repeat_last_n if on else 0,
-                                  (p.temperature, p.top_p, p.min_p, p.repetition_penalty if on else 1.0,
-                                   p.frequency_penalty if on else 0.0, p.presence_penalty if on else 0.0), p.top_k)
-            kinds.append(options[id(p)])
+        # rows that share an options object share its numbers (looked up within this call only): as many columns as objects
+        own = list({id(p): p for p in params}.values())
+        on = [p.has_penalty for p in own]
+        last = [p.repeat_last_n if x else 0 for p, x in zip(own, on)]
+        numbers = np.zeros((6, len(own)), dtype=np.float32)
+        numbers[0] = [p.temperature for p in own]
+        numbers[1] = [p.top_p for p in own]
+        numbers[2] = [p.min_p for p in own]
+        numbers[3] = 1.0
+        if any(on):
+            numbers[3] = [p.repetition_penalty if x else 1.0 for p, x in zip(own, on)]
+            numbers[4] = [p.frequency_penalty if x else 0.0 for p, x in zip(own, on)]
+            numbers[5] = [p.presence_penalty if x else 0.0 for p, x in zip(own, on)]
+        top_k = np.array([p.top_k for p in own], dtype=np.int32)
+        if len(own) == 1:
+            last = last * len(params)
+        elif len(own) < r:
+            column = {id(p): i for i, p in enumerate(own)}
+            which = [column[id(p)] for p in params]
+            numbers, top_k, last = numbers[:, which], top_k[which], [last[i] for i in which]
         width = 0
-        if any(last for _, last, _, _ in options.values()):
+        if any(on):
             if any(pend) and pending_ids is None and pending_from is None:
                 raise ValueError("penalties need the whole history: the one pending token must be given on the device")
-            width = max(1, max(min(k[1], n) for k, n in zip(kinds, length)))
+            width = max(1, max(min(k, n) for k, n in zip(last, length)))
         # the block: seven rows of floats (as their bits), two of ints, the penalties' windows, the pending tokens' places
         look_up = width > 0 and any(pend) and pending_ids is None
         words = np.empty((9 * r + r * width + (r if look_up else 0),), dtype=np.int32)
         floats = words[:7 * r].view(np.float32).reshape(7, r)
-        rows = list(options.values())
-        which = [k[0] for k in kinds] if len(rows) > 1 else 0
-        numbers = np.array([k[2] for k in rows], dtype=np.float32).T
-        floats[:3] = numbers[:3, which].reshape(3, -1)
+        floats[:3] = numbers[:3]
         floats[3] = uniforms_for(seeds, length)
-        floats[4:] = numbers[3:, which].reshape(3, -1)
-        words[7 * r:8 * r] = np.array([k[3] for k in rows], dtype=np.int32)[which]
+        floats[4:] = numbers[3:]
+        words[7 * r:8 * r] = top_k
         n_prev = words[8 * r:9 * r]
         n_prev[:] = 0
         if width:
             # the windows, row by row: -1 in the place of the pending token, the history's tail, -1 up to the width.  The
             # window's order does not matter: the pending token, if any, takes the first place.
             windows, counts, blank = array("i"), [], array("i", [-1]) * width
-            for k, h, x in zip(kinds, histories, pend):
-                known, n = k[1] - x, 0
-                if k[1]:
+            for k, h, x in zip(last, histories, pend):
+                known, n = k - x, 0
+                if k:
                     if x:
                         windows.append(-1)
                     if known > 0:

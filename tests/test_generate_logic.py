@@ -71,6 +71,16 @@ def test_sampling_with_lists_of_other_lengths(monkeypatch):
             _sampler_words(monkeypatch, params, seeds, histories, 4)
 
 
+def test_options_shared_by_rows_or_not(monkeypatch):
+    """Rows that share options objects in part, altogether or not at all hand over the same numbers."""
+    from dataclasses import replace
+    a, b, c = SamplingParams(top_k=3), SamplingParams.greedy(), SamplingParams(temperature=0.3, repeat_last_n=2)
+    seeds, histories = [1, 2, 3, 4], [[1, 2, 3], [4], [5, 6, 7], [8, 9]]
+    for params in ([a, b, a, c], [c, c, c, c], [b, a, c, SamplingParams(repeat_last_n=0)]):
+        assert _sampler_words(monkeypatch, params, seeds, histories, 4) == \
+            _sampler_words(monkeypatch, [replace(p) for p in params], seeds, histories, 4)
+
+
 def test_windows_from_histories_of_every_kind(monkeypatch):
     import numpy as np
     for history in ([4, 6], (4, 6), torch.tensor([4, 6]), np.array([4, 6]), [4.0, 6.0], np.array([4.0, 6.0]),
