@@ -578,19 +578,27 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p,
 
 }  // namespace tc
 
-// How many CTAs share one output tile when the caller does not say
+// How many CTAs share one output tile when the caller does not say.  Each part is a CTA whose ring (80 KB) holds a share of
+// W before the kernel ahead has finished; more parts cost in the cluster's summing and in x read once more.  Products
+// alone, replayed one after the other with cold weights, us with fewer / more parts:
+//   * 60 tiles and more, two or four parts.  One tile more than the GPU holds in clusters of four is a second wave (72
+//     tiles: 10.7 / 15.1), beyond 64 tokens a CTA has an SM to itself (128 tokens, 64 tiles over 2,048: 21.5 / 41.5), and over
+//     a short K the parts are too small, the more so the more tokens they hold.  16 tokens, 64 tiles: K 1,024
+//     7.3 / 7.9, 2,048 11.1 / 10.5, 8,192 30.3 / 26.6; 32 tokens: 2,048 13.8 / 13.7, 4,096 20.6 / 19.4; 64 tokens: 4,096
+//     23.0 / 22.7, 8,192 36.7 / 32.7.
+//   * few tiles, four or eight parts.  Eight over a long K, and where the tiles are so few that four parts leave most
+//     SMs without a CTA: 16 tokens, K 2,048, 2 tiles 6.6 / 6.0, 16 tiles 7.0 / 6.9, 19 tiles 7.0 / 7.8; K 3,072, 16 tiles
+//     8.3 / 7.7; 1,024: never.  32 tokens: K 2,048, 8 tiles 9.9 / 10.8; 6,144, 16 tiles 15.8 / 15.4.  (A decode step of
+//     one request with 1,024 features over 2,048 and 3,072: 1,133 -> 1,083 us.)
+static int resident_for(int bn, int splits);
+
 static int choose_splits(int n_tok, int n_out, int num_kb, int bn, int split_k) {
     int splits = split_k;
     if (splits <= 0) {
         const long tiles = (long)((n_out + tc::BM - 1) / tc::BM) * ((n_tok + bn - 1) / bn);
-        // Few tiles: parts until the CTAs' rings hold most of W before the kernel before them has finished; a ring is
-        // 80 KB, so that is what a CTA has on its way by then.  Eight parts over a long K (the down projection of a
-        // decode step), and over a shorter one too where the tiles are so few that four parts would leave most SMs
-        // without a CTA (1,024 features over 2,048 and 3,072: a decode step of one request 1,133 -> 1,083 us with 64
-        // CTAs in place of 32); 32 tiles over 4,096 are as fast with four (985 us a step of 8 requests, 995 with eight).
-        // Sixty to seventy tiles: four parts still fit as one wave of two CTAs an SM (8,192 features over 2,048, in a
-        // model of four layers: 2 % of the step).
-        splits = tiles >= 120 ? 1 : tiles > 71 ? 2 : tiles >= 60 ? 4 : (tiles < 40 && num_kb >= 128) || (tiles < 20 && num_kb >= 32) ? 8 : 4;
+        const bool eight = (tiles < 40 && num_kb >= 128) || (tiles <= 16 && num_kb >= (bn <= 16 ? 32 : 96));
+        const bool four = num_kb >= 2 * bn && 4 * tiles < resident_for(bn, 4);
+        splits = tiles >= 120 ? 1 : tiles >= 60 ? (four ? 4 : 2) : eight ? 8 : 4;
     }
     if (bn == 256) splits = 1;
     while (splits > 1 && (num_kb + splits - 1) / splits * (splits - 1) >= num_kb) splits >>= 1;  // no empty part

@@ -968,6 +968,21 @@ def test_products_with_tiles_lower_than_the_mma(n, m, k, split_k):
             assert rel_err(rest[1], rest_full[1]) < 1e-2   # the parts of the sums of squares are cut elsewhere
 
 
+@pytest.mark.parametrize("n,tiles,k,parts,other", [
+    (16, 59, 2048, 4, 2), (16, 60, 1984, 2, 4), (16, 60, 2048, 4, 2), (16, 70, 2048, 4, 2), (16, 75, 2048, 2, 4), (128, 64, 2048, 2, 4),
+    (64, 64, 4096, 2, 4), (64, 64, 8192, 4, 2), (32, 66, 2048, 2, 4), (2, 16, 2048, 8, 4), (2, 16, 1984, 4, 8), (2, 17, 2048, 4, 8),
+    (32, 8, 3072, 4, 8), (32, 8, 6144, 8, 4), (3, 39, 8192, 8, 4), (3, 119, 512, 2, 1), (3, 120, 512, 1, 2)])
+def test_parts_of_a_product(n, tiles, k, parts, other):
+    """How many CTAs share a tile at the edges of the rule: the sums have the bits of that number of parts, not of another."""
+    from inferrs_b200 import kernels as K
+    x, w = rand((n, k), torch.bfloat16, 126), rand((tiles * 128, k), torch.bfloat16, 127, scale=0.05)
+    out = {s: torch.empty((n, tiles * 128), device=dev()) for s in (0, parts, other)}
+    for s, y in out.items():
+        K.gemm_tn_tcgen05(x, w, y, s)
+    assert K.gemm_tcgen05_error() == 0
+    assert torch.equal(out[0], out[parts]) and not torch.equal(out[0], out[other])
+
+
 @pytest.mark.parametrize("n,inner,k", [(7, 10000, 136), (24, 12288, 512), (1, 15000, 64)])
 def test_gated_products_with_tiles_lower_than_the_mma(n, inner, k):
     """The gate/up form with fewer than 64 rows of each matrix per tile: the gate box of the last tile reaches into
