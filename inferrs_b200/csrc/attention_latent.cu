@@ -254,7 +254,10 @@ __host__ __device__ constexpr int lm_swizzle(int rk) { return rk % 64 == 0 ? 7 :
 // ROT: cached vectors and queries have rot.width (a multiple of 16) more numbers, which join the scores alone.
 // WARPS: 4, or 8 for two tokens: four warps then score one token each, and a warp sums an eighth of R.
 template <int NT, int TT, bool ROT, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS, WARPS == 8 ? 2 : 1)
+// Four warps have no bound on the blocks an SM holds: with one (of a single block, even) the compiler spends half as many
+// registers again on the one-token form, and steps of many rows lose the blocks that these would have been (1,000 rows of
+// 300 keys, R = 128: 31 us, with the bound 38).
+__global__ void __launch_bounds__(32 * WARPS, WARPS == 8 ? 2 : 0)
 latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, long q_head,
                             const __nv_bfloat16* __restrict__ plane, const int* __restrict__ block_table, int max_pages,
                             int page_size, int n_pages, const int* __restrict__ row_request,
@@ -521,23 +524,23 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
 }
 
 #define LM_MOST_ROT 128                // places of a rotated part that the tensor-core form takes
-static IbDeviceSet latent_mma_smem_set[2][2][17];
+#define LM_RESIDENT 296                // two blocks per SM
+static IbDeviceSet latent_mma_smem_set[2][3][17];
 
-template <int NT, int TT, bool ROT>
+template <int NT, int TT, bool ROT, int WARPS>
 static int launch_latent_mma(const void* q, long q_row, long q_head, const void* plane, const int* block_table,
                              int max_pages, int page_size, int n_pages, const int* row_request, const int* positions,
                              const int* tile_req, const int* tile_row0, const int* q_start, int n_blocks, int n_heads,
                              float scale, int window, int n_slices, void* out, long o_row, long o_head, float* ws_acc,
                              float* ws_ml, const LatentRot& rot, cudaStream_t stream) {
-    // Eight warps a block where two tokens meet and an eighth of R is whole pairs of n-tiles: see WARPS_TIMES
-    constexpr int R = 32 * NT, MR = TT * LM_ROWS, WARPS = TT == 2 && NT % 4 == 0 ? 8 : 4;
+    constexpr int R = 32 * NT, MR = TT * LM_ROWS;
     auto smem_for = [](int width, int pad) {
         return (size_t)((MR + LM_KEYS) * (R + width + pad) + MR * (LM_KEYS + pad)) * 2 + 8 * MR * sizeof(float);
     };
     const size_t smem = ROT ? smem_for(rot.width, lm_swizzle(R + rot.width) ? 0 : LM_PAD) : smem_for(0, LM_PAD);
     const size_t smem_most = smem_for(ROT ? LM_MOST_ROT : 0, LM_PAD);     // the permission is given once per device, for the most
     if (smem_most > 48 * 1024) {
-        const int e = ib_allow_dynamic_smem(latent_mma_smem_set[ROT][TT - 1][NT], latent_attention_mma_kernel<NT, TT, ROT, WARPS>,
+        const int e = ib_allow_dynamic_smem(latent_mma_smem_set[ROT][WARPS == 8 ? 2 : TT - 1][NT], latent_attention_mma_kernel<NT, TT, ROT, WARPS>,
                                             smem_most);
         if (e != IB_OK) return e;
     }
@@ -546,6 +549,26 @@ static int launch_latent_mma(const void* q, long q_row, long q_head, const void*
               (const __nv_bfloat16*)plane, block_table, max_pages, page_size, n_pages, row_request, positions, tile_req,
               tile_row0, q_start, n_heads, scale, window, n_slices, (__nv_bfloat16*)out, o_row, o_head, ws_acc, ws_ml, rot);
     return ib_launch_status();
+}
+
+// Two tokens a block: four warps, or eight where an eighth of R is whole pairs of n-tiles.  Eight finish a tile sooner, but
+// two such blocks fill an SM's registers, where three or more of four warps fit as long as the latents are short.  So
+// R = 128 and 256 take eight only while there are no more blocks than two per SM, longer latents and R = 256 with a
+// rotated part (whose shared memory leaves room for two blocks either way) always.  us with four / eight warps, 16 heads:
+//   R = 128   592 tokens 35 / 30, 1,500 107 / 117, 2,048 171 / 196; 592 behind 1,500 cached 105 / 91, 800 143 / 156
+//   R = 256   592 tokens 45 / 41, 4,096 927 / 954; 592 behind 1,500 167 / 129, 800 194 / 220; rotated, 2,048 tokens 355 / 302
+//   R = 384   2,048 tokens 432 / 355;  R = 512  505 / 433, rotated 514 / 486 (although its eight warps keep 44 bytes of
+//   registers in local memory)
+template <int NT, bool ROT, typename... Args>
+static int launch_latent_pairs(int n_blocks, int n_heads, const Args&... args) {
+    if constexpr (NT % 4 == 0) {
+        constexpr bool always = NT >= 12 || (NT == 8 && ROT);
+        if (always || (long)n_blocks * ((n_heads + LM_ROWS - 1) / LM_ROWS) <= LM_RESIDENT) return launch_latent_mma<NT, 2, ROT, 8>(args...);
+        if constexpr (!always) return launch_latent_mma<NT, 2, ROT, 4>(args...);
+        return IB_ERR_UNSUPPORTED;                       // not reached
+    } else {
+        return launch_latent_mma<NT, 2, ROT, 4>(args...);
+    }
 }
 #endif  // IB_ACT_BF16
 
@@ -602,23 +625,19 @@ IB_EXPORT int ib_latent_attention(const void* q, int q_is_f32, long q_row, long 
         // a list of tiles of up to two tokens (prompt portions, one slice): two tokens per block
         const bool pairs = tile_req != nullptr && tile_row0 != nullptr && q_start != nullptr && n_tiles > 0 && n_slices == 1;
         switch (R / 32) {
-#define IB_LATM_FORM(NT, TT, ROT, N, ...)                                                                            \
-        launch_latent_mma<NT, TT, ROT>(q, q_row, q_head, plane, block_table, max_pages, page_size, n_pages, row_request, \
-                                       positions, __VA_ARGS__, N, n_heads, scale, window, n_slices, out, o_row, o_head, \
-                                       ws_acc, ws_ml, rot, stream)
+#define IB_LATM_ARGS(N, ...)                                                                                          \
+        q, q_row, q_head, plane, block_table, max_pages, page_size, n_pages, row_request, positions, __VA_ARGS__, N, n_heads, \
+        scale, window, n_slices, out, o_row, o_head, ws_acc, ws_ml, rot, stream
+#define IB_LATM_FORM(NT, ROT)                                                                                         \
+        (pairs ? launch_latent_pairs<NT, ROT>(n_tiles, n_heads, IB_LATM_ARGS(n_tiles, tile_req, tile_row0, q_start))  \
+               : launch_latent_mma<NT, 1, ROT, 4>(IB_LATM_ARGS(n_rows, (const int*)nullptr, (const int*)nullptr, (const int*)nullptr)))
 #define IB_LATM(NT)                                                                                                  \
-        case NT:                                                                                                     \
-            if (rot_width > 0)                                                                                       \
-                e = pairs ? IB_LATM_FORM(NT, 2, true, n_tiles, tile_req, tile_row0, q_start)                         \
-                          : IB_LATM_FORM(NT, 1, true, n_rows, nullptr, nullptr, nullptr);                            \
-            else                                                                                                     \
-                e = pairs ? IB_LATM_FORM(NT, 2, false, n_tiles, tile_req, tile_row0, q_start)                        \
-                          : IB_LATM_FORM(NT, 1, false, n_rows, nullptr, nullptr, nullptr);                           \
-            break;
+        case NT: e = rot_width > 0 ? IB_LATM_FORM(NT, true) : IB_LATM_FORM(NT, false); break;
             IB_LATM(1) IB_LATM(2) IB_LATM(3) IB_LATM(4) IB_LATM(5) IB_LATM(6) IB_LATM(7) IB_LATM(8) IB_LATM(9)
             IB_LATM(10) IB_LATM(11) IB_LATM(12) IB_LATM(13) IB_LATM(14) IB_LATM(15) IB_LATM(16)
 #undef IB_LATM
 #undef IB_LATM_FORM
+#undef IB_LATM_ARGS
             default: e = IB_ERR_UNSUPPORTED;
         }
         if (e != IB_ERR_UNSUPPORTED) {

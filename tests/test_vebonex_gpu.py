@@ -463,6 +463,31 @@ def test_latent_attention_kernel(H, R, window, slices, dtype):
             at += len(rows)
 
 
+@pytest.mark.parametrize("R", [64, 128, 256, 384, 512])
+def test_latent_attention_of_two_tokens_with_four_and_eight_warps(R):
+    """A prompt of more tiles than two per SM and the same prompt in two steps of fewer: the sums are the same, whichever
+    number of warps the step's size chooses."""
+    from inferrs_b200 import kernels
+    H, page, n = 3, 16, 605
+    g = torch.Generator().manual_seed(R)
+    c = torch.randn(n, R, generator=g).to(torch.bfloat16).float()
+    plane, table = paged_latents([c], page, 45, torch.bfloat16, seed=R)
+    q = act(torch.randn(H, n, R, generator=g) * 1.5, torch.bfloat16)
+    dev = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")   # noqa: E731
+
+    def step(a, b):
+        out = torch.full((H, b - a, R), float("nan"), dtype=torch.bfloat16, device="cuda")
+        starts = list(range(0, b - a, 2))
+        kernels.latent_attention(q[:, a:b].contiguous(), plane, table, dev([0] * (b - a)), dev(list(range(a, b))), 0.6 / R ** 0.5,
+                                 None, out, 1, (dev([0] * len(starts)), dev(starts), len(starts), dev([0, b - a])))
+        return out
+
+    whole = step(0, n)
+    assert torch.equal(whole, torch.cat([step(0, 300), step(300, n)], dim=1))
+    want = latent_mix(q.float().cpu(), c, 0.6 / R ** 0.5, list(range(n)), None)
+    assert rel_err(whole, want) < 2e-2
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("R", [48, 64])
 @pytest.mark.parametrize("slices", [1, 5])
