@@ -167,24 +167,43 @@ latent_attention_kernel(const QT* __restrict__ q, long q_row, long q_head, const
     }
 }
 
-// Joins the slices of one (row, head): a thread per number, so that the few rows of a decode step have all their loads
-// under way at once.  A lane owns up to two slices' weights exp(m_s - m) (at most 64 slices), every warp all of them; the
-// sums then run over the slices in ascending order, a group of slices' numbers asked for before its weights are used
-// and without a condition (a slice without keys has left zeros and the weight 0).
-#define LJ_THREADS 128
-#define LJ_GROUP 16
+// Joins the slices of one (row, head).  A lane owns up to two slices' weights exp(m_s - m) (at most 64 slices), every warp
+// all of them; the sums then run over the slices in ascending order, a group of slices' numbers asked for before the
+// weights are known.  Bound by the trip to memory.  V = 1: a thread per number, so that the few rows of a decode step have
+// all their loads under way at once (4 rows of 16 heads, R = 512, 16 slices: 2.8 us; a warp per (row, head) 6.2).  V = 4:
+// four numbers a thread, for rows whose numbers (rows x heads x R) would take so many warps that these get in one another's
+// way.  Slices and join, us with V = 1 / 4, R = 512: 32,768 numbers 13.5 / 15.9, 98,304 15.1 / 13.5, 524,288 (64 rows, four
+// slices) 44.4 / 39.2; R = 256: 32,768 8.7 / 9.1, 131,072 20.7 / 14.9.  (A warp per (row, head) instead: 19.8, 17.9, 40.5;
+// 12.9, 17.0.)  Only the slices that there are are fetched: sixteen each time cost 64 rows of R = 512 6 us.
+#define LJ_WARPS 4
+#define LJ_MANY 40960
 
-__global__ void __launch_bounds__(LJ_THREADS) latent_attention_join_kernel(
-    const float* __restrict__ ws_acc, const float* __restrict__ ws_ml, int n_heads, int R, int n_slices,
+template <int V>
+__global__ void __launch_bounds__(32 * LJ_WARPS) latent_attention_join_kernel(
+    const float* __restrict__ ws_acc, const float* __restrict__ ws_ml, long n_items, int n_heads, int R, int n_slices,
     act_t* __restrict__ out, long o_row, long o_head) {
+    constexpr int GROUP = V == 1 ? 16 : 4;
     ib_grid_dependency_sync();
-    const int lane = threadIdx.x & 31, e = blockIdx.y * LJ_THREADS + threadIdx.x;
-    const long item = blockIdx.x;
+    const int lane = threadIdx.x & 31, per_item = (R + 32 * V - 1) / (32 * V);       // warps of a (row, head)
+    const long task = (long)blockIdx.x * LJ_WARPS + (threadIdx.x >> 5), item = task / per_item;
+    if (item >= n_items) return;
+    const int e = ((int)(task % per_item) * 32 + lane) * V;
     const float* ml = ws_ml + item * n_slices * 2;
-    const float* acc = ws_acc + item * n_slices * R + min(e, R - 1);
-    float part[LJ_GROUP];
+    const float* acc = ws_acc + item * n_slices * R + min(e, R - V);
+    float part[GROUP][V];
+    auto fetch = [&](int s0) {
 #pragma unroll
-    for (int j = 0; j < LJ_GROUP; ++j) part[j] = acc[(long)min(j, n_slices - 1) * R];
+        for (int j = 0; j < GROUP; ++j)
+            if (s0 + j < n_slices) {                     // (the same for all threads)
+                if constexpr (V == 4) {
+                    const float4 t = *reinterpret_cast<const float4*>(acc + (long)(s0 + j) * R);
+                    part[j][0] = t.x; part[j][1] = t.y; part[j][2] = t.z; part[j][3] = t.w;
+                } else {
+                    part[j][0] = acc[(long)(s0 + j) * R];
+                }
+            }
+    };
+    fetch(0);
     float ms[2], ls[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
@@ -199,18 +218,35 @@ __global__ void __launch_bounds__(LJ_THREADS) latent_attention_join_kernel(
     for (int k = 0; k < 2; ++k) w[k] = (ms[k] == -INFINITY) ? 0.0f : expf(ms[k] - m);
     const float l = ib_warp_sum(ls[0] * w[0] + ls[1] * w[1]);
     const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-    float v = 0.0f;
-    for (int s0 = 0; s0 < n_slices; s0 += LJ_GROUP) {
+    float v[V];
 #pragma unroll
-        for (int j = 0; j < LJ_GROUP; ++j) {
+    for (int c = 0; c < V; ++c) v[c] = 0.0f;
+    for (int s0 = 0; s0 < n_slices; s0 += GROUP) {
+#pragma unroll
+        for (int j = 0; j < GROUP; ++j) {
             const int s = s0 + j;
-            const float ws = __shfl_sync(0xffffffffu, s < 32 ? w[0] : w[1], s & 31);    // beyond the slices: 0
-            v = s < n_slices ? fmaf(part[j], ws, v) : v;
-        }
+            if (s < n_slices) {
+                const float ws = __shfl_sync(0xffffffffu, s < 32 ? w[0] : w[1], s & 31);
 #pragma unroll
-        for (int j = 0; j < LJ_GROUP; ++j) part[j] = acc[(long)min(s0 + LJ_GROUP + j, n_slices - 1) * R];
+                for (int c = 0; c < V; ++c) v[c] = fmaf(part[j][c], ws, v[c]);
+            }
+        }
+        if (s0 + GROUP < n_slices) fetch(s0 + GROUP);
     }
-    if (e < R) out[(item / n_heads) * o_row + (item % n_heads) * o_head + e] = ib_from_float<act_t>(v * inv);
+    act_t* dst = out + (item / n_heads) * o_row + (item % n_heads) * o_head + e;
+    if (e < R)
+#pragma unroll
+        for (int c = 0; c < V; ++c) dst[c] = ib_from_float<act_t>(v[c] * inv);
+}
+
+static int launch_latent_join(const float* ws_acc, const float* ws_ml, int n_rows, int n_heads, int R, int n_slices, void* out,
+                              long o_row, long o_head, cudaStream_t stream) {
+    const long items = (long)n_rows * n_heads;
+    const bool four = R % 4 == 0 && (uintptr_t)ws_acc % 16 == 0 && items * R > LJ_MANY;
+    const long blocks = (items * (four ? (R + 127) / 128 : (R + 31) / 32) + LJ_WARPS - 1) / LJ_WARPS;
+    ib_launch(four ? latent_attention_join_kernel<4> : latent_attention_join_kernel<1>, dim3((unsigned)blocks), 32 * LJ_WARPS, 0,
+              stream, ws_acc, ws_ml, items, n_heads, R, n_slices, (act_t*)out, o_row, o_head);
+    return ib_launch_status();
 }
 
 #if IB_ACT_BF16
@@ -642,9 +678,7 @@ IB_EXPORT int ib_latent_attention(const void* q, int q_is_f32, long q_row, long 
         }
         if (e != IB_ERR_UNSUPPORTED) {
             if (e != IB_OK || n_slices == 1) return e;
-            ib_launch(latent_attention_join_kernel, dim3((unsigned)((long)n_rows * n_heads), (R + LJ_THREADS - 1) / LJ_THREADS), LJ_THREADS, 0,
-                      stream, ws_acc, ws_ml, n_heads, R, n_slices, (act_t*)out, o_row, o_head);
-            return ib_launch_status();
+            return launch_latent_join(ws_acc, ws_ml, n_rows, n_heads, R, n_slices, out, o_row, o_head, stream);
         }
         e = IB_OK;
     }
@@ -663,7 +697,5 @@ IB_EXPORT int ib_latent_attention(const void* q, int q_is_f32, long q_row, long 
 #undef IB_LAT_R
 #undef IB_LAT
     if (e != IB_OK || n_slices == 1) return e;
-    ib_launch(latent_attention_join_kernel, dim3((unsigned)((long)n_rows * n_heads), (R + LJ_THREADS - 1) / LJ_THREADS), LJ_THREADS, 0, stream,
-              ws_acc, ws_ml, n_heads, R, n_slices, (act_t*)out, o_row, o_head);
-    return ib_launch_status();
+    return launch_latent_join(ws_acc, ws_ml, n_rows, n_heads, R, n_slices, out, o_row, o_head, stream);
 }

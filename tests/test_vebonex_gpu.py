@@ -463,6 +463,31 @@ def test_latent_attention_kernel(H, R, window, slices, dtype):
             at += len(rows)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("R", [32, 96, 160, 512])
+@pytest.mark.parametrize("slices", [2, 4, 5, 16, 17, 32, 33, 64])
+def test_latent_attention_joins_many_slices(R, slices, dtype):
+    """Up to 64 slices, some of them without keys: the join's groups, the weights of the slices beyond the 32nd, rows of
+    no whole block; and so many rows that a thread joins four numbers, with the same bits."""
+    from inferrs_b200 import kernels
+    H, page, positions = 4, 16, [2111, 1200, 70, 0]
+    g = torch.Generator().manual_seed(R + slices)
+    c = torch.randn(2112, R, generator=g).to(dtype).float()
+    plane, table = paged_latents([c], page, 140, dtype, seed=R)
+    q_lat = (torch.randn(H, len(positions), R, generator=g) * 1.5).to(dtype).float()
+    scale = 0.6 / R ** 0.5
+    for copies in (1, 160):
+        n = len(positions) * copies
+        q = act(q_lat, dtype).repeat(1, copies, 1)
+        out = torch.full((H, n, R), float("nan"), dtype=dtype, device="cuda")
+        kernels.latent_attention(q, plane, table, torch.zeros(n, dtype=torch.int32, device="cuda"),
+                                 torch.tensor(positions * copies, dtype=torch.int32, device="cuda"), scale, None, out, slices)
+        first = out if copies == 1 else first
+        assert torch.equal(out, first.repeat(1, copies, 1))
+    want = latent_mix(q_lat, c, scale, positions, None)
+    assert rel_err(first, want) < (2e-5 if dtype == torch.float32 else 2e-2)
+
+
 @pytest.mark.parametrize("R", [64, 128, 256, 384, 512])
 def test_latent_attention_of_two_tokens_with_four_and_eight_warps(R):
     """A prompt of more tiles than two per SM and the same prompt in two steps of fewer: the sums are the same, whichever
