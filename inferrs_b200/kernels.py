@@ -448,18 +448,29 @@ def linear_scan(mode: int, proj: torch.Tensor, q_col: int, k_col: int, v_col: in
 
 LATENT_TILE_TOKENS = 2      # tokens of a prompt portion that one block of the tensor-core form takes
 LATENT_TILE_KEYS = 64       # cached latents that it fetches at a time
-LATENT_SLICE_KEYS = 64     # fewest keys per slice when a row's keys are cut over several blocks
+LATENT_SLICE_KEYS = 128     # fewest keys per slice when many rows' keys are cut over several blocks
 LATENT_RESIDENT_BLOCKS = 296   # two blocks of the tensor-core form per SM
 
 
 def latent_slices(n_rows: int, n_heads: int, max_kv_len: int) -> int:
     """Into how many slices a row's keys are cut: one while the rows alone fill the machine, else as many as give
-    every SM its two blocks, each slice with at least ``LATENT_SLICE_KEYS`` keys, which is one tile of the tensor-core
-    form (inside decode steps of 4 rows behind 200 to 1,300 keys, 16 heads: 11.1 us and 2.8 us for the join; with two
-    tiles a slice 14.4 and more)."""
+    every SM its two blocks.
+
+    Up to 48 blocks of rows every slice is as many whole tiles of ``LATENT_TILE_KEYS`` keys as it takes for all slices to
+    run at once, one tile where that is possible, and no slice is left without keys.  Beyond, slices have at least
+    ``LATENT_SLICE_KEYS`` keys: with less the join costs more than the shorter chain gains, and prompts of 65 to 128 tokens
+    keep the form that takes two tokens a block.  Two tiles are cut for up to 32 blocks only.  Attention and join, us for 16
+    heads, R = 512 + 64 / 256 (in brackets with slices of at least 128 keys): 4 rows of 1,024 keys 13.5 / 8.2 (19.5 / 12.9), 16 of
+    2,048 26.2 / 16.0 with 16 slices, 28.7 / 18.1 with as many as fit, 19; 32 of 256 15.9 / 8.1 (17.4 / 10.7), 48 of 256 16.9 / 10.3
+    (17.9 / 11.3), 80 of 512 in three slices 40.3 / 21.9, in four 46.5 / 20.9; a prompt of 96 tokens 17.7 / 9.2, in two
+    slices 28.0 / 15.8."""
     blocks = n_rows * ((n_heads + 15) // 16)
     if blocks >= LATENT_RESIDENT_BLOCKS:
         return 1
+    tiles = max(1, (max_kv_len + LATENT_TILE_KEYS - 1) // LATENT_TILE_KEYS)
+    if blocks <= 32 or (blocks <= 48 and tiles > 2):
+        per_slice = -(-tiles // min(tiles, LATENT_RESIDENT_BLOCKS // blocks, 64))
+        return -(-tiles // per_slice)
     by_length = max(1, (max_kv_len + LATENT_SLICE_KEYS - 1) // LATENT_SLICE_KEYS)
     return max(1, min(by_length, (LATENT_RESIDENT_BLOCKS + blocks - 1) // blocks, 64))
 

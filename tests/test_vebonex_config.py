@@ -97,3 +97,19 @@ def test_plain_model_in_float32_agrees_with_float64():
         b = pv.forward(case, w, toks, torch.float64)
         assert float((a.double() - b).abs().max()) < 2e-4 * float(b.abs().max())
         assert float(b.std()) > 0.3          # the weights are of a size that moves the logits
+
+
+def test_slices_of_the_latent_attention():
+    """Prompts of up to 128 tokens are not cut, whatever stands beside them; up to 48 rows no slice is left without keys and
+    all slices run at once; more rows have slices of at least 128 keys."""
+    from inferrs_b200.kernels import latent_slices
+    assert [latent_slices(n, 16, n) for n in (1, 33, 64, 65, 96, 128)] == [1] * 6
+    assert [latent_slices(2 * n, 16, n) for n in (65, 128)] == [1, 1]
+    cases = [(1, 2048, 32), (4, 1024, 16), (16, 2048, 16), (32, 128, 2), (33, 128, 1), (48, 129, 3), (49, 129, 2), (48, 1024, 6),
+             (64, 1024, 5), (147, 147, 2), (295, 4096, 2), (296, 4096, 1), (1, 10 ** 6, 64), (1, 0, 1)]
+    assert [latent_slices(n, 16, kv) for n, kv, _ in cases] == [s for _, _, s in cases]
+    assert latent_slices(8, 40, 2048) == latent_slices(24, 16, 2048)
+    for rows in range(1, 49):
+        for kv in range(1, 5000, 37):
+            s, tiles = latent_slices(rows, 16, kv), -(-kv // 64)
+            assert 1 <= s <= 64 and s * rows <= 296 and (s - 1) * -(-tiles // s) < tiles
