@@ -1,7 +1,7 @@
 """Choosing the next token of every row of a step, on the device.
 
 The reference copies each row's logits to the host and samples there (inferrs/src/sampler.rs:146-357).
-Here the rows of a step are sampled together by two kernels (penalties, then selection); what crosses
+Here the rows of a step are sampled together by three kernels (penalties, rows with top-k, the others); what crosses
 to the host is one token id per row.
 """
 from __future__ import annotations
@@ -65,7 +65,7 @@ class Sampler:
         One options object, one seed or one history counts for every row; windows are those of the rows that have
         both an options object and a history of their own.
 
-        Everything the two kernels need per row goes to the device as one block of words in one copy that the
+        Everything the kernels need per row goes to the device as one block of words in one copy that the
         host does not wait for, so a step can be prepared while the one before it still runs.
         """
         r = logits.shape[0]

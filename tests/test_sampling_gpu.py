@@ -112,6 +112,32 @@ def test_top_k_over_two_passes(vocab):
         assert first[4] % 2 == 0                                # never a NaN
 
 
+@pytest.mark.parametrize("vocab", [700, 5000, 40001])
+def test_top_k_of_rows_with_little_mass(vocab):
+    """Rows in which fewer elements than k have any mass (the others masked, or too far below the largest for the
+    temperature) get the token of a top-k beyond the two-pass kernel's; with an infinite logit, or one that the temperature makes
+    infinite, it is the first such place."""
+    from inferrs_b200 import kernels as K
+    rows = 8
+    logits = _logits(rows, vocab, seed=61) * 2
+    for r in range(3):
+        logits[r, torch.arange(vocab) % (vocab // 20) != r + 1] = float("-inf")
+    logits[4, vocab // 3], logits[5, 5], logits[5, vocab - 2], logits[6, 7], logits[7, 9] = [float("inf")] * 3 + [1e38, float("inf")]
+    logits = logits.cuda()
+    temperature = torch.tensor([0.7, 1.3, 0.9, 0.002, 0.7, 1.0, 1e-4, 0.7]).cuda()
+    top_k = torch.tensor([50, 40, 512, 60, 5, 40, 4, 1], dtype=torch.int32).cuda()
+    top_p = torch.tensor([0.9, 1.0, 0.8, 1.0, 0.9, 0.9, 0.9, 1.0]).cuda()
+    min_p = torch.tensor([0.0, 0.0, 0.05, 0.0, 0.0, 0.0, 0.0, 0.1]).cuda()
+    for draw in (0.0, 0.3, 0.8, 0.999999):
+        uniform = torch.full((rows,), draw).cuda()
+        for cluster in (0, 1, 2, 8):
+            got, want = (torch.full((rows,), -5, dtype=torch.int32, device="cuda") for _ in range(2))
+            K.sample(logits, temperature, top_k, top_p, min_p, uniform, got, cluster=cluster)
+            K.sample(logits, temperature, top_k.clamp(min=600), top_p, min_p, uniform, want, cluster=cluster)
+            assert got[:4].tolist() == want[:4].tolist(), (cluster, draw)
+            assert got[4:].tolist() == [vocab // 3, 5, 7, 9], (cluster, draw)
+
+
 def test_penalties_of_long_windows():
     """A window longer than the kernel keeps in shared memory, and one just within it."""
     from inferrs_b200 import kernels as K
