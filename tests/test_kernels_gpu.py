@@ -359,6 +359,86 @@ def test_paged_attention_float32_tiles(nh, nkv, d, dv, window, keep):
     assert torch.equal(one, out)
 
 
+def _attention_64(q, k_pages, v_pages, table, row_request, positions, scale, window, head_scale=None, slopes=None, sinks=None,
+                  cap=None, keep_first=0, gate=None):
+    """Paged attention in 64 bits on the host, key by key."""
+    n, nh, d = q.shape
+    nkv, ps, dv = k_pages.shape[1], k_pages.shape[2], v_pages.shape[3]
+    dq, dk, dvv = q.double().cpu(), k_pages.double().cpu(), v_pages.double().cpu()
+    to = lambda t: None if t is None else t.double().cpu()   # noqa: E731
+    head_scale, slopes, sinks, gate = to(head_scale), to(slopes), to(sinks), to(gate)
+    out = torch.zeros((n, nh, dv), dtype=torch.float64)
+    for r in range(n):
+        pos, req = int(positions[r]), int(row_request[r])
+        lo = 0 if not window else max(0, pos - window + 1) if window > 0 else pos // -window * -window
+        js = [j for j in range(pos + 1) if j >= lo or j < keep_first]
+        if not js:
+            continue
+        pages, slots = table[req, [j // ps for j in js]].cpu().long(), torch.tensor([j % ps for j in js])
+        distance = pos - torch.tensor(js, dtype=torch.float64)
+        for h in range(nh):
+            kv = h // (nh // nkv)
+            s = dk[pages, kv, slots] @ dq[r, h] * scale
+            s = s if head_scale is None else s * head_scale[h]
+            s = s if slopes is None else s - slopes[h] * distance
+            s = cap * torch.tanh(s / cap) if cap else s
+            s = s if sinks is None else torch.cat([s, sinks[h:h + 1]])
+            out[r, h] = torch.softmax(s, 0)[:len(js)] @ dvv[pages, kv, slots]
+            if gate is not None:
+                out[r, h] *= torch.sigmoid(gate[r, h])
+    return out.reshape(n, nh * dv)
+
+
+@pytest.mark.parametrize("nh,nkv,d,dv,window,with_", [
+    (4, 4, 128, 128, None, ""), (8, 4, 64, 96, -48, "slopes head_scale"), (12, 3, 32, 64, 40, "cap sinks keep gate"),
+    (14, 2, 64, 64, None, "slopes gate"), (16, 2, 20, 128, -33, "head_scale sinks cap"), (24, 2, 36, 32, None, "slopes head_scale gate"),
+    (32, 1, 64, 64, 50, "slopes keep")])
+def test_float32_attention_does_not_depend_on_the_step(nh, nkv, d, dv, window, with_):
+    """A token's 32-bit attention has the same bits whatever stands beside it in the step: prompts, short runs and single
+    tokens together, each request and each token in a step of its own, tokens in any order, a few and many single tokens
+    (which differ in how many tiles of keys a block takes at a time), a place without a key.  Against 64 bits: a product of
+    two sums of n terms, within n 2^-23 of the largest value."""
+    from inferrs_b200 import kernels as K
+    ps, lens, new = 8, [300, 17, 64, 1, 139, 40, 200, 90, 12], [70, 17, 1, 1, 9, 3, 2, 16, 12]
+    table, positions, row_request, k_pages, v_pages = _paged_setup(torch.float32, nkv, max(d, dv), ps, lens, new, 90)
+    k_pages, v_pages = k_pages[..., :d].contiguous(), v_pages[..., :dv].contiguous()
+    positions[18] = -1                                   # a row that sees nothing
+    n, opt = sum(new), {}
+    per_head = {name: rand((nh,), torch.float32, 91 + i).abs() * f for i, (name, f) in
+                enumerate([("head_scale", 1.0), ("slopes", 0.05), ("sinks", 1.0)]) if name in with_}
+    gate = rand((n, nh), torch.float32, 95) if "gate" in with_ else None
+    opt = dict(per_head, keep_first=5 if "keep" in with_ else 0, cap=7.0 if "cap" in with_ else None)
+    q = rand((n, nh, d), torch.float32, 96)
+
+    def step(rows, requests=None):
+        """The rows of the step, each belonging to its request (or to one of its own)."""
+        rows = torch.as_tensor(rows, device=dev())
+        out = torch.full((len(rows), nh * dv), float("nan"), device=dev())
+        kept = torch.unique(row_request[rows])
+        req = torch.searchsorted(kept, row_request[rows]).int()
+        tables = table[kept.long()].contiguous()
+        if requests == "own":
+            tables, req = table[row_request[rows].long()].contiguous(), torch.arange(len(rows), dtype=torch.int32, device=dev())
+        K.paged_attention_generic(q[rows].contiguous(), k_pages, v_pages, tables, req, positions[rows].contiguous(), d ** -0.5,
+                                  window, out, **opt, gate=None if gate is None else gate[rows].contiguous())
+        return out
+
+    whole = step(list(range(n)))
+    want = _attention_64(q, k_pages, v_pages, table, row_request, positions, d ** -0.5, window, gate=gate, **opt)
+    err = (whole.double().cpu() - want).abs().max().item()
+    assert err <= (max(lens) + d) * 2.0 ** -23 * float(v_pages.abs().max())
+    starts = [0] + torch.tensor(new).cumsum(0).tolist()
+    for a, b in zip(starts, starts[1:]):                 # every request by itself
+        assert torch.equal(step(list(range(a, b))), whole[a:b]), a
+    for r in list(range(0, n, 7)) + [17, 18, 19]:        # tokens by themselves
+        assert torch.equal(step([r]), whole[r:r + 1]), r
+    order = torch.randperm(n, generator=torch.Generator().manual_seed(97)).tolist()
+    assert torch.equal(step(order), whole[torch.tensor(order, device=dev())])
+    for copies in (1, 5, 12):                            # single tokens, up to more than a thousand
+        rows = list(range(n)) * copies
+        assert torch.equal(step(rows, "own"), whole.repeat(copies, 1)), copies
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("n,m,k", [(70, 130, 100), (1, 517, 96), (64, 64, 16), (129, 65, 33)])
 def test_gemm_tn_simt(dtype, n, m, k):
