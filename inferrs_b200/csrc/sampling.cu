@@ -121,8 +121,9 @@ IB_EXPORT int ib_argmax(const float* logits, int* out, int n_rows, int vocab, lo
 //   frequency:  logit -= f * (times seen);  presence: logit -= q  (seen at least once).
 // prev [rows, max_prev] holds each row's window of previous tokens, n_prev[row] of them valid.
 // ---------------------------------------------------------------------------
-// A window's tokens are read into shared memory first (up to PEN_WINDOW of them; a longer window stays where it is): every
-// token is compared with all others.  64 rows of 64 tokens: 3.7 us, with every comparison read from global memory 35.
+// A window's tokens are read into shared memory first (up to PEN_WINDOW of them): every token is compared with all others.  64
+// rows of 64 tokens: 3.7 us, with every comparison read from global memory 35.  A longer window stays where it is, and a token
+// stops at its first occurrence before it: 9,000 tokens of 50 kinds 0.4 ms, with all comparisons 4.1.
 #define PEN_WINDOW 4096
 
 __global__ void penalties_kernel(float* __restrict__ logits, long ld, int vocab, const int* __restrict__ prev,
@@ -137,7 +138,8 @@ __global__ void penalties_kernel(float* __restrict__ logits, long ld, int vocab,
     if (n <= 0 || (!use_rp && !use_fp)) return;
     const int* p = prev + (long)row * max_prev;
     __shared__ int window[PEN_WINDOW];
-    if (n <= PEN_WINDOW) {
+    const bool near = n <= PEN_WINDOW;
+    if (near) {
         for (int i = threadIdx.x; i < n; i += blockDim.x) window[i] = p[i];
         __syncthreads();
         p = window;
@@ -147,10 +149,16 @@ __global__ void penalties_kernel(float* __restrict__ logits, long ld, int vocab,
         const int id = p[i];
         if (id < 0 || id >= vocab) continue;
         int before = 0, count = 0;
+        if (near) {
 #pragma unroll 8
-        for (int j = 0; j < n; ++j) {
-            count += (p[j] == id);
-            before += (p[j] == id && j < i);
+            for (int j = 0; j < n; ++j) {
+                count += (p[j] == id);
+                before += (p[j] == id && j < i);
+            }
+        } else {
+            for (int j = 0; j < i && !before; ++j) before = (p[j] == id);
+            if (!before)
+                for (int j = i; j < n; ++j) count += (p[j] == id);
         }
         if (before) continue;  // the first occurrence's thread updates the logit: no two threads share one
         float v = l[id];
