@@ -177,14 +177,13 @@ struct Share {
         }
     }
 
-    // dimensions d0 .. d0 + dims - 1 of every head to `so`, a head's row ld numbers behind the one before it
-    __device__ __forceinline__ void put(float* so, int ld, int d0, int dims, int lane, int G) const {
+    // the heads' sums to `so`, a head's row ld numbers behind the one before it
+    __device__ __forceinline__ void put(float* so, int ld, int lane, int G) const {
 #pragma unroll
         for (int n = 0; n < D / 16; ++n)
-            if (n * 16 >= d0 && n * 16 < d0 + dims)
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (head(lane, e & 1) < G) so[head(lane, e & 1) * ld + n * 16 - d0 + (lane >> 2) + 8 * (e >> 1)] = o[n][e];
+            for (int e = 0; e < 4; ++e)
+                if (head(lane, e & 1) < G) so[head(lane, e & 1) * ld + n * 16 + (lane >> 2) + 8 * (e >> 1)] = o[n][e];
     }
 };
 
@@ -301,15 +300,14 @@ struct Share<OPTIONS, false> {
         }
     }
 
-    __device__ __forceinline__ void put(float* so, int ld, int d0, int dims, int lane, int G) const {
+    __device__ __forceinline__ void put(float* so, int ld, int lane, int G) const {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int head = (lane >> 2) + 8 * h;
             if (head >= G) continue;
 #pragma unroll
             for (int n = 0; n < D / 8; ++n)
-                if (n * 8 >= d0 && n * 8 < d0 + dims)
-                    *reinterpret_cast<float2*>(so + head * ld + n * 8 - d0 + 2 * (lane & 3)) = make_float2(o[n][2 * h], o[n][2 * h + 1]);
+                *reinterpret_cast<float2*>(so + head * ld + n * 8 + 2 * (lane & 3)) = make_float2(o[n][2 * h], o[n][2 * h + 1]);
         }
     }
 };
@@ -466,7 +464,7 @@ __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constan
     float* sl = sm + 4 * 16;                                  // [4][16]
     if (warp < 4) {
         mine.close(lane, warp, G, sm, sl);
-        mine.put(so + warp * 16 * LD, LD, 0, D, lane, G);
+        mine.put(so + warp * 16 * LD, LD, lane, G);
     }
     __syncthreads();
     __nv_bfloat16* const out_row = P.out + row * P.opt.out_ld;

@@ -9,9 +9,9 @@
 //   * tiles: BM x BN outputs per CTA, TM x TN per thread, k in blocks of 16 through two shared buffers stored
 //     transposed, so that a thread's operands of one k are 16-byte reads.  Bound by the multiply-adds; two rows'
 //     chains go through one packed instruction (fma.rn.f32x2), which rounds each half as fmaf does.
-//   * rows: up to 16 rows.  Bound by streaming w (and, for few outputs, by the chain itself: four cycles per k).  A ring
+//   * rows: up to 32 rows.  Bound by streaming w (and, for few outputs, by the chain itself: four cycles per k).  A ring
 //     of cp.async stages keeps w's bytes in flight, the first of them asked for before the kernel before this one
-//     has ended; a thread owns one output feature and up to four rows.
+//     has ended; a thread owns one output feature and up to eight rows.
 #include "common.cuh"
 
 namespace simt {
@@ -295,8 +295,8 @@ static int launch_rows(const Product& p) {
     const size_t share = SM_BYTES / ((size_t)((grid.x * (long)grid.z + 147) / 148) + 1);
     size_t smem = (size_t)STAGES * (FT + RT) * (KT + 4) * sizeof(float);
     if (smem < share) smem = share;
-    ib_launch(rows_kernel<RT, FT, RPT, KT, STAGES>, grid, ROWS_THREADS, smem, p.stream, (const float*)p.x, (const float*)p.w, (float*)p.y, p.n_rows, p.n_out, p.k_dim, p.ldx, p.ldw, p.ldy, p.bx,
-              p.bw, p.by);
+    ib_launch(rows_kernel<RT, FT, RPT, KT, STAGES>, grid, ROWS_THREADS, smem, p.stream, (const float*)p.x, (const float*)p.w,
+              (float*)p.y, p.n_rows, p.n_out, p.k_dim, p.ldx, p.ldw, p.ldy, p.bx, p.bw, p.by);
     return ib_launch_status();
 }
 
