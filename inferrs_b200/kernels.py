@@ -458,12 +458,12 @@ def latent_slices(n_rows: int, n_heads: int, max_kv_len: int) -> int:
 
     Up to 48 blocks of rows every slice is as many whole tiles of ``LATENT_TILE_KEYS`` keys as it takes for all slices to
     run at once, one tile where that is possible, and no slice is left without keys.  Beyond, slices have at least
-    ``LATENT_SLICE_KEYS`` keys: with less the join costs more than the shorter chain gains, and prompts of 65 to 128 tokens
-    keep the form that takes two tokens a block.  Two tiles are cut for up to 32 blocks only.  Attention and join, us for 16
-    heads, R = 512 + 64 / 256 (in brackets with slices of at least 128 keys): 4 rows of 1,024 keys 13.5 / 8.2 (19.5 / 12.9), 16 of
-    2,048 26.2 / 16.0 with 16 slices, 28.7 / 18.1 with as many as fit, 19; 32 of 256 15.9 / 8.1 (17.4 / 10.7), 48 of 256 16.9 / 10.3
-    (17.9 / 11.3), 80 of 512 in three slices 40.3 / 21.9, in four 46.5 / 20.9; a prompt of 96 tokens 17.7 / 9.2, in two
-    slices 28.0 / 15.8."""
+    ``LATENT_SLICE_KEYS`` keys, since the join then costs what the shorter chain gains, and prompts of 65 to 128 tokens keep the
+    form that takes two tokens a block.  Two tiles are cut for up to 32 blocks only.  Attention and join, us for 16 heads,
+    R = 512 + 64 / 256, in brackets with slices of at least 128 keys: 4 rows of 1,000 keys 13.5 / 8.2 (16.4 / 10.2), 32 of 256
+    15.8 / 8.3 (17.0 / 10.3), 48 of 256 17.2 / 10.4 (20.0 / 10.9), 48 of 2,048 in six slices 52.7 / 36.5, in seven 58.3 / 35.6; 64
+    tokens behind 1,936 cached in five 53.5 / 44.3, in four 55.9 / 42.5; a prompt of 96 tokens 17.6 / 8.8, in two slices
+    16.9 / 11.0."""
     blocks = n_rows * ((n_heads + 15) // 16)
     if blocks >= LATENT_RESIDENT_BLOCKS:
         return 1
