@@ -180,16 +180,18 @@ latent_attention_kernel(const QT* __restrict__ q, long q_row, long q_head, const
 
 template <int V>
 __global__ void __launch_bounds__(32 * LJ_WARPS) latent_attention_join_kernel(
-    const float* __restrict__ ws_acc, const float* __restrict__ ws_ml, long n_items, int n_heads, int R, int n_slices,
+    const float* __restrict__ ws_acc, const float* __restrict__ ws_ml, unsigned n_items, int n_heads, int R, int n_slices,
     act_t* __restrict__ out, long o_row, long o_head) {
     constexpr int GROUP = V == 1 ? 16 : 4;
+    // (the divisions in 32 bits, and before the wait)
+    const unsigned lane = threadIdx.x & 31, per_item = (R + 32 * V - 1) / (32 * V);  // warps of a (row, head)
+    const unsigned task = blockIdx.x * LJ_WARPS + (threadIdx.x >> 5), item = task / per_item;
+    const int e = (int)((task % per_item) * 32 + lane) * V;
+    const float* ml = ws_ml + (long)item * n_slices * 2;
+    const float* acc = ws_acc + (long)item * n_slices * R + min(e, R - V);
+    act_t* dst = out + (long)(item / n_heads) * o_row + (long)(item % n_heads) * o_head + e;
     ib_grid_dependency_sync();
-    const int lane = threadIdx.x & 31, per_item = (R + 32 * V - 1) / (32 * V);       // warps of a (row, head)
-    const long task = (long)blockIdx.x * LJ_WARPS + (threadIdx.x >> 5), item = task / per_item;
     if (item >= n_items) return;
-    const int e = ((int)(task % per_item) * 32 + lane) * V;
-    const float* ml = ws_ml + item * n_slices * 2;
-    const float* acc = ws_acc + item * n_slices * R + min(e, R - V);
     float part[GROUP][V];
     auto fetch = [&](int s0) {
 #pragma unroll
@@ -207,10 +209,10 @@ __global__ void __launch_bounds__(32 * LJ_WARPS) latent_attention_join_kernel(
     float ms[2], ls[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        const int s = min(lane + 32 * k, n_slices - 1);
+        const int mine = (int)lane + 32 * k, s = min(mine, n_slices - 1);
         ms[k] = ml[s * 2];
         ls[k] = ml[s * 2 + 1];
-        if (lane + 32 * k >= n_slices) { ms[k] = -INFINITY; ls[k] = 0.0f; }
+        if (mine >= n_slices) { ms[k] = -INFINITY; ls[k] = 0.0f; }
     }
     const float m = ib_warp_max(fmaxf(ms[0], ms[1]));
     float w[2];
@@ -233,7 +235,6 @@ __global__ void __launch_bounds__(32 * LJ_WARPS) latent_attention_join_kernel(
         }
         if (s0 + GROUP < n_slices) fetch(s0 + GROUP);
     }
-    act_t* dst = out + (item / n_heads) * o_row + (item % n_heads) * o_head + e;
     if (e < R)
 #pragma unroll
         for (int c = 0; c < V; ++c) dst[c] = ib_from_float<act_t>(v[c] * inv);
@@ -245,7 +246,7 @@ static int launch_latent_join(const float* ws_acc, const float* ws_ml, int n_row
     const bool four = R % 4 == 0 && (uintptr_t)ws_acc % 16 == 0 && items * R > LJ_MANY;
     const long blocks = (items * (four ? (R + 127) / 128 : (R + 31) / 32) + LJ_WARPS - 1) / LJ_WARPS;
     ib_launch(four ? latent_attention_join_kernel<4> : latent_attention_join_kernel<1>, dim3((unsigned)blocks), 32 * LJ_WARPS, 0,
-              stream, ws_acc, ws_ml, items, n_heads, R, n_slices, (act_t*)out, o_row, o_head);
+              stream, ws_acc, ws_ml, (unsigned)items, n_heads, R, n_slices, (act_t*)out, o_row, o_head);
     return ib_launch_status();
 }
 
