@@ -136,7 +136,7 @@ class Sampler:
                     n += x
                 counts.append(n)
                 if n < width:
-                    windows.extend(blank[:width - n])
+                    windows.extend(blank[:width - n] if n else blank)
             prev = words[9 * r:9 * r + r * width]
             prev[:len(windows)] = windows
             prev[len(windows):] = -1
