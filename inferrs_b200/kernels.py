@@ -880,6 +880,59 @@ def gemm_tn_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act_dtype:
     _check(code, "gemm_tn_simt")
 
 
+_SPLIT_LIB = None
+
+
+def _split_lib():
+    global _SPLIT_LIB
+    if _SPLIT_LIB is None:
+        lib = load_library("gemm_f32")
+        lib.ib_gemm_tn_split.argtypes = [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_int, c_int, c_int, c_int,
+                                         c_int, c_void_p]
+        lib.ib_gemm_tn_split.restype = c_int
+        lib.ib_gemm_split_set_pdl.argtypes = [c_int]
+        lib.ib_gemm_split_set_pdl.restype = None
+        lib.ib_gemm_split_error.argtypes = [c_int]
+        lib.ib_gemm_split_error.restype = c_int
+        lib.ib_gemm_split_error_async.argtypes = [c_void_p, c_void_p]
+        lib.ib_gemm_split_error_async.restype = c_int
+        _SPLIT_LIB = lib
+    return _SPLIT_LIB
+
+
+SPLIT_MIN_K = 512    # see gemm_split_supported
+
+
+def gemm_split_supported(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> bool:
+    """Whether a product of 32-bit tensors runs on the tensor cores in pieces (csrc/gemm_split_tcgen05.cu).  The rule asks
+    nothing of the number of rows, so that a row's bits stay those of the row alone.  Below 512 of k a chain of fused
+    multiply-adds is as fast and as exact; TMA wants bases and rows on 16 bytes."""
+    return (x.dtype == w.dtype == out.dtype == torch.float32 and x.shape[1] >= SPLIT_MIN_K and x.shape[1] % 4 == 0
+            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_tn_split(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, splits: int = 0, tile_rows: int = 0):
+    """out = x @ w.T for float32 tensors on the tensor cores: every number as the exact sum of three bfloat16 pieces,
+    the six largest of the nine products of pieces, sums in float32 (closer to 64 bits than a chain of fused
+    multiply-adds).  ``splits`` CTAs (1, 2, 4, 8) share a tile of ``tile_rows`` rows of w; 0 lets the library choose.
+    Neither changes a bit of the result."""
+    for name, t in (("x", x), ("w", w), ("out", out)):
+        _need(t, name, (torch.float32,), 2)
+    n, k = x.shape
+    m = w.shape[0]
+    if w.shape[1] != k or out.shape != (n, m):
+        raise KernelError(f"gemm: x {tuple(x.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    code = _split_lib().ib_gemm_tn_split(_p(x), k, _p(w), k, _p(out), m, n, m, k, splits, tile_rows, _stream())
+    if code == -1:
+        raise KernelError(f"gemm_tn_split: K={k} must be a multiple of 4 and the bases 16-byte aligned")
+    _check(code, "gemm_tn_split")
+
+
+def gemm_split_error(reset: bool = True) -> int:
+    """0, or the code of the first bounded wait that ran out in a 32-bit product (synchronises with the device)."""
+    return _split_lib().ib_gemm_split_error(int(reset))
+
+
 def argmax(logits: torch.Tensor, out: torch.Tensor, act_dtype: torch.dtype = torch.float32):
     """out[r] = index of the largest logit of row r (lowest index among equals).  ``act_dtype`` only
     selects which of the two builds of the kernel library serves the call."""
@@ -2280,6 +2333,8 @@ def set_pdl(on: bool, act_dtype: torch.dtype = torch.bfloat16):
     lib.ib_set_pdl(int(bool(on)))
     if act_dtype == torch.bfloat16:
         gemm_tcgen05_set_pdl(on)
+    else:
+        _split_lib().ib_gemm_split_set_pdl(int(bool(on)))
 
 
 # up to this many rows the own tcgen05 product is the faster one in a decode step (the environment variable is
@@ -2322,6 +2377,7 @@ def error_words_async(host: torch.Tensor, act_dtype: torch.dtype):
     if act_dtype == torch.bfloat16:
         calls += [_gemm_lib().ib_gemm_tcgen05_error_async, _gemm_lib().ib_gemm_chain_error_async]
     else:
+        calls.append(_split_lib().ib_gemm_split_error_async)     # in the place of the bfloat16 products
         host[len(calls):len(ERROR_WORDS)] = 0
     for i, fn in enumerate(calls):
         code = fn(at + 4 * i, stream)
@@ -2337,11 +2393,14 @@ def reset_error_words(act_dtype: torch.dtype) -> dict:
     if row is not None:
         found[ERROR_WORDS[0]] = row + 1
     if act_dtype == torch.bfloat16:
-        for name, fn in zip(ERROR_WORDS[1:], (attention_tcgen05_error, attention_pair_tcgen05_error,
-                                              attention_decode_error, gemm_tcgen05_error, gemm_chain_error)):
-            v = fn(True)
-            if v:
-                found[name] = v
+        words = list(zip(ERROR_WORDS[1:], (attention_tcgen05_error, attention_pair_tcgen05_error,
+                                           attention_decode_error, gemm_tcgen05_error, gemm_chain_error)))
+    else:
+        words = [(ERROR_WORDS[4], gemm_split_error)]
+    for name, fn in words:
+        v = fn(True)
+        if v:
+            found[name] = v
     for counters in _DECODE_COUNTERS.values():
         counters.zero_()
     return found
