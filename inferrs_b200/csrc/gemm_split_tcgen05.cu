@@ -509,26 +509,23 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p,
 struct Cut { int splits, tile_rows; };
 
 static Cut choose_cut(int n_tok, int n_out, int blocks, int bn) {
-    const int tiles_tok = (n_tok + bn - 1) / bn;
-    // CTAs that run at a time (clusters want their SMs in one part of the chip, so fewer with larger ones)
-    const int resident[4] = {148, 148, 142, 132};            // splits 1, 2, 4, 8
-    Cut best = {1, BM};
+    const long tiles = (long)((n_out + BM - 1) / BM) * ((n_tok + bn - 1) / bn);
+    // CTAs that run at a time, per CTA of an SM (clusters want their SMs in one part of the chip: fewer with larger ones)
+    const int resident[4] = {148, 148, 136, 120};            // splits 1, 2, 4, 8
     if (bn <= 16) {
-        // few tokens: the bytes of W count, so every SM holds its two CTAs where the product allows it
-        for (int l = 3; l > 0; --l) {
-            const int tiles = resident[l] * 2 >> l;
-            int rows = ((n_out + tiles - 1) / tiles + 7) / 8 * 8;
-            if (rows < 16) rows = 16;
-            if (rows <= BM) return {1 << l, rows};
-        }
-        return best;
+        // as many parts as the GPU holds at once, two CTAs an SM (1 to 16 tokens, us: 1,024 features over 2,048 eight 8.0, four
+        // 10.1; over 3,072 9.9; 6,144 over 1,024 four 10.9, eight 14.2; lower tiles, so that more SMs have one, lose: 1,024
+        // over 3,072 in 128 / 96 / 32 rows 9.9 / 10.3 / 11.7)
+        for (int l = 3; l > 0; --l)
+            if (tiles << l <= 2 * (resident[l] + 12)) return {1 << l, BM};
+        return {1, BM};
     }
     // else the time of the fullest SM: its blocks, and what every CTA pays at its ends
+    Cut best = {1, BM};
     float least = 0.0f;
     for (int l = 0; l < 4; ++l) {
-        const long ctas = (long)((n_out + BM - 1) / BM) * tiles_tok << l;
-        const long waves = (ctas + resident[l] - 1) / resident[l];
-        const float t = waves * ((float)((blocks + (1 << l) - 1) >> l) * 1.0f + 5.0f + l);
+        const long waves = ((tiles << l) + resident[l] - 1) / resident[l];
+        const float t = waves * ((float)((blocks + (1 << l) - 1) >> l) * 1.2f + 5.0f + l);
         if (l == 0 || t < least) { least = t; best.splits = 1 << l; }
     }
     return best;

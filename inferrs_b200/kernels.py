@@ -1134,7 +1134,10 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, act_dtype: torch.dtype, sink: 
                               f"ask folded_norm_supported first")
         return gemm_tn_tcgen05(x, w, out, sink=sink)
     if act_dtype == torch.float32 or w.dtype == torch.float32:
-        gemm_tn_simt(x, w, out, act_dtype)
+        if act_dtype == torch.float32 and gemm_split_supported(x, w, out):
+            gemm_tn_split(x, w, out)
+        else:
+            gemm_tn_simt(x, w, out, act_dtype)
     elif x.shape[0] <= TCGEN05_MAX_TOKENS and tcgen05_gemm_supported(x, w):
         gemm_tn_tcgen05(x, w, out)
     else:

@@ -61,3 +61,14 @@ def test_split_product_of_infinities_nan_and_the_range_ends():
     want = x[rows].double() @ w[cols].double().t()
     assert bool(((out[rows][:, cols].double() - want).abs() <= bound(x[rows], w[cols])).all())
 
+
+def test_linear_takes_the_split_product_by_its_width_alone():
+    from inferrs_b200 import kernels as K
+    for k in (508, 512, 514, 1024):
+        x, w = rand((70, k), 5), rand((96, k), 6)
+        out = [torch.empty((n, 96), device="cuda") for n in (70, 3)]
+        for o in out:
+            K.linear(x[:o.shape[0]], w, o, torch.float32)
+        ref = torch.empty((70, 96), device="cuda")
+        (K.gemm_tn_split if k >= 512 and k % 4 == 0 else lambda a, b, c: K.gemm_tn_simt(a, b, c, torch.float32))(x, w, ref)
+        assert torch.equal(out[0], ref) and torch.equal(out[1], ref[:3])
