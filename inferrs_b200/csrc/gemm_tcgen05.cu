@@ -105,6 +105,7 @@ struct Params {
     const void* sink_w;
     int sink_w_is_f32;
     float* out_ssq;
+    long by;         // a batch of products (kernel without clusters): y of product b starts by elements after that of b - 1
 };
 
 constexpr int SSQ_LD = 32;    // tokens per part of a list of sums of squares (the folded forms take up to 32 tokens)
@@ -578,6 +579,296 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p,
 
 }  // namespace tc
 
+// ---- few rows, small weights: no clusters -------------------------------------------------------------------------
+// A product of up to sixteen tokens and weights of a few megabytes takes 1 to 4 us of bytes, and the kernel above 5 to 6 us of
+// everything else: the accumulator's way through tensor memory, the cluster's exchange of partial sums, three meetings
+// of its warps.  Here a CTA owns R rows of W and all of K, so nothing crosses CTAs, and each of its eight warps owns every
+// eighth 64 of k with a ring of its own: lane 0 asks for W's and x's boxes by TMA (W's before the kernel ahead has ended, as
+// far as the ring goes: for the small products that is all of W), the warp multiplies them with mma.sync, W as the 16
+// rows and the tokens as the 8 columns.  The warps meet once, to add up their sums in the order of their numbers.
+//
+// Within a 128-byte row of a swizzled stage, lane (g, t) of a warp takes the 16-byte pieces 2 t and 2 t + 1 of rows g and
+// g + 8: the same permutation of k for W and x, so the products are whole, and the eight lanes of a phase meet all
+// 32 banks.
+namespace rows {
+
+using namespace sm100;
+
+constexpr int WARPS = 8, THREADS = 32 * WARPS;
+constexpr int BK = 64;
+constexpr int SMEM_MOST = 113 * 1024;             // two CTAs per SM: the next product fetches while this one ends
+
+template <int R, bool GATED, int TOK> struct Shape {
+    static constexpr int W_BYTES = R * 128, X_BYTES = TOK * 128;
+    static constexpr int STAGE = (GATED ? 2 : 1) * W_BYTES + X_BYTES;
+    static constexpr int FIT = (SMEM_MOST - 640) / (WARPS * STAGE);
+    static constexpr int STAGES = FIT > 8 ? 8 : FIT;   // per warp
+    static constexpr int TILES = (R + 15) / 16;   // of 16 rows, of each matrix
+    static constexpr int SUMS = WARPS * TOK * R * (GATED ? 2 : 1) * 4;    // the warps' sums, over the rings
+    static constexpr size_t smem = (size_t)WARPS * STAGES * STAGE + WARPS * STAGES * 8 + TOK * 4;
+    static_assert(STAGES >= 2 && SUMS + TOK * R * 4 <= WARPS * STAGES * STAGE && smem <= SMEM_MOST, "");
+};
+
+__device__ __forceinline__ void mma16816(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0,
+                                         unsigned b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// BATCH: blockIdx.y numbers the products of a batch (plain ones); x, w and y of product b lie a stride after those of b - 1.
+template <int R, bool GATED, int TOK, bool BATCH>
+__global__ void __launch_bounds__(THREADS, 2) rows_kernel(const __grid_constant__ CUtensorMap map_w,
+                                                          const __grid_constant__ CUtensorMap map_x, const tc::Params p) {
+    using S = Shape<R, GATED, TOK>;
+    constexpr int MATS = GATED ? 2 : 1, TILES = S::TILES, NT = TOK / 8;
+    extern __shared__ __align__(1024) unsigned char rows_smem[];             // (the swizzle counts from multiples of 1 KB)
+    unsigned char* smem = rows_smem;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned char* ring = smem + warp * S::STAGES * S::STAGE;
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + WARPS * S::STAGES * S::STAGE);
+    const unsigned full0 = smem_u32(bars + warp * S::STAGES);
+    float* inv_s = reinterpret_cast<float*>(bars + WARPS * S::STAGES);       // [TOK] row scales
+    const int f0 = blockIdx.x * R;
+    const int n_mine = (p.num_kb - warp + WARPS - 1) / WARPS;                // stages warp, warp + 8, ... of K
+
+    ib_grid_dependency_launch();
+    auto load_w = [&](int i, int s) {
+        const int k0 = (warp + i * WARPS) * BK;
+        mbar_expect_tx(full0 + 8 * s, S::STAGE);
+        if (BATCH) tma_load_3d(smem_u32(ring + s * S::STAGE), &map_w, k0, f0, blockIdx.y, full0 + 8 * s);
+        else tma_load_2d(smem_u32(ring + s * S::STAGE), &map_w, k0, f0, full0 + 8 * s);
+        if (GATED) tma_load_2d(smem_u32(ring + s * S::STAGE + S::W_BYTES), &map_w, k0, p.inner + f0, full0 + 8 * s);
+    };
+    auto load_x = [&](int i, int s) {
+        const unsigned dst = smem_u32(ring + s * S::STAGE + MATS * S::W_BYTES);
+        if (BATCH) tma_load_3d(dst, &map_x, (warp + i * WARPS) * BK, 0, blockIdx.y, full0 + 8 * s);
+        else tma_load_2d(dst, &map_x, (warp + i * WARPS) * BK, 0, full0 + 8 * s);
+    };
+    const int head = n_mine < S::STAGES ? n_mine : S::STAGES;
+    if (lane == 0) {
+        for (int s = 0; s < S::STAGES; ++s) mbar_init(full0 + 8 * s, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        for (int i = 0; i < head; ++i) load_w(i, i);                         // weights: no kernel writes them
+    }
+    // what this thread will finish: output idx is token idx / R, row idx % R
+    constexpr int OUTS = (TOK * R + THREADS - 1) / THREADS;
+    float w_sink[OUTS], old[OUTS];
+#pragma unroll
+    for (int o = 0; o < OUTS; ++o) {
+        const int f = f0 + ((int)threadIdx.x + o * THREADS) % R;
+        w_sink[o] = old[o] = 0.0f;
+        if (!GATED && p.residual != nullptr && f < p.n_out) w_sink[o] = tc::sink_weight(p, f);
+    }
+    ib_grid_dependency_wait();
+    if (lane == 0)
+        for (int i = 0; i < head; ++i) load_x(i, i);
+    __syncwarp();                                                            // the barriers are set up
+    if (!GATED && p.residual != nullptr) {
+#pragma unroll
+        for (int o = 0; o < OUTS; ++o) {
+            const int idx = (int)threadIdx.x + o * THREADS, tok = idx / R, f = f0 + idx % R;
+            if (idx < TOK * R && tok < p.n_tok && f < p.n_out) old[o] = p.residual[(long)tok * p.ld_res + f];
+        }
+    }
+    if (p.in_ssq != nullptr) {
+        // a warp per token: its lanes add up every 32nd part, then the lanes are added
+        for (int tok = warp; tok < p.n_tok; tok += WARPS) {
+            float acc = 0.0f;
+#pragma unroll 4
+            for (int part = lane; part < p.n_in_parts; part += 32) acc += p.in_ssq[(long)part * tc::SSQ_LD + tok];
+            acc = ib_warp_sum(acc);
+            if (lane == 0) inv_s[tok] = 1.0f / sqrtf(acc * p.in_inv_width + p.in_eps);
+        }
+    } else if (threadIdx.x < TOK) {
+        inv_s[threadIdx.x] = 1.0f;
+    }
+
+    float acc[MATS][TILES][NT][4];
+#pragma unroll
+    for (int m = 0; m < MATS; ++m)
+#pragma unroll
+        for (int t = 0; t < TILES; ++t)
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[m][t][n][e] = 0.0f;
+    const int gid = lane >> 2, tig = lane & 3;
+    bool ok = true;
+    int s = 0, phase = 0;
+    for (int i = 0; i < n_mine; ++i) {
+        ok = mbar_wait_bounded(full0 + 8 * s, phase, &tc::g_error, 4);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        const unsigned char* st = ring + s * S::STAGE;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int piece = (((2 * tig + h) ^ gid) << 4) + gid * 128;      // of the eight rows of a 1 KB group
+            uint4 xb[NT];
+#pragma unroll
+            for (int n = 0; n < NT; ++n) xb[n] = *reinterpret_cast<const uint4*>(st + MATS * S::W_BYTES + n * 1024 + piece);
+#pragma unroll
+            for (int m = 0; m < MATS; ++m)
+#pragma unroll
+                for (int t = 0; t < TILES; ++t) {
+                    const unsigned char* wt = st + m * S::W_BYTES + t * 2048 + piece;
+                    const uint4 lo = *reinterpret_cast<const uint4*>(wt);
+                    uint4 hi = make_uint4(0, 0, 0, 0);
+                    if (t * 16 + 8 < R) hi = *reinterpret_cast<const uint4*>(wt + 1024);
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) {
+                        mma16816(acc[m][t][n], lo.x, hi.x, lo.y, hi.y, xb[n].x, xb[n].y);
+                        mma16816(acc[m][t][n], lo.z, hi.z, lo.w, hi.w, xb[n].z, xb[n].w);
+                    }
+                }
+        }
+        __syncwarp();                                                        // the warp has read the stage
+        if (lane == 0 && i + S::STAGES < n_mine) { load_w(i + S::STAGES, s); load_x(i + S::STAGES, s); }
+        if (++s == S::STAGES) { s = 0; phase ^= 1; }
+    }
+    ok = __syncthreads_and(ok);                                              // every ring is idle
+    if (!ok) {   // a wait of this CTA ran out: copies still in flight get time to land before it leaves
+        const unsigned long long t0 = global_ns();
+        while (global_ns() - t0 < 2000000ull) __nanosleep(1000);
+        return;
+    }
+    float* sums = reinterpret_cast<float*>(smem);                            // [matrix][warp][token][row]
+    float* squares = sums + MATS * WARPS * TOK * R;                          // [token][row]
+#pragma unroll
+    for (int m = 0; m < MATS; ++m)
+#pragma unroll
+        for (int t = 0; t < TILES; ++t)
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int row = t * 16 + gid + 8 * (e >> 1), tok = n * 8 + 2 * tig + (e & 1);
+                    if (row < R) sums[((m * WARPS + warp) * TOK + tok) * R + row] = acc[m][t][n][e];
+                }
+    __syncthreads();
+#pragma unroll
+    for (int o = 0; o < OUTS; ++o) {
+        const int idx = (int)threadIdx.x + o * THREADS, tok = idx / R, f = f0 + idx % R;
+        if (idx >= TOK * R) break;
+        float v = 0.0f, ssq = 0.0f;
+#pragma unroll
+        for (int wp = 0; wp < WARPS; ++wp) v += sums[wp * TOK * R + idx];
+        if (tok < p.n_tok && f < p.n_out) {
+            if constexpr (GATED) {
+                float u = 0.0f;
+#pragma unroll
+                for (int wp = 0; wp < WARPS; ++wp) u += sums[(WARPS + wp) * TOK * R + idx];
+                const float g = __bfloat162float(__float2bfloat16_rn(v * inv_s[tok]));
+                u = __bfloat162float(__float2bfloat16_rn(u * inv_s[tok]));
+                reinterpret_cast<__nv_bfloat16*>(p.y)[(long)tok * p.ldy + f] = __float2bfloat16_rn(g / (1.0f + expf(-g)) * u);
+            } else {
+                const float r = tc::finish_value(p, v, tok, f, inv_s[tok], old[o], w_sink[o], ssq);
+                const long at = (BATCH ? (long)blockIdx.y * p.by : 0) + (long)tok * p.ldy + f;
+                if (p.y_is_f32) reinterpret_cast<float*>(p.y)[at] = r;
+                else reinterpret_cast<__nv_bfloat16*>(p.y)[at] = __float2bfloat16_rn(r);
+            }
+        }
+        if (!GATED && p.residual != nullptr) squares[idx] = ssq;
+    }
+    if (!GATED && p.residual != nullptr) {
+        __syncthreads();
+        for (int tok = warp; tok < tc::SSQ_LD; tok += WARPS) {               // this CTA's part of the rows' sums of squares
+            float t = 0.0f;
+            if (tok < p.n_tok)
+                for (int r = lane; r < R; r += 32) t += squares[tok * R + r];
+            t = ib_warp_sum(t);
+            if (lane == 0) p.out_ssq[(long)blockIdx.x * tc::SSQ_LD + tok] = t;
+        }
+    }
+}
+
+template <int R, bool GATED, int TOK, bool BATCH>
+static int launch_maps(const CUtensorMap& mw, const CUtensorMap& mx, const tc::Params& p, int batch, cudaStream_t stream) {
+    using S = Shape<R, GATED, TOK>;
+    static IbDeviceSet allowed;
+    if (const int e = ib_allow_dynamic_smem(allowed, rows_kernel<R, GATED, TOK, BATCH>, S::smem)) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((p.n_out + R - 1) / R, batch);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = S::smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = tc::g_pdl ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, rows_kernel<R, GATED, TOK, BATCH>, mw, mx, p);
+    return e == cudaSuccess ? ib_launch_status() : (int)e;
+}
+
+template <int R, bool GATED, int TOK>
+static int launch(const void* w, long n_w, long ldw, const void* x, long ldx, int k, const tc::Params& p, cudaStream_t stream) {
+    CUtensorMap mw, mx;
+    if (!tc::make_map(&mw, w, n_w, k, ldw, R) || !tc::make_map(&mx, x, p.n_tok, k, ldx, TOK)) return IB_ERR_UNSUPPORTED;
+    return launch_maps<R, GATED, TOK, false>(mw, mx, p, 1, stream);
+}
+
+// a batch of row-major [rows, k] bfloat16 matrices `stride` elements apart, boxes of [box_rows, 64] of one of them
+static bool make_batch_map(CUtensorMap* map, const void* base, long rows, long k, long ld, long stride, int batch, int box_rows) {
+    EncodeTiled enc = encode_fn();
+    if (enc == nullptr) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)k, (cuuint64_t)rows, (cuuint64_t)batch};
+    const cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)stride * 2};
+    const cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1};
+    const cuuint32_t elem[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, elem,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int R, int TOK>
+static int launch_batch(const void* w, const void* x, long ldx, long bx, int k, int batch, const tc::Params& p, cudaStream_t stream) {
+    CUtensorMap mw, mx;
+    if (!make_batch_map(&mw, w, p.n_out, k, k, (long)p.n_out * k, batch, R) ||
+        !make_batch_map(&mx, x, p.n_tok, k, ldx, bx, batch, TOK)) return IB_ERR_UNSUPPORTED;
+    return launch_maps<R, false, TOK, true>(mw, mx, p, batch, stream);
+}
+
+// R rows of W per CTA (gated: of each of the two matrices)
+template <bool GATED>
+static int launch_any(int r, const void* w, long n_w, long ldw, const void* x, long ldx, int k, const tc::Params& p,
+                      cudaStream_t stream) {
+    const bool few = p.n_tok <= 8;
+    switch (r) {
+        case 16: return few ? launch<16, GATED, 8>(w, n_w, ldw, x, ldx, k, p, stream) : launch<16, GATED, 16>(w, n_w, ldw, x, ldx, k, p, stream);
+        case 24: return few ? launch<24, GATED, 8>(w, n_w, ldw, x, ldx, k, p, stream) : IB_ERR_UNSUPPORTED;
+        case 32: if constexpr (!GATED) return few ? launch<32, GATED, 8>(w, n_w, ldw, x, ldx, k, p, stream) : launch<32, GATED, 16>(w, n_w, ldw, x, ldx, k, p, stream);
+        case 48: if constexpr (!GATED) return few ? launch<48, GATED, 8>(w, n_w, ldw, x, ldx, k, p, stream) : IB_ERR_UNSUPPORTED;
+    }
+    return IB_ERR_UNSUPPORTED;
+}
+
+}  // namespace rows
+
+// Rows of W per CTA of the kernel without clusters, or 0: the tcgen05 kernel takes the product.  Products alone, replayed one
+// after the other with cold weights, us, tcgen05 / 16 / 24 / 32 / 48 rows a CTA (gated: of each matrix):
+//   4 tokens:  1,024 over 2,048  6.3 / 3.7 / 3.6 / 3.9 / 4.3      gated 3,072 over 1,024    7.7 /  4.2 /  4.1
+//              4,096 over 1,024  5.6 / 3.5 / 3.7 / 3.6 / 3.9      gated 12,288 over 4,096  34.9 / 33.3 / 32.4
+//              6,144 over 4,096 13.3 / 17.7 / 11.3 / 10.0 / 11.0  10,240 over 5,120  20.8 / 32.3 / 24.4 / 21.9 / 17.6
+//              2,048 over 8,192 11.8 / 15.5 / 12.1 / 10.8 / 11.6  4,096 over 12,288  20.6 / 36.5 / 34.1 / 20.2 / 21.5
+//   16 tokens: 1,024 over 2,048  7.0 / 3.9 /  -  / 4.4            gated 3,072 over 1,024    8.8 /  6.6
+//              4,096 over 4,096 12.2 / 12.1 / -  / 9.8            gated 12,288 over 4,096  36.4 / 39.8
+//              2,048 over 8,192 12.5 / 18.5 / -  / 12.8           10,240 over 5,120  21.7 / 35.6 / -  / 25.8
+// Boxes of few rows are what a long K does not want; more CTAs than two an SM are a second wave with fetches of its own.
+static int rows_form(int n_tok, int n_out, int num_kb, int gated) {
+    constexpr int RESIDENT = 296;
+    if (n_tok <= 8) {
+        if (gated) return 24;
+        if (n_out <= 24 * 148 && num_kb <= 64) return 24;
+        return n_out <= 32 * RESIDENT ? 32 : n_out <= 48 * RESIDENT ? 48 : 0;
+    }
+    if (n_tok > 16) return 0;
+    if (gated) return n_out <= 16 * RESIDENT ? 16 : 0;
+    if (n_out <= 2048) return num_kb <= 64 ? 16 : 0;
+    return n_out <= 32 * RESIDENT ? 32 : 0;
+}
+
 // How many CTAs share one output tile when the caller does not say.  Each part is a CTA whose ring (80 KB) holds a share of
 // W before the kernel ahead has finished; more parts cost in the cluster's summing and in x read once more.  Products
 // alone, replayed one after the other with cold weights, us with fewer / more parts:
@@ -671,12 +962,16 @@ static int gemm_tn(const void* x, long ldx, const void* w, long ldw, void* y, lo
     if ((f.in_ssq != nullptr || f.residual != nullptr) && bn > 32) return IB_ERR_UNSUPPORTED;
     if (f.residual != nullptr && (f.sink_w == nullptr || f.out_ssq == nullptr || y_is_f32)) return IB_ERR_ARGUMENT;
     if (f.in_ssq != nullptr && (f.n_in_parts <= 0 || f.in_width <= 0)) return IB_ERR_ARGUMENT;
-    tc::Params p;
+    tc::Params p = {};
     p.y = y; p.ldy = ldy; p.n_tok = n_tok; p.n_out = n_out; p.num_kb = (k + tc::BK - 1) / tc::BK; p.y_is_f32 = y_is_f32;
     p.inner = 0;
     p.gelu = gelu;
     p.in_ssq = f.in_ssq; p.n_in_parts = f.n_in_parts; p.in_eps = f.in_eps; p.in_inv_width = f.in_width > 0 ? 1.0f / (float)f.in_width : 0.0f;
     p.residual = f.residual; p.ld_res = f.ld_res; p.sink_w = f.sink_w; p.sink_w_is_f32 = f.sink_w_is_f32; p.out_ssq = f.out_ssq;
+    if (const int r = split_k < 0 ? -split_k : split_k == 0 ? rows_form(n_tok, n_out, p.num_kb, 0) : 0) {
+        if (n_tok > 16) return IB_ERR_UNSUPPORTED;
+        return rows::launch_any<false>(r, w, n_out, ldw, x, ldx, k, p, stream);
+    }
     const int splits = choose_splits(n_tok, n_out, p.num_kb, bn, split_k);
     if (splits != 1 && splits != 2 && splits != 4 && splits != 8) return IB_ERR_ARGUMENT;
     p.tile_rows = tile_rows_for(n_out, splits, tc::BM, resident_for(bn, splits));
@@ -693,8 +988,27 @@ static int gemm_tn(const void* x, long ldx, const void* w, long ldw, void* y, lo
     }
 }
 
+// A batch of products of up to sixteen tokens, y_b = x_b w_b^T for b < batch: x_b [n_tok, k] (row stride ldx) starts bx
+// elements after x_(b - 1), w [batch, n_out, k] is contiguous, y_b [n_tok, n_out] (row stride ldy) starts by elements after
+// y_(b - 1); all bfloat16.  Heads of a latent attention, for instance.
+IB_EXPORT int ib_gemm_tn_rows_batched(const void* x, long ldx, long bx, const void* w, void* y, long ldy, long by, int n_tok,
+                                      int n_out, int k, int batch, cudaStream_t stream) {
+    if (n_tok <= 0 || n_out <= 0 || batch <= 0) return IB_OK;
+    if (k <= 0) return IB_ERR_ARGUMENT;
+    if (n_tok > 16 || batch > 65535 || (k % 8) || (ldx % 8) || (bx % 8) || ((uintptr_t)x % 16) || ((uintptr_t)w % 16))
+        return IB_ERR_UNSUPPORTED;
+    tc::Params p = {};
+    p.y = y; p.ldy = ldy; p.by = by; p.n_tok = n_tok; p.n_out = n_out; p.num_kb = (k + tc::BK - 1) / tc::BK;
+    // rows of w per CTA: 32 where that still gives every SM a CTA
+    const bool wide = (long)((n_out + 31) / 32) * batch >= 148;
+    if (n_tok <= 8)
+        return wide ? rows::launch_batch<32, 8>(w, x, ldx, bx, k, batch, p, stream) : rows::launch_batch<16, 8>(w, x, ldx, bx, k, batch, p, stream);
+    return wide ? rows::launch_batch<32, 16>(w, x, ldx, bx, k, batch, p, stream) : rows::launch_batch<16, 16>(w, x, ldx, bx, k, batch, p, stream);
+}
+
 // x [n_tok, k] (row stride ldx), w [n_out, k] (row stride ldw), both bfloat16; y [n_tok, n_out] bfloat16 or float32.
-// split_k: 0 lets the function choose (1, 2, 4 or 8 CTAs per output tile); 8 is taken for up to 32 tokens (4 stands in beyond).
+// split_k: 0 lets the function choose (1, 2, 4 or 8 CTAs per output tile); 8 is taken for up to 32 tokens (4 stands in beyond);
+// -r: the kernel without clusters, r rows of w per CTA.
 IB_EXPORT int ib_gemm_tn_tcgen05(const void* x, long ldx, const void* w, long ldw, void* y, long ldy, int y_is_f32,
                                  int n_tok, int n_out, int k, int split_k, cudaStream_t stream) {
     const Folded none = {nullptr, 0, 0.0f, 0, nullptr, 0, nullptr, 0, nullptr};
@@ -726,6 +1040,8 @@ IB_EXPORT int ib_gemm_tcgen05_ssq_parts(int n_tok, int n_out, int k, int split_k
     if (n_tok <= 0 || n_out <= 0 || k <= 0) return IB_ERR_ARGUMENT;
     const int bn = bn_for(n_tok);
     if (bn > 32) return IB_ERR_UNSUPPORTED;
+    if (const int r = split_k < 0 ? -split_k : split_k == 0 ? rows_form(n_tok, n_out, (k + tc::BK - 1) / tc::BK, 0) : 0)
+        return (n_out + r - 1) / r;
     const int splits = choose_splits(n_tok, n_out, (k + tc::BK - 1) / tc::BK, bn, split_k);
     const int rows = tile_rows_for(n_out, splits, tc::BM, resident_for(bn, splits));
     return ((n_out + rows - 1) / rows) * splits;
@@ -735,20 +1051,26 @@ IB_EXPORT int ib_gemm_tcgen05_ssq_parts(int n_tok, int n_out, int k, int split_k
 // and the gate itself in one kernel.  w [2 * inner, k] holds the gate matrix above the up matrix; y [n_tok, inner]
 // bfloat16.  Up to 32 tokens (IB_ERR_UNSUPPORTED beyond; the caller then runs product and gate separately).  With
 // in_ssq, x holds scaled rows as above and both products are scaled per token before the gate.
+// rows_per_cta: 0 lets the function choose the kernel; else the rows of each matrix per CTA of the kernel without clusters, or
+// -1 for the tcgen05 kernel.
 IB_EXPORT int ib_gemm_swiglu_tcgen05_folded(const void* x, long ldx, const void* w, long ldw, void* y, long ldy, int n_tok,
                                             int inner, int k, const float* in_ssq, int n_in_parts, float in_eps,
-                                            int in_width, cudaStream_t stream) {
+                                            int in_width, int rows_per_cta, cudaStream_t stream) {
     if (n_tok <= 0 || inner <= 0) return IB_OK;
     if (k <= 0) return IB_ERR_ARGUMENT;
     if ((k % 8) || (ldx % 8) || (ldw % 8) || ((uintptr_t)x % 16) || ((uintptr_t)w % 16) || n_tok > 32) return IB_ERR_UNSUPPORTED;
     if (in_ssq != nullptr && (n_in_parts <= 0 || in_width <= 0)) return IB_ERR_ARGUMENT;
     const int bn = n_tok <= 16 ? 16 : 32;
-    tc::Params p;
+    tc::Params p = {};
     p.y = y; p.ldy = ldy; p.n_tok = n_tok; p.n_out = inner; p.num_kb = (k + tc::BK - 1) / tc::BK; p.y_is_f32 = 0;
     p.inner = inner;
     p.gelu = 0;
     p.in_ssq = in_ssq; p.n_in_parts = n_in_parts; p.in_eps = in_eps; p.in_inv_width = in_width > 0 ? 1.0f / (float)in_width : 0.0f;
     p.residual = nullptr; p.ld_res = 0; p.sink_w = nullptr; p.sink_w_is_f32 = 0; p.out_ssq = nullptr;
+    if (const int r = rows_per_cta > 0 ? rows_per_cta : rows_per_cta == 0 ? rows_form(n_tok, inner, p.num_kb, 1) : 0) {
+        if (n_tok > 16) return IB_ERR_UNSUPPORTED;
+        return rows::launch_any<true>(r, w, 2L * inner, ldw, x, ldx, k, p, stream);
+    }
     p.tile_rows = tile_rows_for(inner, 1, 64, resident_for(bn, 1));
     CUtensorMap mw, mx;
     if (!tc::make_map(&mw, w, 2L * inner, k, ldw, p.tile_rows) || !tc::make_map(&mx, x, n_tok, k, ldx, bn)) return IB_ERR_UNSUPPORTED;
@@ -757,7 +1079,7 @@ IB_EXPORT int ib_gemm_swiglu_tcgen05_folded(const void* x, long ldx, const void*
 
 IB_EXPORT int ib_gemm_swiglu_tcgen05(const void* x, long ldx, const void* w, long ldw, void* y, long ldy, int n_tok,
                                      int inner, int k, cudaStream_t stream) {
-    return ib_gemm_swiglu_tcgen05_folded(x, ldx, w, ldw, y, ldy, n_tok, inner, k, nullptr, 0, 0.0f, 0, stream);
+    return ib_gemm_swiglu_tcgen05_folded(x, ldx, w, ldw, y, ldy, n_tok, inner, k, nullptr, 0, 0.0f, 0, 0, stream);
 }
 
 // 1: later launches may start before the kernel before them in the stream has finished (programmatic dependent

@@ -543,7 +543,18 @@ def batched_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act_dtyp
             raise KernelError(f"batched_linear: no kernel for x {x.dtype}, w {w.dtype}, out {out.dtype}")
         _check(code, "gemm_tn_simt_batched")
     else:
-        torch.bmm(x, w.transpose(1, 2), out=out)
+        code = -1
+        if n <= BATCHED_ROWS and x.dtype == w.dtype == out.dtype == torch.bfloat16:
+            # few rows: the library's kernel cannot start before the one ahead has ended, and the one after it waits for it too
+            code = _gemm_lib().ib_gemm_tn_rows_batched(_p(x), x.stride(1), x.stride(0), _p(w), _p(out), out.stride(1),
+                                                       out.stride(0), n, m, k, b, _stream())
+        if code == -1:          # more rows, or rows that do not start on 16 bytes
+            torch.bmm(x, w.transpose(1, 2), out=out)
+        else:
+            _check(code, "gemm_tn_rows_batched")
+
+
+BATCHED_ROWS = 16    # rows up to which a batch of products runs on the kernel for few rows (csrc/gemm_tcgen05.cu)
 
 
 def resolve_tokens(ids: torch.Tensor, carry: torch.Tensor, act_dtype: torch.dtype):
@@ -2179,6 +2190,9 @@ def _gemm_lib():
         lib.ib_gemm_tn_tcgen05.argtypes = [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_int, c_int, c_int,
                                            c_int, c_int, c_void_p]
         lib.ib_gemm_tn_tcgen05.restype = c_int
+        lib.ib_gemm_tn_rows_batched.argtypes = [c_void_p, c_long, c_long, c_void_p, c_void_p, c_long, c_long, c_int, c_int,
+                                                c_int, c_int, c_void_p]
+        lib.ib_gemm_tn_rows_batched.restype = c_int
         lib.ib_gemm_tn_tcgen05_gelu.argtypes = lib.ib_gemm_tn_tcgen05.argtypes
         lib.ib_gemm_tn_tcgen05_gelu.restype = c_int
         lib.ib_gemm_swiglu_tcgen05.argtypes = [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_int, c_int, c_int,
@@ -2189,7 +2203,7 @@ def _gemm_lib():
                                                   c_int, c_void_p, c_void_p]
         lib.ib_gemm_tn_tcgen05_folded.restype = c_int
         lib.ib_gemm_swiglu_tcgen05_folded.argtypes = [c_void_p, c_long, c_void_p, c_long, c_void_p, c_long, c_int, c_int,
-                                                      c_int, c_void_p, c_int, c_float, c_int, c_void_p]
+                                                      c_int, c_void_p, c_int, c_float, c_int, c_int, c_void_p]
         lib.ib_gemm_swiglu_tcgen05_folded.restype = c_int
         lib.ib_gemm_tcgen05_ssq_parts.argtypes = [c_int, c_int, c_int, c_int]
         lib.ib_gemm_tcgen05_ssq_parts.restype = c_int
@@ -2281,7 +2295,7 @@ def gemm_tn_tcgen05(x, w: torch.Tensor, out: torch.Tensor, split_k: int = 0, sin
     return result
 
 
-def gemm_swiglu_tcgen05(x, w_gate_up: torch.Tensor, out: torch.Tensor):
+def gemm_swiglu_tcgen05(x, w_gate_up: torch.Tensor, out: torch.Tensor, rows_per_cta: int = 0):
     """out[t, f] = silu(x[t] . w[f]) * (x[t] . w[inner + f]): both products of a gated feed-forward and the gate
     in one tcgen05 kernel (up to 64 gate rows and the same up rows per tile).  Up to 32 rows of x, which may be
     :class:`ScaledRows`."""
@@ -2294,7 +2308,7 @@ def gemm_swiglu_tcgen05(x, w_gate_up: torch.Tensor, out: torch.Tensor):
     if w_gate_up.shape != (2 * inner, k) or out.shape[0] != n:
         raise KernelError(f"gemm_swiglu: x {tuple(xt.shape)}, w {tuple(w_gate_up.shape)}, out {tuple(out.shape)}")
     code = _gemm_lib().ib_gemm_swiglu_tcgen05_folded(_p(xt), k, _p(w_gate_up), k, _p(out), inner, n, inner, k, *scaled,
-                                                     _stream())
+                                                     rows_per_cta, _stream())
     if code == -1:
         raise KernelError(f"gemm_swiglu_tcgen05: at most 32 rows (got {n}), K={k} a multiple of 8, 16-byte aligned bases")
     _check(code, "gemm_swiglu_tcgen05")

@@ -1,0 +1,74 @@
+"""bfloat16 products of a few rows by the kernel without clusters (csrc/gemm_tcgen05.cu) against 64 bits."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def rand(shape, seed, scale=1.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(shape, generator=g, device="cuda") * scale).to(torch.bfloat16)
+
+
+def close(got, want, terms):
+    """Sums of ``terms`` exact products in float32 (2^-24 each of sum |x w|), then one rounding to the output's type."""
+    half = 2.0 ** -8 if got.dtype == torch.bfloat16 else 2.0 ** -24
+    return bool(((got.double() - want).abs() <= half * want.abs() + terms).all())
+
+
+FORMS = [(16, 1), (16, 3), (16, 16), (24, 1), (24, 8), (32, 8), (32, 13), (48, 5)]
+
+
+@pytest.mark.parametrize("r,n", FORMS)
+@pytest.mark.parametrize("m,k", [(64, 8), (200, 72), (1000, 3080), (1024, 2048)])
+def test_product_with_folded_norms_and_gate(r, n, m, k):
+    from inferrs_b200 import kernels as K
+    x, w = rand((n, k), 1), rand((m, k), 2, 0.05)
+    dot = x.double() @ w.double().t()
+    terms = k * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    for dtype in (torch.bfloat16, torch.float32):
+        out = torch.full((n, m), float("nan"), device="cuda", dtype=dtype)
+        K.gemm_tn_tcgen05(x, w, out, split_k=-r)
+        assert close(out, dot, terms)
+    # rows scaled by the norm before, added to the stream, handed on times the weight of the norm after
+    ssq = torch.rand(7, K.SSQ_LD, device="cuda")
+    inv = 1.0 / torch.sqrt(ssq[:, :n].double().sum(0) / k + 1e-6)
+    scaled = K.ScaledRows(x, ssq, 7, 1e-6, k)
+    stream = torch.randn(n, m, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    weight, old = 0.5 + torch.rand(m, device="cuda"), stream.clone()
+    out = torch.empty(n, m, dtype=torch.bfloat16, device="cuda")
+    got = K.gemm_tn_tcgen05(scaled, w, out, split_k=-r, sink=K.ResidualSink(stream, weight, 1e-5))
+    y = dot * inv[:, None]
+    assert bool(((stream.double() - (old.double() + y)).abs() <= 2.0 ** -8 * y.abs() + terms * inv[:, None] + 1e-6).all())
+    assert torch.equal(out, (stream * weight).to(torch.bfloat16))
+    sums, want = got.ssq[:got.n_parts, :n].double().sum(0), (stream.double() ** 2).sum(1)
+    assert got.n_parts == (m + r - 1) // r and bool(((sums - want).abs() <= m * 2.0 ** -24 * want).all())
+    if r <= (24 if n <= 8 else 16):
+        inner = m // 2
+        out = torch.full((n, inner), float("nan"), dtype=torch.bfloat16, device="cuda")
+        K.gemm_swiglu_tcgen05(scaled, w[:2 * inner], out, rows_per_cta=r)
+        g, u = y[:, :inner], y[:, inner:2 * inner]
+        want = g / (1 + torch.exp(-g)) * u
+        # both factors are rounded to bfloat16 first (2^-9 each; silu changes at most 1.1 times as much as its argument)
+        slack = 2.0 ** -8 * (1.1 * g.abs() * u.abs() + want.abs()) + 1e-4
+        assert bool(((out.double() - want).abs() <= slack).all())
+    assert K.gemm_tcgen05_error() == 0
+
+
+@pytest.mark.parametrize("n", [1, 8, 9, 16])
+@pytest.mark.parametrize("b,m,k", [(1, 40, 8), (3, 100, 72), (16, 512, 128), (16, 128, 512)])
+def test_batch_of_products(n, b, m, k):
+    """Heads of [rows, heads, k] and of [heads, rows, k], read and written in place; and rows that do not start on 16 bytes."""
+    from inferrs_b200 import kernels as K
+    w = rand((b, m, k), 4, 0.1)
+    for x in (rand((n, b, k + 8), 5)[:, :, :k].transpose(0, 1), rand((b, n, k), 6), rand((n, b, k + 1), 7)[:, :, 1:].transpose(0, 1)):
+        want = torch.einsum("bnk,bmk->bnm", x.double(), w.double())
+        terms = k * 2.0 ** -24 * torch.einsum("bnk,bmk->bnm", x.double().abs(), w.double().abs())
+        out = torch.full((n, b, m), float("nan"), dtype=torch.bfloat16, device="cuda")
+        K.batched_linear(x, w, out.transpose(0, 1), torch.bfloat16)
+        assert close(out.transpose(0, 1), want, terms)
+        first = torch.empty((b, n, m), dtype=torch.bfloat16, device="cuda")
+        K.batched_linear(x, w, first, torch.bfloat16)
+        assert torch.equal(first, out.transpose(0, 1))
