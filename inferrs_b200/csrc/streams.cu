@@ -164,7 +164,136 @@ __global__ void stream_add_norm_kernel(float* __restrict__ residual, const act_t
         dst[j] = ib_from_float<act_t>(u_row[j] * inv_g[j / part] * ib_to_float(weight[j]));
 }
 
+// The same for the widths that a block holds in registers (ITER x 4 columns a thread), with parts of whole 128-column
+// pieces: every load is asked for at once, weights before the kernel ahead has ended, and the parts' sums meet once (a
+// warp's 128 columns belong to one part; every thread adds up the pieces of its own).  With a few rows the kernel is
+// nothing but these waits.
+template <typename WT> struct alignas(sizeof(WT) * 4) Weight4 { WT v[4]; };
+
+template <typename WT, int S, int ITER>
+__global__ void __launch_bounds__(512) stream_add_norm_once_kernel(float* __restrict__ residual, const act_t* __restrict__ delta,
+                                                                   const float* __restrict__ mix, const float* __restrict__ gain,
+                                                                   const float* __restrict__ read, const WT* __restrict__ weight,
+                                                                   act_t* __restrict__ out, const int* __restrict__ rows,
+                                                                   int width, int part, float eps) {
+    __shared__ float pieces[ITER * 16];                     // sums of squares of 128 columns each
+    ib_grid_dependency_launch();
+    float m[S][S], gn[S], rd[S];
+    Weight4<WT> w[ITER];
+#pragma unroll
+    for (int t = 0; t < S; ++t) {
+        gn[t] = gain ? gain[t] : 1.0f;
+        rd[t] = read ? read[t] : 1.0f;
+#pragma unroll
+        for (int s = 0; s < S; ++s) m[s][t] = mix ? mix[s * S + t] : (s == t ? 1.0f : 0.0f);
+    }
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) {
+        const int j = (i * (int)blockDim.x + (int)threadIdx.x) * 4;
+        if (j < width) w[i] = *reinterpret_cast<const Weight4<WT>*>(weight + j);
+    }
+    ib_grid_dependency_wait();
+    const int r = blockIdx.x;
+    const int src = rows ? rows[r] : r;
+    float* res = residual + (size_t)src * S * width;
+    const act_t* del = delta ? delta + (size_t)src * width : nullptr;
+    const bool write_back = (rows == nullptr) && (del != nullptr);
+    float4 x[ITER][S];
+    StreamVec4 dv[ITER];
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) {
+        const int j = (i * (int)blockDim.x + (int)threadIdx.x) * 4;
+        if (j < width) {
+#pragma unroll
+            for (int s = 0; s < S; ++s) x[i][s] = *reinterpret_cast<const float4*>(res + (size_t)s * width + j);
+            if (del) dv[i] = *reinterpret_cast<const StreamVec4*>(del + j);
+        }
+    }
+    float u[ITER][4];
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) {
+        const int j = (i * (int)blockDim.x + (int)threadIdx.x) * 4;
+        float ss = 0.0f;
+        if (j < width) {                                    // whole warps: the width is a multiple of 128
+            float xs[S][4];
+#pragma unroll
+            for (int s = 0; s < S; ++s) { xs[s][0] = x[i][s].x; xs[s][1] = x[i][s].y; xs[s][2] = x[i][s].z; xs[s][3] = x[i][s].w; }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) u[i][c] = 0.0f;
+            if (del) {
+#pragma unroll
+                for (int t = 0; t < S; ++t) {
+                    float v[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        v[c] = 0.0f;
+#pragma unroll
+                        for (int s = 0; s < S; ++s) v[c] = fmaf(m[s][t], xs[s][c], v[c]);
+                        v[c] = fmaf(gn[t], ib_to_float(dv[i].v[c]), v[c]);
+                        u[i][c] = fmaf(rd[t], v[c], u[i][c]);
+                    }
+                    if (write_back)
+                        *reinterpret_cast<float4*>(res + (size_t)t * width + j) = make_float4(v[0], v[1], v[2], v[3]);
+                }
+            } else {
+#pragma unroll
+                for (int t = 0; t < S; ++t)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) u[i][c] = fmaf(rd[t], xs[t][c], u[i][c]);
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) ss = fmaf(u[i][c], u[i][c], ss);
+            ss = ib_warp_sum(ss);
+            if ((threadIdx.x & 31) == 0) pieces[j >> 7] = ss;
+        }
+    }
+    __syncthreads();
+    act_t* dst = out + (size_t)r * width;
+    const int n_pieces = part >> 7;
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) {
+        const int j = (i * (int)blockDim.x + (int)threadIdx.x) * 4;
+        if (j < width) {
+            const int first = ((j >> 7) / n_pieces) * n_pieces;
+            float ss = 0.0f;
+            for (int k = 0; k < n_pieces; ++k) ss += pieces[first + k];
+            const float inv = 1.0f / sqrtf(ss / (float)part + eps);
+            StreamVec4 o;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) o.v[c] = ib_from_float<act_t>(u[i][c] * inv * ib_to_float(w[i].v[c]));
+            *reinterpret_cast<StreamVec4*>(dst + j) = o;
+        }
+    }
+}
+
 static IbDeviceSet stream_norm_smem_f32, stream_norm_smem_bf16;
+
+// Whether the kernel that holds a row in registers takes these sizes, and if so launches it.
+template <typename WT>
+static bool stream_add_norm_once(float* residual, const act_t* delta, const float* mix, const float* gain, const float* read,
+                                 const WT* weight, act_t* out, const int* rows, int n_rows, int streams, int width,
+                                 int groups, float eps, cudaStream_t stream) {
+    const int part = width / groups;
+    if (part % 128 || width > 8192 || (streams != 1 && streams != 2 && streams != 4)) return false;
+    if (((uintptr_t)residual | (uintptr_t)weight) % (4 * sizeof(float)) ||
+        ((uintptr_t)delta | (uintptr_t)out) % (4 * sizeof(act_t))) return false;
+    const int threads = width / 4 < 512 ? width / 4 : 512;
+    const int iter = width <= 2048 ? 1 : width <= 4096 ? 2 : 4;
+    if (streams * iter > 8) return false;                   // registers
+    const dim3 grid(n_rows), block(threads);
+#define IB_ONCE(S, ITER)                                                                                            \
+    ib_launch(stream_add_norm_once_kernel<WT, S, ITER>, grid, block, 0, stream, residual, delta, mix, gain, read,   \
+              weight, out, rows, width, part, eps)
+    if (iter == 1) {
+        if (streams == 1) IB_ONCE(1, 1); else if (streams == 2) IB_ONCE(2, 1); else IB_ONCE(4, 1);
+    } else if (iter == 2) {
+        if (streams == 1) IB_ONCE(1, 2); else if (streams == 2) IB_ONCE(2, 2); else IB_ONCE(4, 2);
+    } else {
+        if (streams == 1) IB_ONCE(1, 4); else IB_ONCE(2, 4);
+    }
+#undef IB_ONCE
+    return true;
+}
 
 IB_EXPORT int ib_stream_add_norm(float* residual, const void* delta, const float* mix, const float* gain,
                                  const float* read, const void* weight, int weight_is_f32, void* out, const int* rows,
@@ -172,6 +301,11 @@ IB_EXPORT int ib_stream_add_norm(float* residual, const void* delta, const float
     if (n_rows <= 0) return IB_OK;
     if (width <= 0 || streams <= 0 || groups <= 0 || width % groups || weight == nullptr) return IB_ERR_ARGUMENT;
     if (streams > IB_MAX_STREAMS || groups > IB_MAX_GROUPS) return IB_ERR_UNSUPPORTED;
+    if (weight_is_f32 ? stream_add_norm_once(residual, (const act_t*)delta, mix, gain, read, (const float*)weight, (act_t*)out,
+                                             rows, n_rows, streams, width, groups, eps, stream)
+                      : stream_add_norm_once(residual, (const act_t*)delta, mix, gain, read, (const __nv_bfloat16*)weight,
+                                             (act_t*)out, rows, n_rows, streams, width, groups, eps, stream))
+        return ib_launch_status();
     const size_t smem = (size_t)width * sizeof(float);
     const size_t smem_most = 200 * 1024;      // the permission for more than 48 KB is given once per device, for the most
     if (smem > smem_most) return IB_ERR_UNSUPPORTED;
@@ -240,6 +374,71 @@ __global__ void head_norm_gate_kernel(const OT* __restrict__ o, long o_row, long
     }
 }
 
+// The same for heads that a warp holds in registers (four numbers a lane and step, up to 128 ITER of them): the row, its gate
+// and its weight are asked for together, and the row is read once.
+template <typename OT, typename WT, int ITER>
+__global__ void head_norm_gate_vec_kernel(const OT* __restrict__ o, long o_row, long o_head, const act_t* __restrict__ gate,
+                                          long ld_gate, const WT* __restrict__ w, int w_per_head, int norm_mode,
+                                          int gate_act, float eps, act_t* __restrict__ out, int n_rows, int heads, int e_dim) {
+    ib_grid_dependency_launch();
+    const int lane = threadIdx.x & 31;
+    const long item = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (item >= (long)n_rows * heads) { ib_grid_dependency_wait(); return; }
+    const int row = (int)(item / heads), h = (int)(item - (long)row * heads);
+    Weight4<WT> wv[ITER];
+    if (w) {
+#pragma unroll
+        for (int i = 0; i < ITER; ++i) {
+            const int e = (i * 32 + lane) * 4;
+            if (e < e_dim) wv[i] = *reinterpret_cast<const Weight4<WT>*>(w + (w_per_head ? (long)h * e_dim + e : e));
+        }
+    }
+    ib_grid_dependency_wait();
+    const OT* src = o + (long)row * o_row + (long)h * o_head;
+    const act_t* g = gate ? gate + (long)row * ld_gate + (long)h * e_dim : nullptr;     // no gate: the normed heads alone
+    Weight4<OT> v[ITER];
+    StreamVec4 z[ITER];
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) {
+        const int e = (i * 32 + lane) * 4;
+        if (e < e_dim) {
+            v[i] = *reinterpret_cast<const Weight4<OT>*>(src + e);
+            if (g) z[i] = *reinterpret_cast<const StreamVec4*>(g + e);
+        }
+    }
+    float inv = 1.0f;
+    if (norm_mode) {
+        float ss = 0.0f;
+#pragma unroll
+        for (int i = 0; i < ITER; ++i)
+            if ((i * 32 + lane) * 4 < e_dim) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) ss = fmaf(ib_to_float(v[i].v[c]), ib_to_float(v[i].v[c]), ss);
+            }
+        ss = ib_warp_sum(ss);
+        inv = 1.0f / sqrtf(ss / (float)e_dim + eps);
+    }
+    act_t* dst = out + ((long)row * heads + h) * e_dim;
+#pragma unroll
+    for (int i = 0; i < ITER; ++i) {
+        const int e = (i * 32 + lane) * 4;
+        if (e >= e_dim) continue;
+        StreamVec4 r;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            float t = ib_to_float(v[i].v[c]) * inv;
+            if (w) t *= ib_to_float(wv[i].v[c]);
+            if (g) {
+                const float y = ib_to_float(z[i].v[c]);
+                const float sg = 1.0f / (1.0f + expf(-y));
+                t *= gate_act == 0 ? y * sg : sg;
+            }
+            r.v[c] = ib_from_float<act_t>(t);
+        }
+        *reinterpret_cast<StreamVec4*>(dst + e) = r;
+    }
+}
+
 // The same with a block of eight warps per (row, head), for heads of 512 numbers and more (one norm over all of a
 // mixer's heads side by side, for instance): a warp alone would walk the row twice, 32 numbers at a time.
 template <typename OT, typename WT>
@@ -296,6 +495,24 @@ IB_EXPORT int ib_head_norm_gate(const void* o, int o_is_f32, long o_row, long o_
         return ib_launch_status();
     }
     const dim3 grid((unsigned)((items + warps - 1) / warps));
+    const size_t o_vec = 4 * (o_is_f32 ? sizeof(float) : sizeof(act_t)), w_vec = 4 * (w_is_f32 ? sizeof(float) : 2);
+    if (e_dim % 4 == 0 && e_dim <= 256 && o_row % 4 == 0 && o_head % 4 == 0 && (uintptr_t)o % o_vec == 0 &&
+        (uintptr_t)out % (4 * sizeof(act_t)) == 0 && (uintptr_t)w % w_vec == 0 &&
+        (gate == nullptr || (ld_gate % 4 == 0 && (uintptr_t)gate % (4 * sizeof(act_t)) == 0))) {
+#define IB_HNGV(OT, WT, ITER)                                                                                   \
+    ib_launch(head_norm_gate_vec_kernel<OT, WT, ITER>, grid, 32 * warps, 0, stream, (const OT*)o, o_row, o_head, \
+              (const act_t*)gate, ld_gate, (const WT*)w, w_per_head, norm_mode, gate_act, eps, (act_t*)out,     \
+              n_rows, heads, e_dim)
+#define IB_HNGV2(OT, WT) do { if (e_dim <= 128) IB_HNGV(OT, WT, 1); else IB_HNGV(OT, WT, 2); } while (0)
+        if (o_is_f32) {
+            if (w_is_f32) IB_HNGV2(float, float); else IB_HNGV2(float, __nv_bfloat16);
+        } else {
+            if (w_is_f32) IB_HNGV2(act_t, float); else IB_HNGV2(act_t, __nv_bfloat16);
+        }
+#undef IB_HNGV2
+#undef IB_HNGV
+        return ib_launch_status();
+    }
 #define IB_HNG(OT, WT)                                                                                         \
     ib_launch(head_norm_gate_kernel<OT, WT>, grid, 32 * warps, 0, stream, (const OT*)o, o_row, o_head,        \
               (const act_t*)gate, ld_gate, (const WT*)w, w_per_head, norm_mode, gate_act, eps, (act_t*)out,   \
@@ -314,6 +531,17 @@ IB_EXPORT int ib_head_norm_gate(const void* o, int o_is_f32, long o_row, long o_
 //     out = a * z / r1 + b * z^2 / r2 + c * z^3 / r3 + e,     r_p = sqrt(mean((z^p)^2) + eps)
 // coef = (a, b, c, e) in float32.  Powers element by element; sums in float32.
 // ---------------------------------------------------------------------------
+// Three sums over the block in one meeting; red holds 96 numbers that nothing has read or written before.
+__device__ __forceinline__ void poly_block_sums(float& a, float& b, float& c, float* red) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = (int)blockDim.x >> 5;
+    a = ib_warp_sum(a); b = ib_warp_sum(b); c = ib_warp_sum(c);
+    if (lane == 0) { red[warp] = a; red[32 + warp] = b; red[64 + warp] = c; }
+    __syncthreads();
+    a = ib_warp_sum(lane < n ? red[lane] : 0.0f);
+    b = ib_warp_sum(lane < n ? red[32 + lane] : 0.0f);
+    c = ib_warp_sum(lane < n ? red[64 + lane] : 0.0f);
+}
+
 #define POLY_VEC (16 / (int)sizeof(act_t))      // elements per 16-byte load: 8 bfloat16 or 4 float
 #define POLY_KEEP 4                             // loads that a thread keeps in registers between the two passes
 struct alignas(16) PolyVec { act_t v[POLY_VEC]; };
@@ -321,7 +549,7 @@ struct alignas(16) PolyVec { act_t v[POLY_VEC]; };
 template <bool VEC>
 __global__ void poly_norm_kernel(const act_t* __restrict__ z, const float* __restrict__ coef, act_t* __restrict__ out,
                                  int width, float eps) {
-    __shared__ float red[32];
+    __shared__ float red[96];
     ib_grid_dependency_launch();
     const float a = coef[0], b = coef[1], c = coef[2], e = coef[3];
     ib_grid_dependency_wait();
@@ -346,9 +574,7 @@ __global__ void poly_norm_kernel(const act_t* __restrict__ z, const float* __res
                 }
             }
         }
-        s1 = ib_block_sum(s1, red);
-        s2 = ib_block_sum(s2, red);
-        s3 = ib_block_sum(s3, red);
+        poly_block_sums(s1, s2, s3, red);
         const float k1 = a / sqrtf(s1 / (float)width + eps);
         const float k2 = b / sqrtf(s2 / (float)width + eps);
         const float k3 = c / sqrtf(s3 / (float)width + eps);
@@ -376,9 +602,7 @@ __global__ void poly_norm_kernel(const act_t* __restrict__ z, const float* __res
         s2 += v2 * v2;
         s3 += v3 * v3;
     }
-    s1 = ib_block_sum(s1, red);
-    s2 = ib_block_sum(s2, red);
-    s3 = ib_block_sum(s3, red);
+    poly_block_sums(s1, s2, s3, red);
     const float k1 = a / sqrtf(s1 / (float)width + eps);
     const float k2 = b / sqrtf(s2 / (float)width + eps);
     const float k3 = c / sqrtf(s3 / (float)width + eps);
