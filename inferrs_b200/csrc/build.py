@@ -20,6 +20,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -47,6 +48,10 @@ LIBRARIES: Dict[str, dict] = {
     # host code only (the cache's book-keeping and the step description): the C++ compiler alone builds it
     "host_runtime": {"sources": ["host_runtime.cpp"], "flags": [], "link": [], "host": True},
 }
+# reads Python's own lists; only where the interpreter's headers are installed (its caller has another way)
+_PYTHON_INCLUDE = sysconfig.get_paths()["include"]
+if os.path.isfile(os.path.join(_PYTHON_INCLUDE, "Python.h")):
+    LIBRARIES["host_python"] = {"sources": ["host_python.cpp"], "flags": [f"-I{_PYTHON_INCLUDE}"], "link": [], "host": True}
 
 HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall"]
 

@@ -86,13 +86,37 @@ def uniforms_for(seeds, steps):
 
     from ..cache.manager import host_library
 
-    a, b = [int(s) & _M64 for s in seeds], [int(n) & _M64 for n in steps]
+    a, b = seeds, steps
     if len(a) != len(b):
         if len(a) != 1 and len(b) != 1:
             raise ValueError(f"{len(a)} seeds for {len(b)} steps")
-        a, b = (a * len(b), b) if len(a) == 1 else (a, b * len(a))
-    words, n = array("Q", a + b), len(a)
+        a, b = (list(a) * len(b), b) if len(a) == 1 else (a, list(b) * len(a))
+    n, native = len(a), host_python()
+    words = np.empty((2 * n,), dtype=np.uint64)
+    at = words.__array_interface__["data"][0]
+    if native is None or native.ibh_low_words(a, n, at) or native.ibh_low_words(b, n, at + 8 * n):
+        words = array("Q", [int(x) & _M64 for x in a] + [int(x) & _M64 for x in b])
+        at = words.buffer_info()[0]
     out = np.empty((n,), dtype=np.float32)
-    at = words.buffer_info()[0]
     host_library().ibh_uniforms(at, at + 8 * n, n, out.__array_interface__["data"][0])
     return out
+
+
+_NATIVE = []
+
+
+def host_python():
+    """The native functions that read Python's lists (csrc/host_python.cpp), or None where they cannot be built."""
+    if not _NATIVE:
+        import ctypes
+
+        from ..csrc.build import LIBRARIES, build_library
+
+        lib = None
+        if "host_python" in LIBRARIES:
+            lib = ctypes.PyDLL(build_library("host_python"))       # (called with the interpreter's lock held)
+            i, p, o = ctypes.c_int, ctypes.c_void_p, ctypes.py_object
+            lib.ibh_windows.argtypes, lib.ibh_windows.restype = [o, p, p, i, i, p, p], i
+            lib.ibh_low_words.argtypes, lib.ibh_low_words.restype = [o, i, p], i
+        _NATIVE.append(lib)
+    return _NATIVE[0]

@@ -13,7 +13,7 @@ import numpy as np
 import torch
 
 from .. import kernels
-from .params import SamplingParams, uniforms_for
+from .params import SamplingParams, host_python, uniforms_for
 
 
 class Sampler:
@@ -44,9 +44,26 @@ class Sampler:
         slot[0].numpy()[:n] = words
         dev = torch.empty((n,), dtype=torch.int32, device=self.device)
         dev.copy_(slot[0][:n], non_blocking=True)
-        slot[1] = torch.cuda.Event()
+        if slot[1] is None:
+            slot[1] = torch.cuda.Event()
         slot[1].record()
         return dev
+
+    @staticmethod
+    def _windows_natively(last, histories, pend, width: int, words: np.ndarray, counts: np.ndarray) -> bool:
+        """The windows of :meth:`sample` through csrc/host_python.cpp; False where it does not take these histories."""
+        native = host_python()
+        n = min(len(last), len(histories), len(pend))
+        if native is None or n != len(counts) or any(type(k) is not int or k > 0x7fffffff for k in last):
+            return False
+        lists = histories if type(histories) is list else list(histories)
+        if any(type(h) is not list for h in lists):
+            lists = [h if type(h) is list else [] if k <= x else h.tail(k - x) if hasattr(h, "tail") else h
+                     for k, h, x in zip(last, lists, pend)]
+        sizes = np.array([last[:n], pend[:n]], dtype=np.int32)
+        at = sizes.__array_interface__["data"][0]
+        return native.ibh_windows(lists, at, at + 4 * n, n, width, words.__array_interface__["data"][0],
+                                  counts.__array_interface__["data"][0]) == 0
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], seeds: Sequence[int],
                histories: Sequence[Sequence[int]], pending: "int | Sequence[int]" = 0,
@@ -80,7 +97,8 @@ class Sampler:
             raise ValueError("pending: 0 or 1, one for all rows or one per row")
         if len(params) not in (1, r):
             raise ValueError(f"options of {len(params)} rows for {r}")
-        length = [(h.n_tokens if hasattr(h, "n_tokens") else len(h)) + x for h, x in zip(histories, pend)]
+        length = [(len(h) if type(h) is list else h.n_tokens if hasattr(h, "n_tokens") else len(h)) + x
+                  for h, x in zip(histories, pend)]
         # rows that share an options object share its numbers (looked up within this call only): as many columns as objects
         own = list({id(p): p for p in params}.values())
         on = [p.has_penalty for p in own]
@@ -116,7 +134,7 @@ class Sampler:
         words[7 * r:8 * r] = top_k
         n_prev = words[8 * r:9 * r]
         n_prev[:] = 0
-        if width:
+        if width and not self._windows_natively(last, histories, pend, width, words[9 * r:9 * r + r * width], n_prev):
             # the windows, row by row: -1 in the place of the pending token, the history's tail, -1 up to the width.  The
             # window's order does not matter: the pending token, if any, takes the first place.
             windows, counts, blank = array("i"), [], array("i", [-1]) * width

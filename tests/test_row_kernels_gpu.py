@@ -65,6 +65,6 @@ def test_heads_normed_and_gated(e_dim, gate_act, normed, shared, dtype):
             z = wide[:, offset:offset + heads * e_dim].double().reshape(n, heads, e_dim)
             want = (v * (torch.sigmoid(z) * (z if gate_act == 0 else 1))).reshape(n, -1)
             out = torch.empty((n, heads * e_dim), dtype=dtype, device="cuda")
-            K.head_norm_gate(o.cuda(), wide.cuda()[:, offset:], w.cuda(), normed,
+            K.head_norm_gate(o.cuda(), wide.cuda()[:, offset:offset + heads * e_dim], w.cuda(), normed,
                              K.GATE_SILU if gate_act == 0 else K.GATE_SIGMOID, eps, out)
             assert near(out, want)
