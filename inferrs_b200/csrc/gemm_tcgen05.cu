@@ -598,11 +598,13 @@ constexpr int WARPS = 8, THREADS = 32 * WARPS;
 constexpr int BK = 64;
 constexpr int SMEM_MOST = 113 * 1024;             // two CTAs per SM: the next product fetches while this one ends
 
-template <int R, bool GATED, int TOK> struct Shape {
+// DEEP: a CTA per SM with twice the ring, for products whose CTAs are no more than the SMs and whose K is long.
+template <int R, bool GATED, int TOK, bool DEEP = false> struct Shape {
+    static constexpr int SMEM_MOST = (DEEP ? 2 : 1) * rows::SMEM_MOST;
     static constexpr int W_BYTES = R * 128, X_BYTES = TOK * 128;
     static constexpr int STAGE = (GATED ? 2 : 1) * W_BYTES + X_BYTES;
     static constexpr int FIT = (SMEM_MOST - 640) / (WARPS * STAGE);
-    static constexpr int STAGES = FIT > 8 ? 8 : FIT;   // per warp
+    static constexpr int STAGES = FIT > (DEEP ? 10 : 8) ? (DEEP ? 10 : 8) : FIT;   // per warp
     static constexpr int TILES = (R + 15) / 16;   // of 16 rows, of each matrix
     static constexpr int SUMS = WARPS * TOK * R * (GATED ? 2 : 1) * 4;    // the warps' sums, over the rings
     static constexpr size_t smem = (size_t)WARPS * STAGES * STAGE + WARPS * STAGES * 8 + TOK * 4;
@@ -617,10 +619,10 @@ __device__ __forceinline__ void mma16816(float (&c)[4], unsigned a0, unsigned a1
 }
 
 // BATCH: blockIdx.y numbers the products of a batch (plain ones); x, w and y of product b lie a stride after those of b - 1.
-template <int R, bool GATED, int TOK, bool BATCH>
-__global__ void __launch_bounds__(THREADS, 2) rows_kernel(const __grid_constant__ CUtensorMap map_w,
+template <int R, bool GATED, int TOK, bool BATCH, bool DEEP>
+__global__ void __launch_bounds__(THREADS, DEEP ? 1 : 2) rows_kernel(const __grid_constant__ CUtensorMap map_w,
                                                           const __grid_constant__ CUtensorMap map_x, const tc::Params p) {
-    using S = Shape<R, GATED, TOK>;
+    using S = Shape<R, GATED, TOK, DEEP>;
     constexpr int MATS = GATED ? 2 : 1, TILES = S::TILES, NT = TOK / 8;
     extern __shared__ __align__(1024) unsigned char rows_smem[];             // (the swizzle counts from multiples of 1 KB)
     unsigned char* smem = rows_smem;
@@ -783,11 +785,11 @@ __global__ void __launch_bounds__(THREADS, 2) rows_kernel(const __grid_constant_
     }
 }
 
-template <int R, bool GATED, int TOK, bool BATCH>
+template <int R, bool GATED, int TOK, bool BATCH, bool DEEP>
 static int launch_maps(const CUtensorMap& mw, const CUtensorMap& mx, const tc::Params& p, int batch, cudaStream_t stream) {
-    using S = Shape<R, GATED, TOK>;
+    using S = Shape<R, GATED, TOK, DEEP>;
     static IbDeviceSet allowed;
-    if (const int e = ib_allow_dynamic_smem(allowed, rows_kernel<R, GATED, TOK, BATCH>, S::smem)) return e;
+    if (const int e = ib_allow_dynamic_smem(allowed, rows_kernel<R, GATED, TOK, BATCH, DEEP>, S::smem)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.n_out + R - 1) / R, batch);
     cfg.blockDim = dim3(THREADS);
@@ -798,15 +800,15 @@ static int launch_maps(const CUtensorMap& mw, const CUtensorMap& mx, const tc::P
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = tc::g_pdl ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, rows_kernel<R, GATED, TOK, BATCH>, mw, mx, p);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, rows_kernel<R, GATED, TOK, BATCH, DEEP>, mw, mx, p);
     return e == cudaSuccess ? ib_launch_status() : (int)e;
 }
 
-template <int R, bool GATED, int TOK>
+template <int R, bool GATED, int TOK, bool DEEP = false>
 static int launch(const void* w, long n_w, long ldw, const void* x, long ldx, int k, const tc::Params& p, cudaStream_t stream) {
     CUtensorMap mw, mx;
     if (!tc::make_map(&mw, w, n_w, k, ldw, R) || !tc::make_map(&mx, x, p.n_tok, k, ldx, TOK)) return IB_ERR_UNSUPPORTED;
-    return launch_maps<R, GATED, TOK, false>(mw, mx, p, 1, stream);
+    return launch_maps<R, GATED, TOK, false, DEEP>(mw, mx, p, 1, stream);
 }
 
 // a batch of row-major [rows, k] bfloat16 matrices `stride` elements apart, boxes of [box_rows, 64] of one of them
@@ -827,7 +829,7 @@ static int launch_batch(const void* w, const void* x, long ldx, long bx, int k, 
     CUtensorMap mw, mx;
     if (!make_batch_map(&mw, w, p.n_out, k, k, (long)p.n_out * k, batch, R) ||
         !make_batch_map(&mx, x, p.n_tok, k, ldx, bx, batch, TOK)) return IB_ERR_UNSUPPORTED;
-    return launch_maps<R, false, TOK, true>(mw, mx, p, batch, stream);
+    return launch_maps<R, false, TOK, true, false>(mw, mx, p, batch, stream);
 }
 
 // R rows of W per CTA (gated: of each of the two matrices)
@@ -839,6 +841,9 @@ static int launch_any(int r, const void* w, long n_w, long ldw, const void* x, l
         case 16: return few ? launch<16, GATED, 8>(w, n_w, ldw, x, ldx, k, p, stream) : launch<16, GATED, 16>(w, n_w, ldw, x, ldx, k, p, stream);
         case 24: return few ? launch<24, GATED, 8>(w, n_w, ldw, x, ldx, k, p, stream) : IB_ERR_UNSUPPORTED;
         case 32: if constexpr (!GATED) return few ? launch<32, GATED, 8>(w, n_w, ldw, x, ldx, k, p, stream) : launch<32, GATED, 16>(w, n_w, ldw, x, ldx, k, p, stream);
+        case 1016: if constexpr (!GATED) return few ? launch<16, GATED, 8, true>(w, n_w, ldw, x, ldx, k, p, stream) : launch<16, GATED, 16, true>(w, n_w, ldw, x, ldx, k, p, stream);
+        case 1024: if constexpr (!GATED) return few ? launch<24, GATED, 8, true>(w, n_w, ldw, x, ldx, k, p, stream) : launch<24, GATED, 16, true>(w, n_w, ldw, x, ldx, k, p, stream);
+        case 1032: if constexpr (!GATED) return few ? launch<32, GATED, 8, true>(w, n_w, ldw, x, ldx, k, p, stream) : launch<32, GATED, 16, true>(w, n_w, ldw, x, ldx, k, p, stream);
         case 48: if constexpr (!GATED) return few ? launch<48, GATED, 8>(w, n_w, ldw, x, ldx, k, p, stream) : IB_ERR_UNSUPPORTED;
     }
     return IB_ERR_UNSUPPORTED;
@@ -861,7 +866,8 @@ static int rows_form(int n_tok, int n_out, int num_kb, int gated) {
     if (n_tok <= 8) {
         if (gated) return 24;
         if (n_out <= 24 * 148 && num_kb <= 64) return 24;
-        return n_out <= 32 * RESIDENT ? 32 : n_out <= 48 * RESIDENT ? 48 : 0;
+        // (151,936 over 1,024 and 4,096, one token: tcgen05 56 and 189, 48 rows 48 and 180; 32,000 over 2,048: 21.7 / 22.9)
+        return n_out <= 32 * RESIDENT ? 32 : n_out <= 48 * RESIDENT || n_out >= 4 * 48 * RESIDENT ? 48 : 0;
     }
     if (n_tok > 16) return 0;
     if (gated) return n_out <= 16 * RESIDENT ? 16 : 0;
@@ -968,7 +974,7 @@ static int gemm_tn(const void* x, long ldx, const void* w, long ldw, void* y, lo
     p.gelu = gelu;
     p.in_ssq = f.in_ssq; p.n_in_parts = f.n_in_parts; p.in_eps = f.in_eps; p.in_inv_width = f.in_width > 0 ? 1.0f / (float)f.in_width : 0.0f;
     p.residual = f.residual; p.ld_res = f.ld_res; p.sink_w = f.sink_w; p.sink_w_is_f32 = f.sink_w_is_f32; p.out_ssq = f.out_ssq;
-    if (const int r = split_k < 0 ? -split_k : split_k == 0 ? rows_form(n_tok, n_out, p.num_kb, 0) : 0) {
+    if (const int r = split_k < -1 ? -split_k : split_k == -1 ? rows_form(n_tok, n_out, p.num_kb, 0) : 0) {
         if (n_tok > 16) return IB_ERR_UNSUPPORTED;
         return rows::launch_any<false>(r, w, n_out, ldw, x, ldx, k, p, stream);
     }
@@ -1008,7 +1014,7 @@ IB_EXPORT int ib_gemm_tn_rows_batched(const void* x, long ldx, long bx, const vo
 
 // x [n_tok, k] (row stride ldx), w [n_out, k] (row stride ldw), both bfloat16; y [n_tok, n_out] bfloat16 or float32.
 // split_k: 0 lets the function choose (1, 2, 4 or 8 CTAs per output tile); 8 is taken for up to 32 tokens (4 stands in beyond);
-// -r: the kernel without clusters, r rows of w per CTA.
+// -1: it also chooses between this kernel and the one without clusters; -r: the latter, r rows of w per CTA.
 IB_EXPORT int ib_gemm_tn_tcgen05(const void* x, long ldx, const void* w, long ldw, void* y, long ldy, int y_is_f32,
                                  int n_tok, int n_out, int k, int split_k, cudaStream_t stream) {
     const Folded none = {nullptr, 0, 0.0f, 0, nullptr, 0, nullptr, 0, nullptr};
@@ -1040,7 +1046,7 @@ IB_EXPORT int ib_gemm_tcgen05_ssq_parts(int n_tok, int n_out, int k, int split_k
     if (n_tok <= 0 || n_out <= 0 || k <= 0) return IB_ERR_ARGUMENT;
     const int bn = bn_for(n_tok);
     if (bn > 32) return IB_ERR_UNSUPPORTED;
-    if (const int r = split_k < 0 ? -split_k : split_k == 0 ? rows_form(n_tok, n_out, (k + tc::BK - 1) / tc::BK, 0) : 0)
+    if (const int r = split_k < -1 ? -split_k : split_k == -1 ? rows_form(n_tok, n_out, (k + tc::BK - 1) / tc::BK, 0) : 0)
         return (n_out + r - 1) / r;
     const int splits = choose_splits(n_tok, n_out, (k + tc::BK - 1) / tc::BK, bn, split_k);
     const int rows = tile_rows_for(n_out, splits, tc::BM, resident_for(bn, splits));

@@ -990,6 +990,7 @@ def gemm_tn_bf16(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor):
         gemm_tn_simt(x, w, out, torch.bfloat16)
 
 
+ANY_FORM = -1  # split_k of gemm_tn_tcgen05: the library chooses the kernel too
 SSQ_LD = 32   # tokens per part of a list of sums of squares (csrc/gemm_tcgen05.cu)
 
 
@@ -1143,14 +1144,14 @@ def linear(x, w: torch.Tensor, out: torch.Tensor, act_dtype: torch.dtype, sink: 
         if not folded_norm_supported(rows, act_dtype, w):
             raise KernelError(f"linear: {rows} rows of {act_dtype} with a {w.dtype} weight cannot take folded norms; "
                               f"ask folded_norm_supported first")
-        return gemm_tn_tcgen05(x, w, out, sink=sink)
+        return gemm_tn_tcgen05(x, w, out, ANY_FORM, sink=sink)
     if act_dtype == torch.float32 or w.dtype == torch.float32:
         if act_dtype == torch.float32 and gemm_split_supported(x, w, out):
             gemm_tn_split(x, w, out)
         else:
             gemm_tn_simt(x, w, out, act_dtype)
     elif x.shape[0] <= TCGEN05_MAX_TOKENS and tcgen05_gemm_supported(x, w):
-        gemm_tn_tcgen05(x, w, out)
+        gemm_tn_tcgen05(x, w, out, ANY_FORM)
     else:
         gemm_tn_bf16(x, w, out)
     return None
@@ -1161,7 +1162,7 @@ def gelu_linear(x, w: torch.Tensor, out: torch.Tensor, act_dtype: torch.dtype):
     everything else as the product and the kernel over its rows."""
     if act_dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[0] <= TCGEN05_MAX_TOKENS \
             and tcgen05_gemm_supported(x, w):
-        gemm_tn_tcgen05(x, w, out, gelu=True)
+        gemm_tn_tcgen05(x, w, out, ANY_FORM, gelu=True)
         return
     linear(x, w, out, act_dtype)
     gelu_rows(out, out)
@@ -1177,12 +1178,12 @@ def gated_linear(x, w_gate_up: torch.Tensor, out: torch.Tensor, act_dtype: torch
     if isinstance(x, ScaledRows):
         if not folded_norm_supported(x.shape[0], act_dtype, w_gate_up) or x.shape[0] > SWIGLU_MAX_TOKENS:
             raise KernelError("gated_linear: these rows cannot take a folded norm; ask folded_norm_supported first")
-        gemm_swiglu_tcgen05(x, w_gate_up, out)
+        gemm_swiglu_tcgen05(x, w_gate_up, out, 0)
         return
     if act_dtype == torch.bfloat16 and w_gate_up.dtype == torch.bfloat16 \
             and x.shape[0] <= min(TCGEN05_MAX_TOKENS, SWIGLU_MAX_TOKENS) \
             and tcgen05_gemm_supported(x, w_gate_up):
-        gemm_swiglu_tcgen05(x, w_gate_up, out)
+        gemm_swiglu_tcgen05(x, w_gate_up, out, 0)
         return
     gu = torch.empty((x.shape[0], 2 * inner), dtype=act_dtype, device=x.device)
     linear(x, w_gate_up, gu, act_dtype)
@@ -2249,7 +2250,8 @@ def _scaled_args(x):
 def gemm_tn_tcgen05(x, w: torch.Tensor, out: torch.Tensor, split_k: int = 0, sink: Optional[ResidualSink] = None,
                     gelu: bool = False):
     """out = x @ w.T with TMA-fed tcgen05 MMAs: W is the 128-row operand, the tokens are the N dimension.
-    ``split_k`` 0 lets the kernel library choose how many CTAs of a cluster share one output tile.  ``x`` may be
+    ``split_k`` 0 lets the kernel library choose how many CTAs of a cluster share one output tile, -1 (ANY_FORM) also
+    between that kernel and the one without clusters (up to 16 rows of x), -r names the latter with r rows of w per CTA.  ``x`` may be
     :class:`ScaledRows` and the result may go to a :class:`ResidualSink` (both: up to 32 rows, bfloat16 out); with a
     sink the :class:`ScaledRows` that stand for the next norm's output are returned.  ``gelu``: out = gelu_tanh(x @ w.T)
     (plain rows, no sink)."""
@@ -2295,10 +2297,11 @@ def gemm_tn_tcgen05(x, w: torch.Tensor, out: torch.Tensor, split_k: int = 0, sin
     return result
 
 
-def gemm_swiglu_tcgen05(x, w_gate_up: torch.Tensor, out: torch.Tensor, rows_per_cta: int = 0):
+def gemm_swiglu_tcgen05(x, w_gate_up: torch.Tensor, out: torch.Tensor, rows_per_cta: int = -1):
     """out[t, f] = silu(x[t] . w[f]) * (x[t] . w[inner + f]): both products of a gated feed-forward and the gate
     in one tcgen05 kernel (up to 64 gate rows and the same up rows per tile).  Up to 32 rows of x, which may be
-    :class:`ScaledRows`."""
+    :class:`ScaledRows`.  ``rows_per_cta`` 0 lets the library choose between that kernel and the one without clusters,
+    which takes up to 16 rows; 16 or 24: the latter with so many rows of each matrix per CTA."""
     xt, scaled = _scaled_args(x)
     _need(xt, "x", (torch.bfloat16,), 2)
     _need(w_gate_up, "w_gate_up", (torch.bfloat16,), 2)
