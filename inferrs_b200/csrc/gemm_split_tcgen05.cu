@@ -20,7 +20,7 @@
 //   warps 2-3   x's pieces, to three swizzled tiles in shared memory (the products' B operand)
 //   warps 4-7   W's pieces: a thread reads its row from the stage and writes the three pieces to tensor memory (the
 //               products' A operand, so that W's pieces never pass through shared memory again)
-//   warps 8-11  the sums
+//   warps 8-    the sums: four warps, or beyond 16 tokens eight with half of the tokens each
 //
 // Infinities and NaN: the pieces of an infinity are no numbers, so a result that is not finite is computed again as
 // one chain of fused multiply-adds, by the thread that would store it.  Numbers below 2^-102 have pieces that bfloat16 holds only
@@ -41,7 +41,7 @@ constexpr int BM = 128;                 // rows of W per tile at most (the produ
 constexpr int KS = 32;                  // k per stage of the ring: 32 floats = one 128-byte swizzle row
 constexpr int BK = 64;                  // k per block: two stages, one round of products
 constexpr int SEGMENTS = 8;
-constexpr int THREADS = 384;
+constexpr int SUM_WARP0 = 8;           // the first of the warps that add up
 constexpr int W_STAGE = BM * KS * 4;
 
 __device__ int g_error = 0;             // 0 ok; else (role code) of the first wait that ran out
@@ -65,6 +65,13 @@ __device__ __forceinline__ void cluster_arrive() {
 __device__ __forceinline__ void cluster_wait() {
     __syncwarp();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// one lane of a warp that is here as a whole; the compiler knows that it is one, and keeps what it computes for the
+// tensor cores' descriptors out of the lanes' own registers
+__device__ __forceinline__ bool elect_one() {
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
 }
 __device__ __forceinline__ unsigned cluster_rank() {
     unsigned r;
@@ -100,64 +107,45 @@ __device__ __forceinline__ float finished(const Params& p, float v, int tok, int
 }
 
 // A segment's sum joins those before it: like the carry of a binary counter, so that equal powers of two of segments
-// are added to each other.  Where the waiting sums stay: up to 16 tokens in registers, of 32 in tensor memory; of 64 single
-// segments in tensor memory, pairs in shared memory (where the cluster's parts come later) and fours, which only a CTA
-// without a cluster has, in y.
-template <int BN> struct Waiting {
-    float v[3][BN <= 16 ? BN : 1];
-    unsigned tmem;                      // of this warp's lanes: regions of BN columns
-    float* pairs;                       // of this thread: [BN] numbers BM apart
-    float* fours;                       // ... ldy apart; the first `fit` of them are this product's
-    long ldy;
-    int fit;
+// are added to each other.  A thread has C numbers: 16, all waiting sums in registers; or 32, single segments in tensor memory, pairs
+// in shared memory (where the cluster's parts come later) and fours in registers.
+template <int C> struct Waiting {
+    float v[C <= 16 ? 3 : 1][C];
+    unsigned tmem;                      // of this warp's lanes
+    float* pairs;                       // of this thread: C numbers BM apart
 
-    template <int L> __device__ __forceinline__ void add(float (&s)[BN]) {
-        if constexpr (BN <= 16) {
+    template <int L> __device__ __forceinline__ void add(float (&s)[C]) {
+        if constexpr (C > 16 && L == 0) {
+            unsigned t[32];
+            tmem_ld32_issue(tmem, t);
+            tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < BN; ++j) s[j] = v[L][j] + s[j];
-        } else if constexpr (BN <= 32 || L == 0) {
+            for (int j = 0; j < C; ++j) s[j] = __uint_as_float(t[j]) + s[j];
+        } else if constexpr (C > 16 && L == 1) {
 #pragma unroll
-            for (int c = 0; c < BN; c += 16) {
-                float t[16];
-                tmem_ld16(tmem + L * BN + c, t);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) s[c + j] = t[j] + s[c + j];
-            }
-        } else if constexpr (L == 1) {
-#pragma unroll
-            for (int j = 0; j < BN; ++j) s[j] = pairs[j * BM] + s[j];
+            for (int j = 0; j < C; ++j) s[j] = pairs[j * BM] + s[j];
         } else {
-            const float* f = fours;
 #pragma unroll
-            for (int j = 0; j < BN; ++j, f += ldy)
-                if (j < fit) s[j] = *f + s[j];
+            for (int j = 0; j < C; ++j) s[j] = v[C <= 16 ? L : 0][j] + s[j];
         }
     }
-    template <int L> __device__ __forceinline__ void put(const float (&s)[BN]) {
-        if constexpr (BN <= 16) {
+    template <int L> __device__ __forceinline__ void put(const float (&s)[C]) {
+        if constexpr (C > 16 && L == 0) {
+            unsigned t[32];
 #pragma unroll
-            for (int j = 0; j < BN; ++j) v[L][j] = s[j];
-        } else if constexpr (BN <= 32 || L == 0) {
-#pragma unroll
-            for (int c = 0; c < BN; c += 16) {
-                unsigned t[16];
-#pragma unroll
-                for (int j = 0; j < 16; ++j) t[j] = __float_as_uint(s[c + j]);
-                tmem_st16(tmem + L * BN + c, t);
-            }
+            for (int j = 0; j < C; ++j) t[j] = __float_as_uint(s[j]);
+            tmem_st32(tmem, t);
             tmem_st_wait();
-        } else if constexpr (L == 1) {
+        } else if constexpr (C > 16 && L == 1) {
 #pragma unroll
-            for (int j = 0; j < BN; ++j) pairs[j * BM] = s[j];
+            for (int j = 0; j < C; ++j) pairs[j * BM] = s[j];
         } else {
-            float* f = fours;
 #pragma unroll
-            for (int j = 0; j < BN; ++j, f += ldy)
-                if (j < fit) *f = s[j];
+            for (int j = 0; j < C; ++j) v[C <= 16 ? L : 0][j] = s[j];
         }
     }
     // `n`: segments that this CTA has summed before; `last`: s is complete once everything that waits has joined
-    __device__ __forceinline__ void join(float (&s)[BN], int n, bool last) {
+    __device__ __forceinline__ void join(float (&s)[C], int n, bool last) {
         if (!(n & 1)) { if (!last) put<0>(s); return; }
         add<0>(s);
         if (!(n & 2)) { if (!last) put<1>(s); return; }
@@ -172,8 +160,11 @@ constexpr size_t smem_bytes() {
     return 1024 + (size_t)STAGES * (W_STAGE + BN * KS * 4) + 2 * 3 * BN * BK * 2 + (size_t)BN * BM * 4 + 256;
 }
 
+constexpr int sum_warps(int bn) { return bn <= 16 ? 4 : 8; }
+constexpr int threads_of(int bn) { return 32 * (SUM_WARP0 + sum_warps(bn)); }
+
 template <int BN, int STAGES>
-__global__ void __launch_bounds__(THREADS, (BN <= 16 ? 2 : 1)) split_kernel(const __grid_constant__ CUtensorMap map_w,
+__global__ void __launch_bounds__(threads_of(BN), (BN <= 16 ? 2 : 1)) split_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                            const __grid_constant__ CUtensorMap map_x,
                                                                            const Params p) {
     constexpr int X_STAGE = BN * KS * 4, PIECE = BN * BK * 2;
@@ -181,7 +172,8 @@ __global__ void __launch_bounds__(THREADS, (BN <= 16 ? 2 : 1)) split_kernel(cons
     // accumulators: of the largest product per block parity, and of the others (two sizes side by side)
     constexpr int TMEM_ACC = 2 * A_COLS, TMEM_SMALL = TMEM_ACC + 2 * BN, TMEM_WAITING = TMEM_SMALL + 2 * BN;
     constexpr int TMEM_COLS = BN <= 16 ? 256 : 512;
-    static_assert(TMEM_WAITING + (BN <= 16 ? 0 : BN <= 32 ? 3 * BN : BN) <= TMEM_COLS, "");
+    constexpr int SUM_WARPS = sum_warps(BN), C = BN * 4 / SUM_WARPS;         // C: tokens of a thread that adds up
+    static_assert(TMEM_WAITING + (C > 16 ? BN : 0) <= TMEM_COLS && (C == 16 || C == 32), "");
     static_assert((2 * STAGES + 7) * 8 + 8 <= 256, "");
     extern __shared__ unsigned char raw_smem[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~(uintptr_t)1023);
@@ -197,7 +189,7 @@ __global__ void __launch_bounds__(THREADS, (BN <= 16 ? 2 : 1)) split_kernel(cons
     const unsigned small0 = smem_u32(bars + 2 * STAGES + 6); // a segment's small products have been read
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 2 * STAGES + 7);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int splits = gridDim.z;
     const int tok0 = blockIdx.y * BN, feat0 = blockIdx.x * p.tile_rows;
     const int my_segments = SEGMENTS / splits;
@@ -209,8 +201,8 @@ __global__ void __launch_bounds__(THREADS, (BN <= 16 ? 2 : 1)) split_kernel(cons
     ib_grid_dependency_launch();
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 6); }
-        for (int s = 0; s < 2; ++s) { mbar_init(ready0 + 8 * s, 6); mbar_init(done0 + 8 * s, 1); mbar_init(taken0 + 8 * s, 4); }
-        mbar_init(small0, 4);
+        for (int s = 0; s < 2; ++s) { mbar_init(ready0 + 8 * s, 6); mbar_init(done0 + 8 * s, 1); mbar_init(taken0 + 8 * s, SUM_WARPS); }
+        mbar_init(small0, SUM_WARPS);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -220,7 +212,7 @@ __global__ void __launch_bounds__(THREADS, (BN <= 16 ? 2 : 1)) split_kernel(cons
     fence_before();
     __syncthreads();
     fence_after();
-    const unsigned tmem = *tmem_slot;
+    const unsigned tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     bool ok = true;
     // A CTA's shared memory may be written by its cluster only once the CTA runs and, beyond 32 tokens, keeps nothing there
     // any more: every CTA says so and looks at the others' word just before its first store to them.
@@ -259,7 +251,7 @@ __global__ void __launch_bounds__(THREADS, (BN <= 16 ? 2 : 1)) split_kernel(cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const unsigned idesc1 = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(BM >> 4) << 24);
             const unsigned idesc2 = idesc1 + ((unsigned)(BN >> 3) << 17);        // two pieces of x side by side
             int m = 0, segment = 0;
@@ -287,7 +279,7 @@ __global__ void __launch_bounds__(THREADS, (BN <= 16 ? 2 : 1)) split_kernel(cons
             }
         }
     } else if (warp < 4) {
-        const int e = (int)threadIdx.x - 64;
+        const int e = (int)threadIdx.x - 64, r0 = ((e >> 3) & 1) + ((e >> 4) & 1) * 4 + (e >> 5) * 2;
         for (int i = 0; i < n_blocks && ok; ++i) {
             const int b = i & 1;
             if (i >= 2 && !mbar_wait(done0 + 8 * b, ((i >> 1) - 1) & 1, 6)) ok = false;
@@ -298,15 +290,15 @@ __global__ void __launch_bounds__(THREADS, (BN <= 16 ? 2 : 1)) split_kernel(cons
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 float4 v[BN / 8];                            // four numbers of a row at a time, all asked for together
-                const int c = e & 7;
+                const int c = e & 7;                         // (a warp's rows differ in bit 2: its stores meet all banks)
 #pragma unroll
                 for (int j = 0; j < BN / 8; ++j) {
-                    const int r = (e >> 3) + j * 8;
+                    const int r = r0 + j * 8;
                     v[j] = *reinterpret_cast<const float4*>(x_ring + s * X_STAGE + r * 128 + ((c ^ (r & 7)) << 4));
                 }
 #pragma unroll
                 for (int j = 0; j < BN / 8; ++j) {
-                    const int r = (e >> 3) + j * 8;
+                    const int r = r0 + j * 8;
                     uint2 w0, w1, w2;
                     split_pair(v[j].x, v[j].y, w0.x, w1.x, w2.x);
                     split_pair(v[j].z, v[j].w, w0.y, w1.y, w2.y);
@@ -360,36 +352,31 @@ __global__ void __launch_bounds__(THREADS, (BN <= 16 ? 2 : 1)) split_kernel(cons
         }
     } else {
         ib_grid_dependency_wait();                           // y may still be read by the kernel before; x, if read again
-        const unsigned lanes = tmem + ((unsigned)(q * 32) << 16);
+        const int col0 = ((warp - SUM_WARP0) >> 2) * C;      // this warp's tokens
+        const unsigned lanes = tmem + ((unsigned)(q * 32) << 16) + col0;
         const int feature = feat0 + row;
-        Waiting<BN> waiting;
+        Waiting<C> waiting;
         waiting.tmem = lanes + TMEM_WAITING;
-        waiting.pairs = recv + row;
-        waiting.fours = p.y + (long)tok0 * p.ldy + feature;
-        waiting.ldy = p.ldy;
-        waiting.fit = row < p.tile_rows && feature < p.n_out ? p.n_tok - tok0 : 0;
-        float sum[BN];
+        waiting.pairs = recv + col0 * BM + row;
+        float sum[C];
         auto add = [&](unsigned at) {
-            if constexpr (BN <= 16) {
+            if constexpr (C == 16) {
                 float v[16];
                 tmem_ld16(at, v);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) sum[j] += v[j];
             } else {
+                unsigned v[32];
+                tmem_ld32_issue(at, v);
+                tmem_ld_wait();
 #pragma unroll
-                for (int c = 0; c < BN; c += 32) {
-                    unsigned v[32];
-                    tmem_ld32_issue(at + c, v);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) sum[c + j] += __uint_as_float(v[j]);
-                }
+                for (int j = 0; j < 32; ++j) sum[j] += __uint_as_float(v[j]);
             }
         };
         int i = 0;
         for (int g = 0; g < my_segments && ok; ++g) {
 #pragma unroll
-            for (int j = 0; j < BN; ++j) sum[j] = 0.0f;
+            for (int j = 0; j < C; ++j) sum[j] = 0.0f;
             for (int m = 0; m < p.blocks_per_segment && i < n_blocks; ++m, ++i) {
                 const int b = i & 1;
                 ok = mbar_wait(done0 + 8 * b, (i >> 1) & 1, 8);
@@ -412,10 +399,10 @@ __global__ void __launch_bounds__(THREADS, (BN <= 16 ? 2 : 1)) split_kernel(cons
         }
         if (splits == 1) {
             if (ok && row < p.tile_rows && feature < p.n_out) {
-                float* y = p.y + (long)tok0 * p.ldy + feature;
+                float* y = p.y + (long)(tok0 + col0) * p.ldy + feature;
 #pragma unroll
-                for (int j = 0; j < BN; ++j, y += p.ldy)
-                    if (tok0 + j < p.n_tok) *y = finished(p, sum[j], tok0 + j, feature);
+                for (int j = 0; j < C; ++j, y += p.ldy)
+                    if (tok0 + col0 + j < p.n_tok) *y = finished(p, sum[j], tok0 + col0 + j, feature);
             }
         } else {
             // every CTA of the cluster owns an equal share of the tile's rows: its neighbours' branches of the sums come
@@ -426,16 +413,16 @@ __global__ void __launch_bounds__(THREADS, (BN <= 16 ? 2 : 1)) split_kernel(cons
             cluster_wait();
             if (ok && row < p.tile_rows) {
                 const unsigned owner = (unsigned)(row / owned);
-                float* slot = recv + (size_t)my_rank * BN * owned + (row - (int)owner * owned);
+                float* slot = recv + ((size_t)my_rank * BN + col0) * owned + (row - (int)owner * owned);
 #pragma unroll
-                for (int j = 0; j < BN; ++j)
-                    if (tok0 + j < p.n_tok) st_cluster(smem_u32(slot + j * owned), owner, sum[j]);
+                for (int j = 0; j < C; ++j)
+                    if (tok0 + col0 + j < p.n_tok) st_cluster(smem_u32(slot + j * owned), owner, sum[j]);
             }
             cluster_arrive();
             cluster_wait();
             if (ok && g_error == 0) {
                 const int per = BN * owned;
-                for (int idx = row; idx < per; idx += 128) {
+                for (int idx = (int)threadIdx.x - 32 * SUM_WARP0; idx < per; idx += 32 * SUM_WARPS) {
                     const int tok = tok0 + idx / owned, f = feat0 + (int)my_rank * owned + idx % owned;
                     if (tok >= p.n_tok || f >= p.n_out) continue;
                     const float* part = recv + idx;
@@ -449,7 +436,7 @@ __global__ void __launch_bounds__(THREADS, (BN <= 16 ? 2 : 1)) split_kernel(cons
             }
         }
     }
-    if (splits > 1 && warp < 8) {      // the other warps' part in the cluster's two barriers
+    if (splits > 1 && warp < SUM_WARP0) {      // the other warps' part in the cluster's two barriers
         if (BN > 32) cluster_arrive();
         cluster_wait();
         cluster_arrive();
@@ -489,7 +476,7 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p,
     if (const int e = ib_allow_dynamic_smem(allowed, split_kernel<BN, STAGES>, smem)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.n_out + p.tile_rows - 1) / p.tile_rows, (p.n_tok + BN - 1) / BN, splits);
-    cfg.blockDim = dim3(THREADS);
+    cfg.blockDim = dim3(threads_of(BN));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
