@@ -317,7 +317,9 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
     __nv_bfloat16* p_s = c_s + LM_KEYS * LDC;                                // [TT * 16][LDP]
     float* pmax = reinterpret_cast<float*>(p_s + MR * LDP);                  // [4][TT * 16]
     float* psum = pmax + 4 * MR;                                             // [4][TT * 16]
-    ib_grid_dependency_sync();
+    // a row's place and the cached vectors of earlier steps are fetched while the kernel ahead still runs, one token a block
+    ib_grid_dependency_launch();
+    if (TT > 1) ib_grid_dependency_wait();
     const int slice = blockIdx.z, head0 = blockIdx.y * LM_ROWS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kw = warp & 3, ts0 = (warp >> 2) * TS;     // this warp's 16 keys of a tile, its first token
@@ -340,27 +342,12 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
     const int per_slice = (n_tiles + n_slices - 1) / n_slices;
     const int t0 = slice * per_slice, t1 = min(n_tiles, t0 + per_slice);
 
-    // the queries of the group's heads (rows of heads and tokens that do not exist are zeros)
-    for (int i = threadIdx.x; i < MR * (R / 8); i += blockDim.x) {
-        const int m = i / (R / 8), ch = i % (R / 8);
-        const int tok = m / LM_ROWS, h = head0 + m % LM_ROWS;
-        const bool ok = h < n_heads && tok < n_tok;
-        const __nv_bfloat16* src = q + (long)(row + (ok ? tok : 0)) * q_row + (long)min(h, n_heads - 1) * q_head + ch * 8;
-        lm_cp_async16(q_s + at(m, LDC, ch * 8), src, ok ? 16 : 0);
-    }
-    if constexpr (ROT) {                              // their rotated parts, turned as they are fetched
-        for (int i = threadIdx.x; i < MR * rot.width; i += blockDim.x) {
-            const int m = i / rot.width, e = i % rot.width;
-            const int tok = m / LM_ROWS, h = head0 + m % LM_ROWS;
-            const bool ok = h < n_heads && tok < n_tok;
-            q_s[at(m, LDC, (R + e) & ~7) + (e & 7)] = __float2bfloat16_rn(ok ? latent_rot_value<__nv_bfloat16>(rot, row + tok, h, e, pos0 + tok) : 0.0f);
-        }
-    }
     // two or four threads per key: each looks the page up and copies its share of the latent
-    auto load_tile = [&](int t) {
+    auto load_tile = [&](int t, bool own, bool others) {    // own: the row's own key
         constexpr int PER = WARPS / 2;                   // threads per key
         const int jj = threadIdx.x / PER, half = threadIdx.x % PER;
         const int j = first + t * LM_KEYS + jj;
+        if (!(j == pos_last ? own : others)) return;
         const __nv_bfloat16* src = plane;
         int bytes = 0;
         if (j >= lo0 && j <= pos_last) {
@@ -375,7 +362,50 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
         if constexpr (ROT)
             for (int ch = R / 8 + half; ch < RK / 8; ch += PER) lm_cp_async16(c_s + at(jj, LDC, ch * 8), bytes ? src + ch * 8 : src, bytes);
     };
-    if (t0 < t1) load_tile(t0);
+    const bool early = TT == 1 && (row == 0 || row_request[row - 1] != req);     // no key but its own is this step's
+    if (TT == 1) {
+        if (early && t0 < t1) load_tile(t0, false, true);
+        ib_grid_dependency_wait();
+    }
+    // the queries of the group's heads (rows of heads and tokens that do not exist are zeros)
+    for (int i = threadIdx.x; i < MR * (R / 8); i += blockDim.x) {
+        const int m = i / (R / 8), ch = i % (R / 8);
+        const int tok = m / LM_ROWS, h = head0 + m % LM_ROWS;
+        const bool ok = h < n_heads && tok < n_tok;
+        const __nv_bfloat16* src = q + (long)(row + (ok ? tok : 0)) * q_row + (long)min(h, n_heads - 1) * q_head + ch * 8;
+        lm_cp_async16(q_s + at(m, LDC, ch * 8), src, ok ? 16 : 0);
+    }
+    if constexpr (ROT) {                              // their rotated parts, turned as they are fetched: eight at a time, all asked for together
+        constexpr int AT_ONCE = 8;
+        const int total = MR * rot.width;
+        for (int i0 = threadIdx.x; i0 < total; i0 += 32 * WARPS * AT_ONCE) {
+            float v[AT_ONCE], w[AT_ONCE], c[AT_ONCE], s[AT_ONCE];
+#pragma unroll
+            for (int u = 0; u < AT_ONCE; ++u) {
+                const int i = i0 + u * 32 * WARPS, m = i / rot.width, e = i - m * rot.width;
+                const int tok = m / LM_ROWS, h = head0 + m % LM_ROWS, pos = pos0 + tok;
+                v[u] = w[u] = s[u] = 0.0f;
+                c[u] = 1.0f;
+                if (i < total && h < n_heads && tok < n_tok && e < rot.src) {
+                    const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(rot.q) + (long)(row + tok) * rot.q_row + (long)h * rot.q_head;
+                    v[u] = ib_to_float(src[e]);
+                    if (e < 2 * rot.half && pos >= 0 && pos < rot.table_rows) {
+                        const int k = e < rot.half ? e : e - rot.half;
+                        w[u] = ib_to_float(src[e < rot.half ? e + rot.half : k]);
+                        c[u] = rot.cos_table[(long)pos * rot.half + k];
+                        s[u] = rot.sin_table[(long)pos * rot.half + k];
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < AT_ONCE; ++u) {
+                const int i = i0 + u * 32 * WARPS, m = i / rot.width, e = i - m * rot.width;
+                if (i < total)
+                    q_s[at(m, LDC, (R + e) & ~7) + (e & 7)] = __float2bfloat16_rn(e < rot.half ? v[u] * c[u] - w[u] * s[u] : v[u] * c[u] + w[u] * s[u]);
+            }
+        }
+    }
+    if (t0 < t1) load_tile(t0, true, !early);
     asm volatile("cp.async.commit_group;" ::: "memory");
 
     float o[TT][NW][4];
@@ -524,7 +554,7 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
             }
         }
         __syncthreads();      // the buffer, P and the maxima are free for the next tile
-        if (t + 1 < t1) load_tile(t + 1);
+        if (t + 1 < t1) load_tile(t + 1, true, true);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");

@@ -607,9 +607,14 @@ template <int R, bool GATED, int TOK, bool DEEP = false> struct Shape {
     static constexpr int STAGES = FIT > (DEEP ? 10 : 8) ? (DEEP ? 10 : 8) : FIT;   // per warp
     static constexpr int TILES = (R + 15) / 16;   // of 16 rows, of each matrix
     static constexpr int SUMS = WARPS * TOK * R * (GATED ? 2 : 1) * 4;    // the warps' sums, over the rings
-    static constexpr size_t smem = (size_t)WARPS * STAGES * STAGE + WARPS * STAGES * 8 + TOK * 4;
-    static_assert(STAGES >= 2 && SUMS + TOK * R * 4 <= WARPS * STAGES * STAGE && smem <= SMEM_MOST, "");
+    static constexpr size_t smem(int stages) { return (size_t)WARPS * stages * STAGE + WARPS * stages * 8 + TOK * 4; }
+    static_assert(STAGES >= 2 && SUMS + TOK * R * 4 <= WARPS * STAGE && smem(STAGES) <= SMEM_MOST, "");
 };
+
+// A short K leaves most of a ring unused: what it does not ask for is room for the kernels after it, which then start sooner.
+template <typename S> __host__ __device__ constexpr int stages_for(int num_kb) {
+    return (num_kb + WARPS - 1) / WARPS < S::STAGES ? (num_kb + WARPS - 1) / WARPS : S::STAGES;
+}
 
 __device__ __forceinline__ void mma16816(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0,
                                          unsigned b1) {
@@ -627,10 +632,11 @@ __global__ void __launch_bounds__(THREADS, DEEP ? 1 : 2) rows_kernel(const __gri
     extern __shared__ __align__(1024) unsigned char rows_smem[];             // (the swizzle counts from multiples of 1 KB)
     unsigned char* smem = rows_smem;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned char* ring = smem + warp * S::STAGES * S::STAGE;
-    unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + WARPS * S::STAGES * S::STAGE);
-    const unsigned full0 = smem_u32(bars + warp * S::STAGES);
-    float* inv_s = reinterpret_cast<float*>(bars + WARPS * S::STAGES);       // [TOK] row scales
+    const int stages = stages_for<S>(p.num_kb);
+    unsigned char* ring = smem + warp * stages * S::STAGE;
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + WARPS * stages * S::STAGE);
+    const unsigned full0 = smem_u32(bars + warp * stages);
+    float* inv_s = reinterpret_cast<float*>(bars + WARPS * stages);          // [TOK] row scales
     const int f0 = blockIdx.x * R;
     const int n_mine = (p.num_kb - warp + WARPS - 1) / WARPS;                // stages warp, warp + 8, ... of K
 
@@ -647,9 +653,9 @@ __global__ void __launch_bounds__(THREADS, DEEP ? 1 : 2) rows_kernel(const __gri
         if (BATCH) tma_load_3d(dst, &map_x, (warp + i * WARPS) * BK, 0, blockIdx.y, full0 + 8 * s);
         else tma_load_2d(dst, &map_x, (warp + i * WARPS) * BK, 0, full0 + 8 * s);
     };
-    const int head = n_mine < S::STAGES ? n_mine : S::STAGES;
+    const int head = n_mine < stages ? n_mine : stages;
     if (lane == 0) {
-        for (int s = 0; s < S::STAGES; ++s) mbar_init(full0 + 8 * s, 1);
+        for (int s = 0; s < stages; ++s) mbar_init(full0 + 8 * s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         for (int i = 0; i < head; ++i) load_w(i, i);                         // weights: no kernel writes them
@@ -726,8 +732,8 @@ __global__ void __launch_bounds__(THREADS, DEEP ? 1 : 2) rows_kernel(const __gri
                 }
         }
         __syncwarp();                                                        // the warp has read the stage
-        if (lane == 0 && i + S::STAGES < n_mine) { load_w(i + S::STAGES, s); load_x(i + S::STAGES, s); }
-        if (++s == S::STAGES) { s = 0; phase ^= 1; }
+        if (lane == 0 && i + stages < n_mine) { load_w(i + stages, s); load_x(i + stages, s); }
+        if (++s == stages) { s = 0; phase ^= 1; }
     }
     ok = __syncthreads_and(ok);                                              // every ring is idle
     if (!ok) {   // a wait of this CTA ran out: copies still in flight get time to land before it leaves
@@ -789,11 +795,11 @@ template <int R, bool GATED, int TOK, bool BATCH, bool DEEP>
 static int launch_maps(const CUtensorMap& mw, const CUtensorMap& mx, const tc::Params& p, int batch, cudaStream_t stream) {
     using S = Shape<R, GATED, TOK, DEEP>;
     static IbDeviceSet allowed;
-    if (const int e = ib_allow_dynamic_smem(allowed, rows_kernel<R, GATED, TOK, BATCH, DEEP>, S::smem)) return e;
+    if (const int e = ib_allow_dynamic_smem(allowed, rows_kernel<R, GATED, TOK, BATCH, DEEP>, S::smem(S::STAGES))) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((p.n_out + R - 1) / R, batch);
     cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = S::smem;
+    cfg.dynamicSmemBytes = S::smem(stages_for<S>(p.num_kb));
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -832,6 +838,8 @@ static int launch_batch(const void* w, const void* x, long ldx, long bx, int k, 
     return launch_maps<R, false, TOK, true, false>(mw, mx, p, batch, stream);
 }
 
+constexpr int DEEP = 1024;    // R + DEEP names the form with the deep ring
+
 // R rows of W per CTA (gated: of each of the two matrices)
 template <bool GATED>
 static int launch_any(int r, const void* w, long n_w, long ldw, const void* x, long ldx, int k, const tc::Params& p,
@@ -841,9 +849,8 @@ static int launch_any(int r, const void* w, long n_w, long ldw, const void* x, l
         case 16: return few ? launch<16, GATED, 8>(w, n_w, ldw, x, ldx, k, p, stream) : launch<16, GATED, 16>(w, n_w, ldw, x, ldx, k, p, stream);
         case 24: return few ? launch<24, GATED, 8>(w, n_w, ldw, x, ldx, k, p, stream) : IB_ERR_UNSUPPORTED;
         case 32: if constexpr (!GATED) return few ? launch<32, GATED, 8>(w, n_w, ldw, x, ldx, k, p, stream) : launch<32, GATED, 16>(w, n_w, ldw, x, ldx, k, p, stream);
-        case 1016: if constexpr (!GATED) return few ? launch<16, GATED, 8, true>(w, n_w, ldw, x, ldx, k, p, stream) : launch<16, GATED, 16, true>(w, n_w, ldw, x, ldx, k, p, stream);
-        case 1024: if constexpr (!GATED) return few ? launch<24, GATED, 8, true>(w, n_w, ldw, x, ldx, k, p, stream) : launch<24, GATED, 16, true>(w, n_w, ldw, x, ldx, k, p, stream);
-        case 1032: if constexpr (!GATED) return few ? launch<32, GATED, 8, true>(w, n_w, ldw, x, ldx, k, p, stream) : launch<32, GATED, 16, true>(w, n_w, ldw, x, ldx, k, p, stream);
+        case DEEP + 16: if constexpr (!GATED) return few ? launch<16, GATED, 8, true>(w, n_w, ldw, x, ldx, k, p, stream) : launch<16, GATED, 16, true>(w, n_w, ldw, x, ldx, k, p, stream);
+        case DEEP + 32: if constexpr (!GATED) return few ? launch<32, GATED, 8, true>(w, n_w, ldw, x, ldx, k, p, stream) : launch<32, GATED, 16, true>(w, n_w, ldw, x, ldx, k, p, stream);
         case 48: if constexpr (!GATED) return few ? launch<48, GATED, 8>(w, n_w, ldw, x, ldx, k, p, stream) : IB_ERR_UNSUPPORTED;
     }
     return IB_ERR_UNSUPPORTED;
@@ -861,18 +868,20 @@ static int launch_any(int r, const void* w, long n_w, long ldw, const void* x, l
 //              4,096 over 4,096 12.2 / 12.1 / -  / 9.8            gated 12,288 over 4,096  36.4 / 39.8
 //              2,048 over 8,192 12.5 / 18.5 / -  / 12.8           10,240 over 5,120  21.7 / 35.6 / -  / 25.8
 // Boxes of few rows are what a long K does not want; more CTAs than two an SM are a second wave with fetches of its own.
+//
+// With the deep ring (a CTA per SM), 1 / 8 / 16 tokens, 16 rows and 32 rows a CTA, against the best above: 1,024 over 3,072 3.7
+// / 3.8 / 4.4 and 4.1 / 4.1 / 4.8 (4.3 / 4.3 / 4.7); 2,048 over 2,048 3.5 / 4.1 / 5.2 both (4.0 / 4.6 / 6.4); over 8,192 12.0
+// each and 8.7 / 9.3 / 10.8 (10.8 / 11.5 / 12.3); 4,096 over 4,096 16.1 and 7.7 / 7.9 / 8.4 (8.8 / 9.0 / 9.8); over 12,288
+// 17.8 / 17.8 / 18.2 with 32 (20.1 / 20.2 / 21.9).
 static int rows_form(int n_tok, int n_out, int num_kb, int gated) {
-    constexpr int RESIDENT = 296;
-    if (n_tok <= 8) {
-        if (gated) return 24;
-        if (n_out <= 24 * 148 && num_kb <= 64) return 24;
-        // (151,936 over 1,024 and 4,096, one token: tcgen05 56 and 189, 48 rows 48 and 180; 32,000 over 2,048: 21.7 / 22.9)
-        return n_out <= 32 * RESIDENT ? 32 : n_out <= 48 * RESIDENT || n_out >= 4 * 48 * RESIDENT ? 48 : 0;
-    }
+    constexpr int SMS = 148, RESIDENT = 2 * SMS;
     if (n_tok > 16) return 0;
-    if (gated) return n_out <= 16 * RESIDENT ? 16 : 0;
-    if (n_out <= 2048) return num_kb <= 64 ? 16 : 0;
-    return n_out <= 32 * RESIDENT ? 32 : 0;
+    if (gated) return n_tok <= 8 ? 24 : n_out <= 16 * RESIDENT ? 16 : 0;
+    if (n_out <= 8 * SMS && num_kb <= 64) return rows::DEEP + 16;
+    if (n_out <= 32 * SMS) return rows::DEEP + 32;
+    if (n_out <= 32 * RESIDENT) return 32;
+    // (151,936 over 1,024 and 4,096, one token: tcgen05 56 and 189, 48 rows 48 and 180; 32,000 over 2,048: 21.7 / 22.9)
+    return n_tok <= 8 && (n_out <= 48 * RESIDENT || n_out >= 4 * 48 * RESIDENT) ? 48 : 0;
 }
 
 // How many CTAs share one output tile when the caller does not say.  Each part is a CTA whose ring (80 KB) holds a share of
@@ -1047,7 +1056,7 @@ IB_EXPORT int ib_gemm_tcgen05_ssq_parts(int n_tok, int n_out, int k, int split_k
     const int bn = bn_for(n_tok);
     if (bn > 32) return IB_ERR_UNSUPPORTED;
     if (const int r = split_k < -1 ? -split_k : split_k == -1 ? rows_form(n_tok, n_out, (k + tc::BK - 1) / tc::BK, 0) : 0)
-        return (n_out + r - 1) / r;
+        return (n_out + r % rows::DEEP - 1) / (r % rows::DEEP);
     const int splits = choose_splits(n_tok, n_out, (k + tc::BK - 1) / tc::BK, bn, split_k);
     const int rows = tile_rows_for(n_out, splits, tc::BM, resident_for(bn, splits));
     return ((n_out + rows - 1) / rows) * splits;

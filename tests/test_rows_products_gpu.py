@@ -18,7 +18,7 @@ def close(got, want, terms):
     return bool(((got.double() - want).abs() <= half * want.abs() + terms).all())
 
 
-FORMS = [(16, 1), (16, 3), (16, 16), (24, 1), (24, 8), (32, 8), (32, 13), (48, 5)]
+FORMS = [(16, 1), (16, 3), (16, 16), (24, 1), (24, 8), (32, 8), (32, 13), (48, 5), (1024 + 16, 7), (1024 + 32, 16), (1024 + 32, 2)]
 
 
 @pytest.mark.parametrize("r,n", FORMS)
@@ -44,7 +44,7 @@ def test_product_with_folded_norms_and_gate(r, n, m, k):
     assert bool(((stream.double() - (old.double() + y)).abs() <= 2.0 ** -8 * y.abs() + terms * inv[:, None] + 1e-6).all())
     assert torch.equal(out, (stream * weight).to(torch.bfloat16))
     sums, want = got.ssq[:got.n_parts, :n].double().sum(0), (stream.double() ** 2).sum(1)
-    assert got.n_parts == (m + r - 1) // r and bool(((sums - want).abs() <= m * 2.0 ** -24 * want).all())
+    assert got.n_parts == -(-m // (r % 1024)) and bool(((sums - want).abs() <= m * 2.0 ** -24 * want).all())
     if r <= (24 if n <= 8 else 16):
         inner = m // 2
         out = torch.full((n, inner), float("nan"), dtype=torch.bfloat16, device="cuda")
