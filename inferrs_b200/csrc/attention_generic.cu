@@ -394,13 +394,17 @@ __global__ void __launch_bounds__(32 * T * (G < 4 ? G : 4), 1024 / (32 * T * (G 
     float* ks = smem;                                   // [T * KEYS][d + 4]
     float* vs = ks + T * KEYS * kld;                    // [T * KEYS][dv]
     float* qs = vs + T * KEYS * dv;                     // [G][d]
-    ib_grid_dependency_sync();
+    // a row's place and the keys and values of earlier steps are fetched while the kernel ahead still runs
+    ib_grid_dependency_launch();
     const int req = row_request[row], pos = positions[row];
     if (shared) {
         const int beside = row - SHORT_RUN + lane;
         const bool known = lane <= 2 * SHORT_RUN && beside >= 0 && beside < n_rows;
         const unsigned same = __ballot_sync(0xffffffffu, (known ? row_request[beside] : -1) == req && known);
-        if (__clz(~(same << (32 - SHORT_RUN))) + __ffs(~(same >> SHORT_RUN)) - 1 > SHORT_RUN) return;
+        if (__clz(~(same << (32 - SHORT_RUN))) + __ffs(~(same >> SHORT_RUN)) - 1 > SHORT_RUN) {
+            ib_grid_dependency_wait();
+            return;
+        }
     }
     const int* bt = block_table + (long)req * max_pages;
     const int lo = ib_first_visible(pos, window), t_first = lo / KEYS;
@@ -413,7 +417,8 @@ __global__ void __launch_bounds__(32 * T * (G < 4 ? G : 4), 1024 / (32 * T * (G 
         const int page = bt[j / page_size];
         return page >= 0 && page < n_pages ? ((long)page * n_kv_heads + kvh) * page_size + j % page_size : -1;
     };
-    auto fetch = [&](float* dst, int ld, const float* pages, int n, int i, long at) {
+    // own: the row's own key, the last of the last tile
+    auto fetch = [&](float* dst, int ld, const float* pages, int n, int i, long at, bool own, bool others) {
         const float* mine = at >= 0 ? pages + at * n : nullptr;
         dst += tile * KEYS * ld + lane * 4;
         auto copy = [&](int j) {                        // the warps of a tile share its rows
@@ -421,17 +426,29 @@ __global__ void __launch_bounds__(32 * T * (G < 4 ? G : 4), 1024 / (32 * T * (G 
             if (lane * 4 < n) copy16(dst + j * ld, src ? src + lane * 4 : pages, src != nullptr);
         };
         if (i < n_tiles - 1) {
+            if (others) {
 #pragma unroll 2
-            for (int j = side; j < KEYS; j += SIDE) copy(j);
+                for (int j = side; j < KEYS; j += SIDE) copy(j);
+            }
         } else if (i == n_tiles - 1) {                  // the last tile ends with the row's own key
+            const int last = pos % KEYS;
+            if (others) {
 #pragma unroll 1
-            for (int j = side; j <= pos % KEYS; j += SIDE) copy(j);
+                for (int j = side; j < last; j += SIDE) copy(j);
+            }
+            if (own && last % SIDE == side) copy(last);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     long at = place(tile);
-    fetch(ks, kld, k_pages, d, tile, at);
-    fetch(vs, dv, v_pages, dv, tile, at);
+    const bool early = row == 0 || row_request[row - 1] != req;         // no key but its own is this step's
+    if (early) {
+        fetch(ks, kld, k_pages, d, tile, at, false, true);
+        fetch(vs, dv, v_pages, dv, tile, at, false, true);
+    }
+    ib_grid_dependency_wait();
+    fetch(ks, kld, k_pages, d, tile, at, true, !early);
+    fetch(vs, dv, v_pages, dv, tile, at, true, !early);
     for (int e = tid; e < group * d; e += THREADS) qs[e] = q[((long)row * n_heads + kvh * group) * d + e];
     for (int c = tid; c < G; c += THREADS) {
         s_m[c] = -INFINITY;
@@ -482,7 +499,7 @@ __global__ void __launch_bounds__(32 * T * (G < 4 ? G : 4), 1024 / (32 * T * (G 
         }
         __syncthreads();                                                // everyone has left the keys
         at = place(i0 + T + tile);
-        fetch(ks, kld, k_pages, d, i0 + T + tile, at);
+        fetch(ks, kld, k_pages, d, i0 + T + tile, at, true, true);
         if (live) {
 #pragma unroll
             for (int c_ = 0; c_ < PER; ++c_) {
@@ -558,7 +575,7 @@ __global__ void __launch_bounds__(32 * T * (G < 4 ? G : 4), 1024 / (32 * T * (G 
             }
         }
         __syncthreads();                                                // everyone has left the values
-        fetch(vs, dv, v_pages, dv, i0 + T + tile, at);
+        fetch(vs, dv, v_pages, dv, i0 + T + tile, at, true, true);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();

@@ -58,7 +58,7 @@ __global__ void qk_norm_rope_store_kernel(
     act_t* __restrict__ k_pages, act_t* __restrict__ v_pages, act_t* __restrict__ q_out,
     const float* __restrict__ bias, int value_is_key) {
     extern __shared__ float smem[];
-    ib_grid_dependency_sync();
+    ib_grid_dependency_launch();          // the row's place is looked up while the kernel ahead still runs
     const int row = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int d = head_dim;
@@ -68,7 +68,7 @@ __global__ void qk_norm_rope_store_kernel(
     const int pos = positions[row];
     const int heads_total = n_heads + (store_kv ? 2 * n_kv_heads : 0);
     // a position outside the rotation tables: the row is left out and the fault is recorded
-    if (pos < 0 || (rot_dim > 0 && pos >= table_rows)) { ib_note_row_fault(row); return; }
+    if (pos < 0 || (rot_dim > 0 && pos >= table_rows)) { ib_note_row_fault(row); ib_grid_dependency_wait(); return; }
 
     // Where this row's key and value go: page and place within the page.
     long kv_place = -1;  // (page, kv head 0, slot) counted in heads' rows
@@ -80,6 +80,7 @@ __global__ void qk_norm_rope_store_kernel(
     }
     const bool clear_tail = kv_place >= 0 && ib_last_row_of_request(row_request, row, gridDim.x);
     const bool norm_after = (norm_flags & 4) != 0;
+    ib_grid_dependency_wait();
 
     // one warp per head: blockIdx.y picks the group of QRS_WARPS heads
     for (int head = blockIdx.y * QRS_WARPS + warp; head < heads_total; head += heads_total) {

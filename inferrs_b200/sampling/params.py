@@ -91,9 +91,10 @@ def uniforms_for(seeds, steps):
         if len(a) != 1 and len(b) != 1:
             raise ValueError(f"{len(a)} seeds for {len(b)} steps")
         a, b = (list(a) * len(b), b) if len(a) == 1 else (a, list(b) * len(a))
-    n, native = len(a), host_python()
-    words = np.empty((2 * n,), dtype=np.uint64)
-    at = words.__array_interface__["data"][0]
+    n = len(a)
+    native = host_python() if n >= NATIVE_ROWS else None
+    words = None if native is None else np.empty((2 * n,), dtype=np.uint64)
+    at = 0 if native is None else words.__array_interface__["data"][0]
     if native is None or native.ibh_low_words(a, n, at) or native.ibh_low_words(b, n, at + 8 * n):
         words = array("Q", [int(x) & _M64 for x in a] + [int(x) & _M64 for x in b])
         at = words.buffer_info()[0]
@@ -103,6 +104,7 @@ def uniforms_for(seeds, steps):
 
 
 _NATIVE = []
+NATIVE_ROWS = 12     # rows from which the calls into native code cost less than they save (a call and its arrays: about 5 us)
 
 
 def host_python():

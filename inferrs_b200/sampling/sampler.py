@@ -13,7 +13,7 @@ import numpy as np
 import torch
 
 from .. import kernels
-from .params import SamplingParams, host_python, uniforms_for
+from .params import NATIVE_ROWS, SamplingParams, host_python, uniforms_for
 
 
 class Sampler:
@@ -134,7 +134,7 @@ class Sampler:
         words[7 * r:8 * r] = top_k
         n_prev = words[8 * r:9 * r]
         n_prev[:] = 0
-        if width and not self._windows_natively(last, histories, pend, width, words[9 * r:9 * r + r * width], n_prev):
+        if width and not (r >= NATIVE_ROWS and self._windows_natively(last, histories, pend, width, words[9 * r:9 * r + r * width], n_prev)):
             # the windows, row by row: -1 in the place of the pending token, the history's tail, -1 up to the width.  The
             # window's order does not matter: the pending token, if any, takes the first place.
             windows, counts, blank = array("i"), [], array("i", [-1]) * width

@@ -51,10 +51,11 @@ def test_product_with_folded_norms_and_gate(r, n, m, k):
         K.gemm_swiglu_tcgen05(scaled, w[:2 * inner], out, rows_per_cta=r)
         g, u = y[:, :inner], y[:, inner:2 * inner]
         want = g / (1 + torch.exp(-g)) * u
-        # both factors are rounded to bfloat16 first (2^-9 each; silu changes at most 1.1 times as much as its argument)
+        # both factors are rounded to bfloat16 first (2^-8 each; silu changes at most 1.1 times as much as its argument), the
+        # result again
         off = terms * inv[:, None]                           # of the float32 sums
         off_g, off_u = off[:, :inner], off[:, inner:2 * inner]
-        slack = 2.0 ** -8 * (1.1 * g.abs() * u.abs() + want.abs()) + 1.2 * (off_g * u.abs() + off_u * g.abs() + off_g * off_u)
+        slack = 2.0 ** -8 * (1.11 * g.abs() * u.abs() + 2.1 * want.abs()) + 1.2 * (off_g * u.abs() + off_u * g.abs() + off_g * off_u)
         assert bool(((out.double() - want).abs() <= slack).all())
     assert K.gemm_tcgen05_error() == 0
 

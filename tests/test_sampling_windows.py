@@ -54,11 +54,12 @@ def test_what_is_no_list_of_integers_is_left_to_the_general_way(history):
     assert not Sampler._windows_natively([4, 4], [[1, 2]] * 2, [0, 0], 4, words, counts)
 
 
-def test_seeds_of_every_kind_give_the_bits_of_the_plain_generator():
-    seeds, steps = [0, 1, -5, 2 ** 63 + 7, 2 ** 70 + 1], [3, 0, 2 ** 40, 7, 1]
+@pytest.mark.parametrize("copies", [1, 3])
+def test_seeds_of_every_kind_give_the_bits_of_the_plain_generator(copies):
+    seeds, steps = [0, 1, -5, 2 ** 63 + 7, 2 ** 70 + 1] * copies, [3, 0, 2 ** 40, 7, 1] * copies
     want = [float(np.float32(uniform_for(a, b))) for a, b in zip(seeds, steps)]
     assert uniforms_for(seeds, steps).tolist() == want
     assert uniforms_for(tuple(seeds), np.array(steps)).tolist() == want
-    assert uniforms_for([9], steps).tolist() == uniforms_for([9] * 5, steps).tolist()
+    assert uniforms_for([9], steps).tolist() == uniforms_for([9] * 5 * copies, steps).tolist()
     with pytest.raises(ValueError):
         uniforms_for([1, 2], steps)
