@@ -8,6 +8,11 @@
 // a counter of its (request, head group), and the CTA that finds it was the last one merges all slices and
 // writes the output, so no second kernel is needed.  How many slices are used is decided from the request's real length (at least `min_tiles`
 // tiles per slice); CTAs of unused slices leave at once.
+//
+// More (request, head) pairs than run at a time, in lists of up to 256 requests: CTAs are handed out longest request first (every
+// CTA ranks the requests by their tiles, before it waits for the kernel ahead), and a request of more than five quarters
+// of a resident CTA's even share is cut in two.  In the order of the list, the last head's longest request starts when most CTAs have
+// ended, and runs on alone.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -68,11 +73,15 @@ struct Params {
     const int* rows;           // [R] or null: the row of q, positions and out that place i of the grid works on
     const int* reqs;           // [R] or null: its request (row of the block table); a negative row is no work
     int max_pages, page_size, n_pages, n_heads, n_kv_heads, window, max_splits, min_tiles;
+    int ranked;                // requests to rank (0: CTAs come in the order of the list)
     float scale_log2;
     float slope_factor;        // log2(e); with a cap it and scale_log2 carry ib_cap_factor too (see ib_capped_log2)
     float cap_c;
     IbScoreOptions opt;
 };
+
+constexpr int RANKED_MOST = 256;            // requests that are ranked
+constexpr int RESIDENT = 296;               // CTAs that run at a time
 
 // One warp's share of a row: 16 keys of every tile against the group's query heads; scores, softmax in float32, values.
 //
@@ -361,7 +370,38 @@ __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constan
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // place i of the grid is row i of request i in a step of single tokens; in a step that also holds prompt
     // portions a list says which rows are single tokens and whose they are
-    const int place = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
+    const int keep = OPTIONS ? P.opt.keep_first : 0;
+    auto tiles_of = [&](int pos) {          // the request's tiles: those that hold kept keys, then the window's from t_first on
+        const int t = ib_first_visible(pos, P.window) / KEYS;
+        return ib_kept_tiles(keep, t, KEYS) + pos / KEYS + 1 - t;
+    };
+    int place = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z, share = 0;
+    if (P.ranked > 0) {
+        __shared__ __align__(16) int tiles[RANKED_MOST + 4];
+        __shared__ int ranked_place, ranked_total;
+        split = blockIdx.x % P.max_splits;
+        kvh = blockIdx.x / P.max_splits;
+        if (threadIdx.x == 0) ranked_total = 0;
+        for (int i = threadIdx.x; i < P.ranked + 4; i += THREADS) {
+            const int r = i >= P.ranked ? -1 : P.rows != nullptr ? P.rows[i] : i;
+            tiles[i] = r < 0 ? -1 : tiles_of(P.positions[r]);
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < P.ranked; i += THREADS) {
+            const int mine = tiles[i];
+            int rank = 0;
+            for (int j = 0; j < P.ranked; j += 4) {
+                const int4 t = *reinterpret_cast<const int4*>(tiles + j);
+                rank += (t.x > mine || (t.x == mine && j < i)) + (t.y > mine || (t.y == mine && j + 1 < i)) +
+                        (t.z > mine || (t.z == mine && j + 2 < i)) + (t.w > mine || (t.w == mine && j + 3 < i));
+            }
+            if (rank == (int)blockIdx.y) ranked_place = i;
+            if (mine > 0) atomicAdd(&ranked_total, mine);
+        }
+        __syncthreads();
+        place = ranked_place;
+        share = (int)(((long)ranked_total * P.n_kv_heads + RESIDENT - 1) / RESIDENT);
+    }
     const int row = P.rows != nullptr ? P.rows[place] : place;
     // A CTA that has nothing to do still waits for the kernels before this one: a grid that has let its
     // dependents start must not complete before its own predecessors have, or the kernel after it could read
@@ -371,12 +411,11 @@ __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constan
     const int G = P.n_heads / P.n_kv_heads;
     const int pos = P.positions[row];
     const int lo = ib_first_visible(pos, P.window);
-    // the request's tiles: those that hold kept keys, then the window's from t_first on
-    const int keep = OPTIONS ? P.opt.keep_first : 0;
     const int t_first = lo / KEYS, n_kept = ib_kept_tiles(keep, t_first, KEYS);
     const int n_all = n_kept + pos / KEYS + 1 - t_first;
     int n_splits = (n_all + P.min_tiles - 1) / P.min_tiles;
     if (n_splits > P.max_splits) n_splits = P.max_splits;
+    if (P.ranked > 0 && 4 * n_all <= 5 * share) n_splits = 1;
     if (split >= n_splits) { asm volatile("griddepcontrol.wait;" ::: "memory"); return; }   // an unused slice
     const int per = (n_all + n_splits - 1) / n_splits;
     const int i_begin = split * per;                          // this slice's tiles: places i_begin .. of that list
@@ -555,16 +594,18 @@ __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constan
 // One new token per request: row r = request r, or, with `rows` and `reqs` (n_rows entries each), row rows[i] of
 // request reqs[i] (a negative row is skipped).  part_o [rows, n_heads, max_splits, 128] and part_ml
 // [rows, n_heads, max_splits, 2] are float32 scratch; counters [rows * n_kv_heads] are ints that are zero
-// (the kernel leaves them zero).  Launches that share scratch and counters must not overlap.
+// (the kernel leaves them zero).  Launches that share scratch and counters must not overlap.  ranked: CTAs come longest request first
+// (up to 256 rows), and slices of min_tiles tiles or more are for requests beyond the even share alone.
 IB_EXPORT int ib_paged_attention_decode(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                                         int max_pages, int page_size, int n_pages, const int* positions, int n_rows,
                                         int n_heads, int n_kv_heads, int head_dim, float scale, int window, void* out,
                                         int max_splits, int min_tiles, float* part_o, float* part_ml, int* counters,
                                         const int* rows, const int* reqs, const float* head_scale, const float* slopes,
                                         const float* sinks, float cap, int keep_first, const void* gate, long gate_ld,
-                                        long out_ld, cudaStream_t stream) {
+                                        long out_ld, int ranked, cudaStream_t stream) {
     if (n_rows <= 0) return IB_OK;
     if (min_tiles <= 0) return IB_ERR_ARGUMENT;
+    if (ranked && (n_rows > dec::RANKED_MOST || (long)n_kv_heads * max_splits > 65535)) return IB_ERR_UNSUPPORTED;
     if ((rows == nullptr) != (reqs == nullptr)) return IB_ERR_ARGUMENT;
     if (n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads || page_size <= 0 || max_pages <= 0 || max_splits <= 0)
         return IB_ERR_ARGUMENT;
@@ -593,13 +634,14 @@ IB_EXPORT int ib_paged_attention_decode(const void* q, const void* k_pages, cons
     P.max_pages = max_pages; P.page_size = page_size;
     P.n_pages = n_pages; P.n_heads = n_heads; P.n_kv_heads = n_kv_heads; P.window = window; P.max_splits = max_splits;
     P.min_tiles = min_tiles;
+    P.ranked = ranked ? n_rows : 0;
     P.scale_log2 = scale * 1.4426950408889634f;
     if (cap > 0.0f) P.scale_log2 *= ib_cap_factor(cap);
     P.slope_factor = 1.4426950408889634f * (cap > 0.0f ? ib_cap_factor(cap) : 1.0f);
     P.cap_c = cap * 1.4426950408889634f;
     P.opt = {head_scale, slopes, sinks, cap, keep_first, (const act_t*)gate, gate_ld, out_ld};
     const size_t smem = 2 * dec::STAGES * dec::TILE_BYTES + 16 * dec::D * 2 + (2 * dec::STAGES + 1) * 8 + 1024;
-    const dim3 grid(n_rows, n_kv_heads, max_splits);
+    const dim3 grid = ranked ? dim3(n_kv_heads * max_splits, n_rows) : dim3(n_rows, n_kv_heads, max_splits);
     const bool options = head_scale != nullptr || slopes != nullptr || sinks != nullptr || cap > 0.0f || gate != nullptr || keep_first > 0;
 #define IB_DECODE(OPTIONS, FEW)                                                                                \
     do {                                                                                                       \
@@ -636,7 +678,7 @@ IB_EXPORT int ib_attention_decode_error_async(int* out, cudaStream_t stream) {
 IB_EXPORT int ib_paged_attention_decode(const void*, const void*, const void*, const int*, int, int, int, const int*, int,
                                         int, int, int, float, int, void*, int, int, float*, float*, int*, const int*,
                                         const int*, const float*, const float*, const float*, float, int, const void*, long,
-                                        long, cudaStream_t) {
+                                        long, int, cudaStream_t) {
     return IB_ERR_UNSUPPORTED;
 }
 

@@ -1,0 +1,55 @@
+"""Decode attention that hands its CTAs out longest request first (csrc/attention_decode.cu)."""
+from __future__ import annotations
+
+import random
+
+import pytest
+import torch
+
+import kernel_refs as R
+from helpers import rel_err
+from test_kernels_gpu import _paged_setup, rand
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,nkv,window", [(2, 2, None), (37, 8, None), (64, 8, 300), (255, 1, None), (256, 2, None)])
+def test_ranked_requests_give_what_the_list_gives(n, nkv, window):
+    """Lengths around the tiles' edges, equal ones and one far beyond the others (which is cut in two where that pays), alone
+    and as a list of rows with gaps: the reference's values, and the unranked kernel's bits for every request that stays in one
+    slice."""
+    from inferrs_b200 import kernels as K
+    rng = random.Random(n)
+    lens = [rng.choice([1, 63, 64, 65, 128, rng.randint(1, 200)]) for _ in range(n)]
+    lens[n // 2] = 1500
+    table, positions, row_request, k_pages, v_pages = _paged_setup(torch.bfloat16, nkv, 128, 16, lens, [1] * n, 7)
+    q = rand((n, 2 * nkv, 128), torch.bfloat16, 8)
+    ref = torch.empty((n, 2 * nkv * 128), dtype=torch.bfloat16, device="cuda")
+    R.paged_attention_generic(q, k_pages, v_pages, table, row_request, positions, 128 ** -0.5, window, ref)
+    plain, out = torch.empty_like(ref), torch.full_like(ref, float("nan"))
+    K.paged_attention_decode(q, k_pages, v_pages, table, positions, 128 ** -0.5, window, plain, 1)
+    for _ in range(2):                                   # twice: the counters are back at zero
+        K.paged_attention_decode(q, k_pages, v_pages, table, positions, 128 ** -0.5, window, out, 2, min_tiles=8, ranked=True)
+        assert K.attention_decode_error() == 0
+        assert rel_err(out, ref) < 2e-2
+        others = torch.tensor([i for i in range(n) if i != n // 2], device="cuda")
+        assert torch.equal(out[others], plain[others])
+    rows = torch.tensor([i if i % 3 else -1 for i in range(n)], dtype=torch.int32, device="cuda")
+    some = torch.full_like(ref, 7.0)
+    K.paged_attention_decode(q, k_pages, v_pages, table, positions, 128 ** -0.5, window, some, 2, rows, rows, min_tiles=8,
+                             ranked=True)
+    kept = torch.tensor([i for i in range(n) if i % 3], dtype=torch.long, device="cuda")
+    left = torch.tensor([i for i in range(n) if i % 3 == 0], dtype=torch.long, device="cuda")
+    assert bool((some[left] == 7.0).all()) and rel_err(some[kept], ref[kept]) < 2e-2
+
+
+def test_more_requests_than_are_ranked_are_refused_and_the_plan_keeps_to_the_list():
+    from inferrs_b200 import kernels as K
+    assert K.decode_plan(64, 8, 4096) == {"max_splits": 2, "min_tiles": 8, "ranked": True}
+    assert K.decode_plan(8, 8, 4096) == {"max_splits": 4, "min_tiles": 4}
+    assert K.decode_plan(75, 8, 4096) == K.decode_plan(257, 8, 4096) == {"max_splits": 1, "min_tiles": 4}
+    table, positions, _, k_pages, v_pages = _paged_setup(torch.bfloat16, 1, 128, 16, [3] * 257, [1] * 257, 9)
+    q = rand((257, 1, 128), torch.bfloat16, 10)
+    with pytest.raises(K.KernelError):
+        K.paged_attention_decode(q, k_pages, v_pages, table, positions, 0.1, None, torch.empty((257, 128), dtype=torch.bfloat16,
+                                                                                              device="cuda"), 2, ranked=True)
