@@ -17,10 +17,17 @@
 // Roles in a CTA (tile_rows <= 128 rows of W as the M of the products, BN tokens as their N):
 //   warp 0      TMA producer: 32 of k of W and x, as float32, per stage of the ring
 //   warp 1      issuer of the products, owner of the tensor-memory allocation
-//   warps 2-3   x's pieces, to three swizzled tiles in shared memory (the products' B operand)
+//   warps 2-3   x's pieces, to three swizzled tiles in shared memory (the products' B operand); beyond 16 tokens two more
+//               warps at the end, on the SM's other schedulers
 //   warps 4-7   W's pieces: a thread reads its row from the stage and writes the three pieces to tensor memory (the
 //               products' A operand, so that W's pieces never pass through shared memory again)
 //   warps 8-    the sums: four warps, or beyond 16 tokens eight with half of the tokens each
+//
+// What bounds it (512 rows, 4,096 features over 1,024): 44 us = 98 TFLOP/s, where a chain of multiply-adds took 110 to 160 us
+// (36 TFLOP/s); 2,048 rows 111.  The tensor pipe is busy 30 % of the time, the issue slots 52, memory hands over 0.4 TB/s: the
+// warps that make the pieces and add up are what a block of 64 of k waits for.  With two warps for x's pieces instead of
+// four 45.8 us, with four summing warps instead of eight 63.5.  Up to 16 rows: a row 7 to 10 us, the way of x
+// and the cluster's exchange; memory takes 1.3 to 4 of them.
 //
 // Infinities and NaN: the pieces of an infinity are no numbers, so a result that is not finite is computed again as
 // one chain of fused multiply-adds, by the thread that would store it.  Numbers below 2^-102 have pieces that bfloat16 holds only
@@ -161,7 +168,8 @@ constexpr size_t smem_bytes() {
 }
 
 constexpr int sum_warps(int bn) { return bn <= 16 ? 4 : 8; }
-constexpr int threads_of(int bn) { return 32 * (SUM_WARP0 + sum_warps(bn)); }
+constexpr int x_warps(int bn) { return bn <= 16 ? 2 : 4; }
+constexpr int threads_of(int bn) { return 32 * (SUM_WARP0 + sum_warps(bn) + x_warps(bn) - 2); }
 
 template <int BN, int STAGES>
 __global__ void __launch_bounds__(threads_of(BN), (BN <= 16 ? 2 : 1)) split_kernel(const __grid_constant__ CUtensorMap map_w,
@@ -172,7 +180,7 @@ __global__ void __launch_bounds__(threads_of(BN), (BN <= 16 ? 2 : 1)) split_kern
     // accumulators: of the largest product per block parity, and of the others (two sizes side by side)
     constexpr int TMEM_ACC = 2 * A_COLS, TMEM_SMALL = TMEM_ACC + 2 * BN, TMEM_WAITING = TMEM_SMALL + 2 * BN;
     constexpr int TMEM_COLS = BN <= 16 ? 256 : 512;
-    constexpr int SUM_WARPS = sum_warps(BN), C = BN * 4 / SUM_WARPS;         // C: tokens of a thread that adds up
+    constexpr int X_WARPS = x_warps(BN), SUM_WARPS = sum_warps(BN), C = BN * 4 / SUM_WARPS;         // C: tokens of a thread that adds up
     static_assert(TMEM_WAITING + (C > 16 ? BN : 0) <= TMEM_COLS && (C == 16 || C == 32), "");
     static_assert((2 * STAGES + 7) * 8 + 8 <= 256, "");
     extern __shared__ unsigned char raw_smem[];
@@ -200,8 +208,8 @@ __global__ void __launch_bounds__(threads_of(BN), (BN <= 16 ? 2 : 1)) split_kern
 
     ib_grid_dependency_launch();
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 6); }
-        for (int s = 0; s < 2; ++s) { mbar_init(ready0 + 8 * s, 6); mbar_init(done0 + 8 * s, 1); mbar_init(taken0 + 8 * s, SUM_WARPS); }
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 4 + X_WARPS); }
+        for (int s = 0; s < 2; ++s) { mbar_init(ready0 + 8 * s, 4 + X_WARPS); mbar_init(done0 + 8 * s, 1); mbar_init(taken0 + 8 * s, SUM_WARPS); }
         mbar_init(small0, SUM_WARPS);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -278,8 +286,9 @@ __global__ void __launch_bounds__(threads_of(BN), (BN <= 16 ? 2 : 1)) split_kern
                 if (++m == p.blocks_per_segment) { m = 0; ++segment; }
             }
         }
-    } else if (warp < 4) {
-        const int e = (int)threadIdx.x - 64, r0 = ((e >> 3) & 1) + ((e >> 4) & 1) * 4 + (e >> 5) * 2;
+    } else if (warp < 4 || warp >= SUM_WARP0 + SUM_WARPS) {
+        const int part = warp < 4 ? warp - 2 : warp - (SUM_WARP0 + SUM_WARPS) + 2;
+        const int r0 = ((lane >> 3) & 1) + ((lane >> 4) & 1) * 4 + (part & 1) * 2 + (part >> 1) * 8;
         for (int i = 0; i < n_blocks && ok; ++i) {
             const int b = i & 1;
             if (i >= 2 && !mbar_wait(done0 + 8 * b, ((i >> 1) - 1) & 1, 6)) ok = false;
@@ -289,16 +298,16 @@ __global__ void __launch_bounds__(threads_of(BN), (BN <= 16 ? 2 : 1)) split_kern
                 if (ok && !mbar_wait(full0 + 8 * s, (t / STAGES) & 1, 7)) ok = false;
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                float4 v[BN / 8];                            // four numbers of a row at a time, all asked for together
-                const int c = e & 7;                         // (a warp's rows differ in bit 2: its stores meet all banks)
+                float4 v[BN / (4 * X_WARPS)];                // four numbers of a row at a time, all asked for together
+                const int c = lane & 7;                      // (a warp's rows differ in bit 2: its stores meet all banks)
 #pragma unroll
-                for (int j = 0; j < BN / 8; ++j) {
-                    const int r = r0 + j * 8;
+                for (int j = 0; j < BN / (4 * X_WARPS); ++j) {
+                    const int r = r0 + j * 4 * X_WARPS;
                     v[j] = *reinterpret_cast<const float4*>(x_ring + s * X_STAGE + r * 128 + ((c ^ (r & 7)) << 4));
                 }
 #pragma unroll
-                for (int j = 0; j < BN / 8; ++j) {
-                    const int r = r0 + j * 8;
+                for (int j = 0; j < BN / (4 * X_WARPS); ++j) {
+                    const int r = r0 + j * 4 * X_WARPS;
                     uint2 w0, w1, w2;
                     split_pair(v[j].x, v[j].y, w0.x, w1.x, w2.x);
                     split_pair(v[j].z, v[j].w, w0.y, w1.y, w2.y);
@@ -436,7 +445,7 @@ __global__ void __launch_bounds__(threads_of(BN), (BN <= 16 ? 2 : 1)) split_kern
             }
         }
     }
-    if (splits > 1 && warp < SUM_WARP0) {      // the other warps' part in the cluster's two barriers
+    if (splits > 1 && (warp < SUM_WARP0 || warp >= SUM_WARP0 + SUM_WARPS)) {      // the other warps' part in the cluster's two barriers
         if (BN > 32) cluster_arrive();
         cluster_wait();
         cluster_arrive();
