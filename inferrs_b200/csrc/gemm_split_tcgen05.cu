@@ -516,12 +516,17 @@ static Cut choose_cut(int n_tok, int n_out, int blocks, int bn) {
             if (tiles << l <= 2 * (resident[l] + 12)) return {1 << l, BM};
         return {1, BM};
     }
-    // else the time of the fullest SM: its blocks, and what every CTA pays at its ends
+    // else the time of the fullest SM, us: its blocks, and what a wave of CTAs pays at its ends (least where the segments are
+    // shared by eight: none is added to another by the CTA itself).  Fitted to 32 to 2,048 rows of 4,096 and 6,144
+    // features over 1,024, of 1,024 over 2,048 and 3,072 in 1 / 2 / 4 / 8 parts: 64 tiles over 1,024 21.7 / 18.2 / 23.0 /
+    // 40.4, over 3,072 52.7 / 33.1 / 38.1 / 59.9; 192 tiles over 1,024 44.6 / 53.6 / 68.0 / 106.8; 8 tiles over 2,048 36.4 / 24.3 /
+    // 14.2 / 10.0
+    const float ends[4] = {6.5f, 9.8f, 7.5f, 5.0f};
     Cut best = {1, BM};
     float least = 0.0f;
     for (int l = 0; l < 4; ++l) {
         const long waves = ((tiles << l) + resident[l] - 1) / resident[l];
-        const float t = waves * ((float)((blocks + (1 << l) - 1) >> l) * 1.2f + 5.0f + l);
+        const float t = waves * ((float)((blocks + (1 << l) - 1) >> l) * 0.93f + ends[l]);
         if (l == 0 || t < least) { least = t; best.splits = 1 << l; }
     }
     return best;
