@@ -52,16 +52,34 @@ __device__ __forceinline__ void sw_store4(float* p, const float (&d)[4]) {
     *reinterpret_cast<float4*>(p) = make_float4(d[0], d[1], d[2], d[3]);
 }
 
+// The sum over the block as ib_block_sum makes it, with one meeting: `red` holds 32 numbers that nothing has used before.
+__device__ __forceinline__ float sw_block_sum(float v, float* red) {
+    const int lane = threadIdx.x & 31;
+    v = ib_warp_sum(v);
+    if (lane == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    return ib_warp_sum(lane < (int)((blockDim.x + 31) >> 5) ? red[lane] : 0.0f);
+}
+
+#define SW_EARLY_TAPS 4                  // taps of a convolution whose kept rows are fetched before the wait
+
+// A decode step has few rows, and a launch is a chain: the wait, the row, two meetings of the block.  So what no kernel of the
+// step writes before this one is fetched while the kernel ahead still runs (the norms' and the convolution's weights, and
+// the convolution's kept rows, which this kernel alone moves, once a step), and a meeting is one barrier.  Replay of a design
+// with 162 launches of 4 to 5 us: 7.32 -> 7.24 ms.  Rows of more than 4,096 numbers fill the registers: there the weights
+// are read last, as they are needed.
 // The row in registers: NV groups of four columns per thread (thread t has groups t, t + blockDim, ...).  A group
 // beyond the row is read as the last one and not written, so that loads carry no condition.
 template <typename WT, int NV, int THREADS, bool CONV>
 __global__ void __launch_bounds__(THREADS) sandwich_norm_vec_kernel(const SandwichArgs a) {
-    __shared__ float red[32];
+    __shared__ float red[2][32];
     ib_grid_dependency_launch();
-    const int W = a.width, nv = W >> 2;
+    const int W = a.width, nv = W >> 2, r = blockIdx.x;
     int col[NV];
     bool in[NV];
-    float post[NV][4];
+    constexpr bool EARLY = NV <= 2;      // (the registers of four groups are full)
+    float post[NV][4], weight[NV][4], cv[CONV ? NV : 1][4], cw[CONV ? NV : 1][4];
+    float kept_rows[CONV ? SW_EARLY_TAPS - 1 : 1][CONV ? NV : 1][4];
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         const int g = threadIdx.x + k * blockDim.x;
@@ -69,20 +87,42 @@ __global__ void __launch_bounds__(THREADS) sandwich_norm_vec_kernel(const Sandwi
         col[k] = min(g, nv - 1) * 4;
         if (a.post) sw_load4(post[k], a.post + col[k]);
         else post[k][0] = post[k][1] = post[k][2] = post[k][3] = 1.0f;
+        if (EARLY) sw_load4(weight[k], reinterpret_cast<const WT*>(a.weight) + col[k]);
+    }
+    float* kept = nullptr;
+    const bool early = CONV && EARLY && a.taps <= SW_EARLY_TAPS;
+    if constexpr (CONV) {
+        if (a.taps > 1) kept = a.state + (long)a.slots[a.row_request[r]] * a.slot_stride + a.state_off;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            if (EARLY) sw_load4(cw[k], a.conv_w + (long)(a.taps - 1) * W + col[k]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) cv[k][i] = 0.0f;
+        }
+        if (early) {
+#pragma unroll
+            for (int j = 0; j < SW_EARLY_TAPS - 1; ++j)
+                if (j + 1 < a.taps) {
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) {
+                        float w[4];
+                        sw_load4(kept_rows[j][k], kept + (long)j * W + col[k]);
+                        sw_load4(w, a.conv_w + (long)j * W + col[k]);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) cv[k][i] = fmaf(w[i], kept_rows[j][k][i], cv[k][i]);
+                    }
+                }
+        }
     }
     ib_grid_dependency_wait();
-    const int r = blockIdx.x;
     const long src = a.rows ? a.rows[r] : r;
-    float x[NV][4], d[NV][4], v[NV][4], cv[CONV ? NV : 1][4];
+    float x[NV][4], d[NV][4], v[NV][4];
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         sw_load4(x[k], a.source + src * W + col[k]);
         if (a.delta) sw_load4(d[k], a.delta + src * W + col[k]);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            v[k][i] = 0.0f;
-            if constexpr (CONV) cv[k][i] = 0.0f;
-        }
+        for (int i = 0; i < 4; ++i) v[k][i] = 0.0f;
     }
     if (a.mix) {
         const float* p = a.planes + src * W;
@@ -98,10 +138,17 @@ __global__ void __launch_bounds__(THREADS) sandwich_norm_vec_kernel(const Sandwi
             }
         }
     }
-    float* kept = nullptr;
     if constexpr (CONV) {
-        if (a.taps > 1) kept = a.state + (long)a.slots[a.row_request[r]] * a.slot_stride + a.state_off;
-        for (int j = 0; j + 1 < a.taps; ++j) {
+        if (early) {
+#pragma unroll
+            for (int j = 1; j < SW_EARLY_TAPS - 1; ++j)
+                if (j + 1 < a.taps) {
+#pragma unroll
+                    for (int k = 0; k < NV; ++k)
+                        if (in[k]) sw_store4(kept + (long)(j - 1) * W + col[k], kept_rows[j][k]);
+                }
+        }
+        for (int j = early ? a.taps : 0; j + 1 < a.taps; ++j) {
 #pragma unroll
             for (int k = 0; k < NV; ++k) {
                 float t[4], w[4];
@@ -121,7 +168,7 @@ __global__ void __launch_bounds__(THREADS) sandwich_norm_vec_kernel(const Sandwi
             for (int k = 0; k < NV; ++k)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) ss = in[k] ? fmaf(d[k][i], d[k][i], ss) : ss;
-            ss = ib_block_sum(ss, red);
+            ss = sw_block_sum(ss, red[0]);
             inv = 1.0f / sqrtf(ss / (float)W + a.post_eps);
         }
 #pragma unroll
@@ -141,23 +188,22 @@ __global__ void __launch_bounds__(THREADS) sandwich_norm_vec_kernel(const Sandwi
         }
         if (in[k] && a.residual) sw_store4(a.residual + src * W + col[k], v[k]);
     }
-    ss = ib_block_sum(ss, red);
+    ss = sw_block_sum(ss, red[1]);
     const float inv = 1.0f / sqrtf(ss / (float)W + a.eps);
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-        float w[4], h[4];
-        sw_load4(w, reinterpret_cast<const WT*>(a.weight) + col[k]);
+        float h[4];
+        if (!EARLY) sw_load4(weight[k], reinterpret_cast<const WT*>(a.weight) + col[k]);
         SandwichVec4 o;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            o.v[i] = ib_from_float<act_t>(v[k][i] * inv * w[i]);
+            o.v[i] = ib_from_float<act_t>(v[k][i] * inv * weight[k][i]);
             h[i] = ib_to_float(o.v[i]);
         }
         if constexpr (CONV) {
-            float cw[4];
-            sw_load4(cw, a.conv_w + (long)(a.taps - 1) * W + col[k]);
+            if (!EARLY) sw_load4(cw[k], a.conv_w + (long)(a.taps - 1) * W + col[k]);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) o.v[i] = ib_from_float<act_t>(fmaf(cw[i], h[i], cv[k][i]) + h[i]);
+            for (int i = 0; i < 4; ++i) o.v[i] = ib_from_float<act_t>(fmaf(cw[k][i], h[i], cv[k][i]) + h[i]);
             if (kept && in[k]) sw_store4(kept + (long)(a.taps - 2) * W + col[k], h);
         }
         if (in[k]) *reinterpret_cast<SandwichVec4*>(a.out + (long)r * W + col[k]) = o;
