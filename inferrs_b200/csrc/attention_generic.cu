@@ -447,6 +447,7 @@ __global__ void __launch_bounds__(32 * T * (G < 4 ? G : 4), 1024 / (32 * T * (G 
         fetch(vs, dv, v_pages, dv, tile, at, false, true);
     }
     ib_grid_dependency_wait();
+    q = ib_after_wait(q);
     fetch(ks, kld, k_pages, d, tile, at, true, !early);
     fetch(vs, dv, v_pages, dv, tile, at, true, !early);
     for (int e = tid; e < group * d; e += THREADS) qs[e] = q[((long)row * n_heads + kvh * group) * d + e];

@@ -367,6 +367,7 @@ latent_attention_mma_kernel(const __nv_bfloat16* __restrict__ q, long q_row, lon
         if (early && t0 < t1) load_tile(t0, false, true);
         ib_grid_dependency_wait();
     }
+    q = ib_after_wait(q);
     // the queries of the group's heads (rows of heads and tokens that do not exist are zeros)
     for (int i = threadIdx.x; i < MR * (R / 8); i += blockDim.x) {
         const int m = i / (R / 8), ch = i % (R / 8);

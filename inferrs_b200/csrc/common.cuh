@@ -147,6 +147,14 @@ __device__ __forceinline__ void ib_grid_dependency_launch() {
 __device__ __forceinline__ void ib_grid_dependency_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// A pointer to what the kernels ahead write, as it is to be used after the wait.  Loads through a `__restrict__` parameter
+// count as loads of numbers that nobody else writes, and the compiler may move them ahead of the wait; through the pointer
+// that comes out of here it cannot.
+template <typename T>
+__device__ __forceinline__ T* ib_after_wait(T* p) {
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
 
 extern int ib_pdl_enabled;  // one per library, defined beside its exported setter ib_set_pdl
 

@@ -126,6 +126,8 @@ __global__ void add_rms_norm_vec4_kernel(float* __restrict__ residual, const act
         if (j < n4) wk[k] = w4[j];
     }
     ib_grid_dependency_wait();
+    residual = ib_after_wait(residual);
+    delta = ib_after_wait(delta);
     const int r = blockIdx.x;
     const int src = rows ? rows[r] : r;
     float4* res = reinterpret_cast<float4*>(residual + (size_t)src * width);

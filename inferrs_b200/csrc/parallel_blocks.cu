@@ -57,6 +57,9 @@ __global__ void __launch_bounds__(SNR_THREADS) sum_norm_route_kernel(
     };
     if (kept) fetch(warp);
     ib_grid_dependency_wait();
+    residual = ib_after_wait(residual);
+    delta = ib_after_wait(delta);
+    plus = ib_after_wait(plus);
     const long r = rows ? rows[blockIdx.x] : blockIdx.x;
     float* res = residual + r * width;
     const bool write_back = rows == nullptr && (delta || bias || plus);

@@ -81,6 +81,7 @@ __global__ void qk_norm_rope_store_kernel(
     const bool clear_tail = kv_place >= 0 && ib_last_row_of_request(row_request, row, gridDim.x);
     const bool norm_after = (norm_flags & 4) != 0;
     ib_grid_dependency_wait();
+    qkv = ib_after_wait(qkv);
 
     // one warp per head: blockIdx.y picks the group of QRS_WARPS heads
     for (int head = blockIdx.y * QRS_WARPS + warp; head < heads_total; head += heads_total) {
@@ -185,6 +186,7 @@ __global__ void qk_norm_rope_store_d128_kernel(
         if (k_weight != nullptr && head0 + HPW > n_heads) wk[e] = ib_to_float(k_weight[4 * lane + e]);
     }
     ib_grid_dependency_wait();
+    qkv = ib_after_wait(qkv);
     uint2 raw[HPW];
 #pragma unroll
     for (int h = 0; h < HPW; ++h)
@@ -285,6 +287,7 @@ __global__ void qk_norm_rope_store_d128_wide_kernel(
         if (has_k) { four(k_weight, e0, wk); four(k_weight, 64 + e0, wk + 4); }
     }
     ib_grid_dependency_wait();
+    qkv = ib_after_wait(qkv);
     uint2 raw_lo[HPW / 2], raw_hi[HPW / 2];
 #pragma unroll
     for (int j = 0; j < HPW / 2; ++j) {
@@ -394,6 +397,7 @@ __global__ void qk_rope_store_shared_kernel(
     const int turning = INTERLEAVED ? rot_dim / VEC : half / VEC;      // items of a head that turn
     const int items = turning + (d - rot_dim) / VEC;                    // items of a head
     ib_grid_dependency_wait();
+    qk = ib_after_wait(qk);
     for (int it = threadIdx.x; it < (n_heads + n_kv_heads) * items; it += blockDim.x) {
         const int head = it / items, k = it - head * items;
         const bool key = head >= n_heads;

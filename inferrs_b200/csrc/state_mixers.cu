@@ -71,6 +71,8 @@ __global__ void scaled_add_norm_vec4_kernel(float* __restrict__ residual, const 
         if (j < n4) wk[k] = reinterpret_cast<const float4*>(weight)[j];
     }
     ib_grid_dependency_wait();
+    residual = ib_after_wait(residual);
+    delta = ib_after_wait(delta);
     float4* res = reinterpret_cast<float4*>(residual + (size_t)blockIdx.x * width);
     const SanActVec4* del = delta ? reinterpret_cast<const SanActVec4*>(delta + (size_t)blockIdx.x * width) : nullptr;
     float4 keep[SAN_KEEP];

@@ -83,6 +83,8 @@ __global__ void stream_add_norm_kernel(float* __restrict__ residual, const act_t
         s_read[threadIdx.x] = read ? read[threadIdx.x] : 1.0f;
     }
     ib_grid_dependency_wait();
+    residual = ib_after_wait(residual);
+    delta = ib_after_wait(delta);
     __syncthreads();
     const int r = blockIdx.x;
     const int src = rows ? rows[r] : r;
@@ -193,6 +195,8 @@ __global__ void __launch_bounds__(512) stream_add_norm_once_kernel(float* __rest
         if (j < width) w[i] = *reinterpret_cast<const Weight4<WT>*>(weight + j);
     }
     ib_grid_dependency_wait();
+    residual = ib_after_wait(residual);
+    delta = ib_after_wait(delta);
     const int r = blockIdx.x;
     const int src = rows ? rows[r] : r;
     float* res = residual + (size_t)src * S * width;
@@ -394,6 +398,8 @@ __global__ void head_norm_gate_vec_kernel(const OT* __restrict__ o, long o_row, 
         }
     }
     ib_grid_dependency_wait();
+    o = ib_after_wait(o);
+    gate = ib_after_wait(gate);
     const OT* src = o + (long)row * o_row + (long)h * o_head;
     const act_t* g = gate ? gate + (long)row * ld_gate + (long)h * e_dim : nullptr;     // no gate: the normed heads alone
     Weight4<OT> v[ITER];
@@ -553,6 +559,7 @@ __global__ void poly_norm_kernel(const act_t* __restrict__ z, const float* __res
     ib_grid_dependency_launch();
     const float a = coef[0], b = coef[1], c = coef[2], e = coef[3];
     ib_grid_dependency_wait();
+    z = ib_after_wait(z);
     const act_t* src = z + (size_t)blockIdx.x * width;
     act_t* dst = out + (size_t)blockIdx.x * width;
     float s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
