@@ -352,9 +352,10 @@ def fuse_rows(tensors: Sequence[torch.Tensor]) -> torch.Tensor:
 class Linear:
     """y = x W^T (+ bias), W stored [out, in] (candle-nn/src/linear.rs:41-82).
 
-    float32 runs: FFMA kernel.  bfloat16 runs: tensor-core product with float32 accumulation for a
-    bfloat16 weight; a weight that is stored in float32 keeps its precision and goes through the
-    FFMA kernel with the bfloat16 activations widened on the fly.
+    float32 runs: exact bfloat16 pieces on the tensor cores over K of 512 and more, the FFMA kernel
+    otherwise.  bfloat16 runs: tensor-core product with float32 accumulation for a bfloat16 weight; a
+    weight that is stored in float32 keeps its precision and goes through the FFMA kernel with the
+    bfloat16 activations widened on the fly.
     """
 
     def __init__(self, weight: torch.Tensor, rt: Runtime, bias: Optional[torch.Tensor] = None):
