@@ -86,7 +86,7 @@ def uniforms_for(seeds, steps):
 
     from ..cache.manager import host_library
 
-    a, b = seeds, steps
+    a, b = (v if hasattr(v, "__len__") else list(v) for v in (seeds, steps))
     if len(a) != len(b):
         if len(a) != 1 and len(b) != 1:
             raise ValueError(f"{len(a)} seeds for {len(b)} steps")

@@ -63,3 +63,4 @@ def test_seeds_of_every_kind_give_the_bits_of_the_plain_generator(copies):
     assert uniforms_for([9], steps).tolist() == uniforms_for([9] * 5 * copies, steps).tolist()
     with pytest.raises(ValueError):
         uniforms_for([1, 2], steps)
+    assert uniforms_for((s for s in seeds), iter(steps)).tolist() == want
