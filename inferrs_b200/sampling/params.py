@@ -2,6 +2,7 @@
 (inferrs/src/sampler.rs:27-112)."""
 from __future__ import annotations
 
+import sys
 from array import array
 from dataclasses import dataclass, field
 from typing import Optional, Tuple
@@ -108,15 +109,20 @@ NATIVE_ROWS = 12     # rows from which the calls into native code cost less than
 
 
 def host_python():
-    """The native functions that read Python's lists (csrc/host_python.cpp), or None where they cannot be built."""
+    """The native functions that read Python's lists (csrc/host_python.cpp), or None where they cannot be built or loaded
+    (tried once: every caller has a way without them)."""
     if not _NATIVE:
         import ctypes
 
-        from ..csrc.build import LIBRARIES, build_library
+        from ..csrc.build import LIBRARIES, BuildError, build_library
 
         lib = None
         if "host_python" in LIBRARIES:
-            lib = ctypes.PyDLL(build_library("host_python"))       # (called with the interpreter's lock held)
+            try:
+                lib = ctypes.PyDLL(build_library("host_python"))       # (called with the interpreter's lock held)
+            except (BuildError, OSError) as e:
+                print(f"[inferrs_b200] without native code for Python's lists: {str(e).splitlines()[0]}", file=sys.stderr, flush=True)
+        if lib is not None:
             i, p, o = ctypes.c_int, ctypes.c_void_p, ctypes.py_object
             lib.ibh_windows.argtypes, lib.ibh_windows.restype = [o, p, p, i, i, p, p], i
             lib.ibh_low_words.argtypes, lib.ibh_low_words.restype = [o, i, p], i

@@ -24,6 +24,7 @@ class Sampler:
         self.act_dtype = act_dtype
         self._staging = []       # [pinned int32 buffer, event of its last copy or None]
         self._turn = 0
+        host_python()            # built with the sampler, not inside a step
 
     def _upload(self, words: np.ndarray) -> torch.Tensor:
         """The step's numbers (int32 words, floats as their bits) to the device with one copy that the host does not

@@ -6,6 +6,8 @@ import random
 import numpy as np
 import pytest
 
+from inferrs_b200.csrc import build
+from inferrs_b200.sampling import params
 from inferrs_b200.sampling.params import host_python, uniform_for, uniforms_for
 from inferrs_b200.sampling.sampler import Sampler
 
@@ -64,3 +66,25 @@ def test_seeds_of_every_kind_give_the_bits_of_the_plain_generator(copies):
     with pytest.raises(ValueError):
         uniforms_for([1, 2], steps)
     assert uniforms_for((s for s in seeds), iter(steps)).tolist() == want
+
+
+@pytest.mark.parametrize("error", [build.BuildError("no compiler"), OSError("cannot be loaded")])
+def test_without_the_native_functions_everything_goes_the_general_way(monkeypatch, error):
+    """A library that cannot be built is asked for once, when a sampler is made, and no step fails for it."""
+    asked = []
+
+    def refuse(name):
+        asked.append(name)
+        raise error
+
+    monkeypatch.setitem(build.LIBRARIES, "host_python", {})
+    monkeypatch.setattr(build, "build_library", refuse)
+    monkeypatch.setattr(params, "_NATIVE", [])
+    torch = pytest.importorskip("torch")
+    Sampler(torch.device("cpu"))
+    assert asked == ["host_python"] and host_python() is None
+    seeds, steps = list(range(20)), list(range(20, 40))
+    assert uniforms_for(seeds, steps).tolist() == [float(np.float32(uniform_for(a, b))) for a, b in zip(seeds, steps)]
+    words, counts = np.empty(4, dtype=np.int32), np.empty(1, dtype=np.int32)
+    assert not Sampler._windows_natively([4], [[1, 2, 3, 4]], [0], 4, words, counts)
+    assert asked == ["host_python"]
