@@ -1844,17 +1844,19 @@ def decode_slices(n_requests: int, n_kv_heads: int, max_kv_len: int):
 
 
 def decode_plan(n_requests: int, n_kv_heads: int, max_kv_len: int) -> dict:
-    """How a decode step's tokens run: :func:`decode_slices`, or, with pairs between a wave and a half and two waves, longest
-    requests first and those beyond the even share in two slices of at least eight tiles (lists of equal requests stay in
-    one slice).  In the order of the list the second wave's longest request runs on alone: a step of 64 requests of 128 to 2,048
-    keys (8 layers of 8B) 1,470 -> 1,385 us.  With more waves the CTAs' starts count and ranking them costs what it gains (96 short
-    requests beside prompts: 4.16 -> 4.18 ms)."""
+    """How a decode step's tokens run: :func:`decode_slices`, or, with pairs between a wave and a half and two waves and room for
+    sixteen tiles, longest requests first and those beyond the even share in two slices of at least eight tiles (lists of
+    equal requests stay in one slice).  In the order of the list the second wave's longest request runs on alone.  With more
+    waves the CTAs' starts count and ranking them costs what it gains (96 short requests beside prompts: 4.16 -> 4.18 ms)."""
     max_splits, min_tiles = decode_slices(n_requests, n_kv_heads, max_kv_len)
-    ranked = max_splits == 1 and 1 < n_requests <= DECODE_RANKED \
-        and DECODE_RESIDENT_CTAS < n_requests * n_kv_heads <= 2 * DECODE_RESIDENT_CTAS
-    return {"max_splits": 2, "min_tiles": 8, "ranked": True} if ranked else {"max_splits": max_splits, "min_tiles": min_tiles}
+    pairs = n_requests * n_kv_heads
+    if 1 < n_requests <= DECODE_RANKED and 3 * DECODE_RESIDENT_CTAS < 2 * pairs <= 4 * DECODE_RESIDENT_CTAS \
+            and max_kv_len > (2 * RANKED_TILES - 1) * MMA_KEYS:
+        return {"max_splits": 2, "min_tiles": RANKED_TILES, "ranked": True}
+    return {"max_splits": max_splits, "min_tiles": min_tiles}
 
 
+RANKED_TILES = 8      # tiles that both slices of a ranked request have at least
 DECODE_RANKED = 256   # requests that the decode kernel ranks (csrc/attention_decode.cu)
 
 

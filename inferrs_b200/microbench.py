@@ -129,10 +129,14 @@ def attention(args) -> dict:
                                                      positions, scale, window, out, True, splits, **per_head)
         else:
             reach = seen(args.context) + 2 * kernels.MMA_KEYS if window else args.context
-            splits, min_tiles = kernels.decode_slices(args.batch, nkv, args.max_context or min(reach, args.context))
-            splits, min_tiles = args.splits or splits, args.min_tiles or min_tiles
+            plan = kernels.decode_plan(args.batch, nkv, args.max_context or min(reach, args.context))
+            if args.splits:
+                plan = {"max_splits": args.splits, "min_tiles": plan["min_tiles"]}
+            if args.min_tiles:
+                plan["min_tiles"] = args.min_tiles
+            splits = plan["max_splits"]
             fn = lambda: kernels.paged_attention_decode(q, k_pages, v_pages, table, positions, scale, window, out,  # noqa: E731
-                                                        splits, min_tiles=min_tiles, **per_head)
+                                                        **plan, **per_head)
         byts = 2 * 2 * sum(seen(n_keys) for n_keys in lens) * nkv * d
         flops = 4 * nh * d * sum(seen(n_keys) for n_keys in lens)
         extra = {"batch": args.batch, "context": args.context, "splits": splits}

@@ -48,6 +48,10 @@ def test_more_requests_than_are_ranked_are_refused_and_the_plan_keeps_to_the_lis
     assert K.decode_plan(64, 8, 4096) == {"max_splits": 2, "min_tiles": 8, "ranked": True}
     assert K.decode_plan(8, 8, 4096) == {"max_splits": 4, "min_tiles": 4}
     assert K.decode_plan(75, 8, 4096) == K.decode_plan(257, 8, 4096) == {"max_splits": 1, "min_tiles": 4}
+    # up to a wave and a half, and where no request has two slices' tiles, the list is as it was
+    for n, keys in ((40, 200), (48, 256), (55, 4096), (56, 512), (64, 256), (64, 960)):
+        assert K.decode_plan(n, 8, keys) == dict(zip(("max_splits", "min_tiles"), K.decode_slices(n, 8, keys)))
+    assert K.decode_plan(56, 8, 961)["ranked"] and K.decode_plan(74, 8, 961)["ranked"]
     table, positions, _, k_pages, v_pages = _paged_setup(torch.bfloat16, 1, 128, 16, [3] * 257, [1] * 257, 9)
     q = rand((257, 1, 128), torch.bfloat16, 10)
     with pytest.raises(K.KernelError):
