@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constan
     const int n_all = n_kept + pos / KEYS + 1 - t_first;
     int n_splits = (n_all + P.min_tiles - 1) / P.min_tiles;
     if (n_splits > P.max_splits) n_splits = P.max_splits;
-    if (P.ranked > 0 && 4 * n_all <= 5 * share) n_splits = 1;
+    if (P.ranked > 0 && (4 * n_all <= 5 * share || n_all < 2 * P.min_tiles)) n_splits = 1;    // (two slices of min_tiles at least)
     if (split >= n_splits) { asm volatile("griddepcontrol.wait;" ::: "memory"); return; }   // an unused slice
     const int per = (n_all + n_splits - 1) / n_splits;
     const int i_begin = split * per;                          // this slice's tiles: places i_begin .. of that list

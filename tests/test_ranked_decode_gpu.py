@@ -13,6 +13,12 @@ from test_kernels_gpu import _paged_setup, rand
 pytestmark = pytest.mark.gpu
 
 
+def cut_in_two(tiles, nkv, min_tiles=8, resident=296):
+    """The requests beyond five quarters of a resident CTA's even share, if both halves have min_tiles."""
+    share = -(-sum(tiles) * nkv // resident)
+    return [4 * t > 5 * share and t >= 2 * min_tiles for t in tiles]
+
+
 @pytest.mark.parametrize("n,nkv,window", [(2, 2, None), (37, 8, None), (64, 8, 300), (255, 1, None), (256, 2, None)])
 def test_ranked_requests_give_what_the_list_gives(n, nkv, window):
     """Lengths around the tiles' edges, equal ones and one far beyond the others (which is cut in two where that pays), alone
@@ -41,6 +47,28 @@ def test_ranked_requests_give_what_the_list_gives(n, nkv, window):
     kept = torch.tensor([i for i in range(n) if i % 3], dtype=torch.long, device="cuda")
     left = torch.tensor([i for i in range(n) if i % 3 == 0], dtype=torch.long, device="cuda")
     assert bool((some[left] == 7.0).all()) and rel_err(some[kept], ref[kept]) < 2e-2
+
+
+@pytest.mark.parametrize("lens,nkv", [
+    ([513, 575, 576, 577, 700, 960, 961, 1023, 1024, 1025] + [40] * 54, 8),      # 9 to 17 tiles: from 16 on in two
+    ([4000] * 14 + [64] * 50, 8), ([300] * 64, 8), ([2000] * 64, 8)])
+def test_two_slices_are_for_long_requests_beyond_the_even_share_alone(lens, nkv):
+    """Every request in one slice has the unranked kernel's bits with one slice, every other one those with two."""
+    from inferrs_b200 import kernels as K
+    n = len(lens)
+    order = random.Random(5).sample(range(n), n)
+    lens = [lens[i] for i in order]
+    table, positions, row_request, k_pages, v_pages = _paged_setup(torch.bfloat16, nkv, 128, 16, lens, [1] * n, 7)
+    q = rand((n, 2 * nkv, 128), torch.bfloat16, 8)
+    one, two, out = (torch.full((n, 2 * nkv * 128), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    K.paged_attention_decode(q, k_pages, v_pages, table, positions, 128 ** -0.5, None, one, 1)
+    K.paged_attention_decode(q, k_pages, v_pages, table, positions, 128 ** -0.5, None, two, 2, min_tiles=8)
+    K.paged_attention_decode(q, k_pages, v_pages, table, positions, 128 ** -0.5, None, out, 2, min_tiles=8, ranked=True)
+    assert K.attention_decode_error() == 0
+    cut = torch.tensor(cut_in_two([(x + 63) // 64 for x in lens], nkv), device="cuda")
+    assert torch.equal(out, torch.where(cut[:, None], two, one))
+    K.paged_attention_decode(q, k_pages, v_pages, table, positions, 128 ** -0.5, None, out, 1, ranked=True)
+    assert torch.equal(out, one)                    # no slices to choose from
 
 
 def test_more_requests_than_are_ranked_are_refused_and_the_plan_keeps_to_the_list():
