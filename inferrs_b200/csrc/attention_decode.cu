@@ -12,7 +12,13 @@
 // More (request, head) pairs than run at a time, in lists of up to 256 requests: CTAs are handed out longest request first (every
 // CTA ranks the requests by their tiles, before it waits for the kernel ahead), and a request of more than five quarters
 // of a resident CTA's even share is cut in two.  In the order of the list, the last head's longest request starts when most CTAs have
-// ended, and runs on alone.
+// ended, and runs on alone.  A place of the grid without work is behind all those with work: before them it would hold one of
+// the resident CTAs' places while the kernel ahead runs, and no keys would be fetched there.  Where more than a wave of
+// CTAs has three quarters of the longest one's tiles there is nothing to gain by an order, and the list's staggers their
+// starts and ends: it is kept, uncut; looking costs a CTA 0.25 us.  Us a layer (32 heads over 8, pages of 16, cold keys) in the list's
+// order / with every second place empty / now: 64 requests of 128 to 2,048 keys 52.4 / 42.5 / 40.8, of 1,000 to 2,000
+// 72.5 / 69.6 / 66.6, of 100 to 700 25.4 / 26.1 / 24.2, 72 of 300 to 2,000 62.8 / 55.3 / 53.4; 64 of 512 31.7 / 35.3 / 32.3, of 1,000
+// 50.7 / 55.0 / 51.2, of 2,048 88.7 / 92.3 / 89.3.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -74,6 +80,7 @@ struct Params {
     const int* reqs;           // [R] or null: its request (row of the block table); a negative row is no work
     int max_pages, page_size, n_pages, n_heads, n_kv_heads, window, max_splits, min_tiles;
     int ranked;                // requests to rank (0: CTAs come in the order of the list)
+    int ranked_places;         // ... and the places for them and for second slices, of each key/value head
     float scale_log2;
     float slope_factor;        // log2(e); with a cap it and scale_log2 carry ib_cap_factor too (see ib_capped_log2)
     float cap_c;
@@ -82,6 +89,14 @@ struct Params {
 
 constexpr int RANKED_MOST = 256;            // requests that are ranked
 constexpr int RESIDENT = 296;               // CTAs that run at a time
+
+// Whether a ranked request of so many tiles is cut in two: beyond five quarters of a resident CTA's even share of all the
+// requests' tiles, and only if both slices have min_tiles.  So 5 * cut requests * heads < 4 * RESIDENT, whatever the
+// lengths: there are no more places than that beyond one per request.
+__device__ __forceinline__ bool ranked_cut(int tiles, int total, int n_kv_heads, int min_tiles) {
+    return 4LL * RESIDENT * tiles > 5LL * total * n_kv_heads && tiles >= 2 * min_tiles;
+}
+constexpr int ranked_cut_most(int n_kv_heads) { return (4 * RESIDENT - 1) / (5 * n_kv_heads); }
 
 // One warp's share of a row: 16 keys of every tile against the group's query heads; scores, softmax in float32, values.
 //
@@ -350,7 +365,8 @@ __device__ __forceinline__ void store_row(const Params& P, __nv_bfloat16* out_ro
 
 // OPTIONS: a factor, a slope and a sink per head, a cap on the scores, a sequence's first keys beside the window, a
 // gate per head.
-template <bool OPTIONS, bool FEW>
+// RANKED is a form of its own: with both in one, either pays for what the other keeps in registers.
+template <bool OPTIONS, bool FEW, bool RANKED>
 __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constant__ CUtensorMap map_k,
                                                             const __grid_constant__ CUtensorMap map_v, const Params P) {
     extern __shared__ unsigned char raw_smem[];
@@ -375,32 +391,73 @@ __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constan
         const int t = ib_first_visible(pos, P.window) / KEYS;
         return ib_kept_tiles(keep, t, KEYS) + pos / KEYS + 1 - t;
     };
-    int place = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z, share = 0;
-    if (P.ranked > 0) {
-        __shared__ __align__(16) int tiles[RANKED_MOST + 4];
-        __shared__ int ranked_place, ranked_total;
-        split = blockIdx.x % P.max_splits;
-        kvh = blockIdx.x / P.max_splits;
-        if (threadIdx.x == 0) ranked_total = 0;
-        for (int i = threadIdx.x; i < P.ranked + 4; i += THREADS) {
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 4); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    int place = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z, ranked_splits = 0, ranked_pos = 0;
+    if constexpr (RANKED) {
+        // keys: a request's tiles, then its place from behind, so that no two are alike; zeros up to the next 64.  (Loops that
+        // are not unrolled further: a CTA runs through this once, and its instructions come from far.)
+        __shared__ __align__(16) unsigned keys[RANKED_MOST];
+        __shared__ int at[RANKED_MOST], by_rank[RANKED_MOST];
+        static_assert(RANKED_MOST % 64 == 0, "");
+        const int padded = (P.ranked + 63) & ~63;
+#pragma unroll 1
+        for (int i = threadIdx.x; i < padded; i += THREADS) {
             const int r = i >= P.ranked ? -1 : P.rows != nullptr ? P.rows[i] : i;
-            tiles[i] = r < 0 ? -1 : tiles_of(P.positions[r]);
+            const int p = r < 0 ? 0 : P.positions[r];
+            keys[i] = i >= P.ranked ? 0u : (unsigned)(r < 0 ? 0 : max(tiles_of(p), 0)) << 8 | (RANKED_MOST - 1 - i);
+            at[i] = p;
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < P.ranked; i += THREADS) {
-            const int mine = tiles[i];
-            int rank = 0;
-            for (int j = 0; j < P.ranked; j += 4) {
-                const int4 t = *reinterpret_cast<const int4*>(tiles + j);
-                rank += (t.x > mine || (t.x == mine && j < i)) + (t.y > mine || (t.y == mine && j + 1 < i)) +
-                        (t.z > mine || (t.z == mine && j + 2 < i)) + (t.w > mine || (t.w == mine && j + 3 < i));
+        // every warp looks at all requests for itself, 64 at a time
+        unsigned most = 0;
+        int near = 0;
+#pragma unroll 1
+        for (int i = lane; i < padded; i += 64) most = max(most, max(keys[i] >> 8, keys[i + 32] >> 8));
+        most = __reduce_max_sync(0xffffffffu, most);
+#pragma unroll 1
+        for (int i = lane; i < padded; i += 64)
+            near += __popc(__ballot_sync(0xffffffffu, 4 * (keys[i] >> 8) > 3 * most)) +
+                    __popc(__ballot_sync(0xffffffffu, 4 * (keys[i + 32] >> 8) > 3 * most));
+        split = 0;
+        ranked_splits = 1;
+        if (near * P.n_kv_heads > RESIDENT) {                 // the list as it is, as without ranks
+            if (kvh >= P.n_kv_heads) { asm volatile("griddepcontrol.wait;" ::: "memory"); return; }
+        } else {
+            const unsigned l = blockIdx.y * gridDim.x + blockIdx.x;
+            const int slot = (int)(l / (unsigned)P.n_kv_heads);
+            kvh = (int)(l - (unsigned)slot * P.n_kv_heads);
+            // the requests in two slices are the first ranks; their slices come first, CTAs without work last
+            int total = 0, cut = 0;
+            if (P.max_splits > 1) {
+#pragma unroll 1
+                for (int i = lane; i < padded; i += 64) total += (int)(keys[i] >> 8) + (int)(keys[i + 32] >> 8);
+                total = __reduce_add_sync(0xffffffffu, total);
+#pragma unroll 1
+                for (int i = lane; i < padded; i += 64)
+                    cut += __popc(__ballot_sync(0xffffffffu, ranked_cut((int)(keys[i] >> 8), total, P.n_kv_heads, P.min_tiles))) +
+                           __popc(__ballot_sync(0xffffffffu, ranked_cut((int)(keys[i + 32] >> 8), total, P.n_kv_heads, P.min_tiles)));
+                cut = min(cut, P.ranked_places - P.ranked);
             }
-            if (rank == (int)blockIdx.y) ranked_place = i;
-            if (mine > 0) atomicAdd(&ranked_total, mine);
+            if (slot >= P.ranked + cut) { asm volatile("griddepcontrol.wait;" ::: "memory"); return; }
+#pragma unroll 1
+            for (int i = threadIdx.x; i < P.ranked; i += THREADS) {
+                const unsigned mine = keys[i];
+                int rank[4] = {0, 0, 0, 0};
+#pragma unroll 2
+                for (int j = 0; j < P.ranked; j += 4) {
+                    const uint4 k = *reinterpret_cast<const uint4*>(keys + j);
+                    rank[0] += k.x > mine; rank[1] += k.y > mine; rank[2] += k.z > mine; rank[3] += k.w > mine;
+                }
+                by_rank[rank[0] + rank[1] + rank[2] + rank[3]] = i;
+            }
+            __syncthreads();
+            if (slot < 2 * cut) { ranked_splits = 2; split = slot & 1; }
+            place = by_rank[slot < 2 * cut ? slot >> 1 : slot - cut];
         }
-        __syncthreads();
-        place = ranked_place;
-        share = (int)(((long)ranked_total * P.n_kv_heads + RESIDENT - 1) / RESIDENT);
+        ranked_pos = at[place];
     }
     const int row = P.rows != nullptr ? P.rows[place] : place;
     // A CTA that has nothing to do still waits for the kernels before this one: a grid that has let its
@@ -409,23 +466,19 @@ __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constan
     if (row < 0) { asm volatile("griddepcontrol.wait;" ::: "memory"); return; }
     const int req = P.reqs != nullptr ? P.reqs[place] : place;
     const int G = P.n_heads / P.n_kv_heads;
-    const int pos = P.positions[row];
+    const int pos = RANKED ? ranked_pos : P.positions[row];
     const int lo = ib_first_visible(pos, P.window);
     const int t_first = lo / KEYS, n_kept = ib_kept_tiles(keep, t_first, KEYS);
     const int n_all = n_kept + pos / KEYS + 1 - t_first;
     int n_splits = (n_all + P.min_tiles - 1) / P.min_tiles;
     if (n_splits > P.max_splits) n_splits = P.max_splits;
-    if (P.ranked > 0 && (4 * n_all <= 5 * share || n_all < 2 * P.min_tiles)) n_splits = 1;    // (two slices of min_tiles at least)
+    if (RANKED) n_splits = ranked_splits;
     if (split >= n_splits) { asm volatile("griddepcontrol.wait;" ::: "memory"); return; }   // an unused slice
     const int per = (n_all + n_splits - 1) / n_splits;
     const int i_begin = split * per;                          // this slice's tiles: places i_begin .. of that list
     const int i_end = i_begin + per < n_all ? i_begin + per : n_all;
     const int n_tiles = i_end > i_begin ? i_end - i_begin : 0;
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 4); }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
     __syncthreads();   // the barriers are ready: the producer starts at once
     bool ok = true;
     if (warp < 4) {
@@ -595,7 +648,7 @@ __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constan
 // request reqs[i] (a negative row is skipped).  part_o [rows, n_heads, max_splits, 128] and part_ml
 // [rows, n_heads, max_splits, 2] are float32 scratch; counters [rows * n_kv_heads] are ints that are zero
 // (the kernel leaves them zero).  Launches that share scratch and counters must not overlap.  ranked: CTAs come longest request first
-// (up to 256 rows), and slices of min_tiles tiles or more are for requests beyond the even share alone.
+// (up to 256 rows), and two slices (max_splits 2 or more), of min_tiles tiles at least, are for requests beyond the even share alone.
 IB_EXPORT int ib_paged_attention_decode(const void* q, const void* k_pages, const void* v_pages, const int* block_table,
                                         int max_pages, int page_size, int n_pages, const int* positions, int n_rows,
                                         int n_heads, int n_kv_heads, int head_dim, float scale, int window, void* out,
@@ -605,7 +658,7 @@ IB_EXPORT int ib_paged_attention_decode(const void* q, const void* k_pages, cons
                                         long out_ld, int ranked, cudaStream_t stream) {
     if (n_rows <= 0) return IB_OK;
     if (min_tiles <= 0) return IB_ERR_ARGUMENT;
-    if (ranked && (n_rows > dec::RANKED_MOST || (long)n_kv_heads * max_splits > 65535)) return IB_ERR_UNSUPPORTED;
+    if (ranked && n_rows > dec::RANKED_MOST) return IB_ERR_UNSUPPORTED;
     if ((rows == nullptr) != (reqs == nullptr)) return IB_ERR_ARGUMENT;
     if (n_heads <= 0 || n_kv_heads <= 0 || n_heads % n_kv_heads || page_size <= 0 || max_pages <= 0 || max_splits <= 0)
         return IB_ERR_ARGUMENT;
@@ -635,24 +688,30 @@ IB_EXPORT int ib_paged_attention_decode(const void* q, const void* k_pages, cons
     P.n_pages = n_pages; P.n_heads = n_heads; P.n_kv_heads = n_kv_heads; P.window = window; P.max_splits = max_splits;
     P.min_tiles = min_tiles;
     P.ranked = ranked ? n_rows : 0;
+    const int most = max_splits > 1 ? dec::ranked_cut_most(n_kv_heads) : 0;
+    P.ranked_places = n_rows + (most < n_rows ? most : n_rows);
     P.scale_log2 = scale * 1.4426950408889634f;
     if (cap > 0.0f) P.scale_log2 *= ib_cap_factor(cap);
     P.slope_factor = 1.4426950408889634f * (cap > 0.0f ? ib_cap_factor(cap) : 1.0f);
     P.cap_c = cap * 1.4426950408889634f;
     P.opt = {head_scale, slopes, sinks, cap, keep_first, (const act_t*)gate, gate_ld, out_ld};
     const size_t smem = 2 * dec::STAGES * dec::TILE_BYTES + 16 * dec::D * 2 + (2 * dec::STAGES + 1) * 8 + 1024;
-    const dim3 grid = ranked ? dim3(n_kv_heads * max_splits, n_rows) : dim3(n_rows, n_kv_heads, max_splits);
+    // (ranked: as many CTAs as the places take, in rows as long as the list)
+    const dim3 grid = ranked ? dim3(n_rows, (unsigned)(((long)P.ranked_places * n_kv_heads + n_rows - 1) / n_rows))
+                             : dim3(n_rows, n_kv_heads, max_splits);
     const bool options = head_scale != nullptr || slopes != nullptr || sinks != nullptr || cap > 0.0f || gate != nullptr || keep_first > 0;
-#define IB_DECODE(OPTIONS, FEW)                                                                                \
-    do {                                                                                                       \
-        static IbDeviceSet configured; /* the attribute is kept per device */                                  \
-        if (const int e = ib_allow_dynamic_smem(configured, dec::decode_kernel<OPTIONS, FEW>, smem)) return e; \
-        ib_launch(dec::decode_kernel<OPTIONS, FEW>, grid, dec::THREADS, smem, stream, mk, mv, P);              \
+#define IB_DECODE(OPTIONS, FEW, RANKED)                                                                                \
+    do {                                                                                                               \
+        static IbDeviceSet configured; /* the attribute is kept per device */                                          \
+        if (const int e = ib_allow_dynamic_smem(configured, dec::decode_kernel<OPTIONS, FEW, RANKED>, smem)) return e; \
+        ib_launch(dec::decode_kernel<OPTIONS, FEW, RANKED>, grid, dec::THREADS, smem, stream, mk, mv, P);              \
     } while (0)
-    if (options && G <= 8) IB_DECODE(true, true);
-    else if (options) IB_DECODE(true, false);
-    else if (G <= 8) IB_DECODE(false, true);
-    else IB_DECODE(false, false);
+#define IB_DECODE2(OPTIONS, FEW) do { if (ranked) IB_DECODE(OPTIONS, FEW, true); else IB_DECODE(OPTIONS, FEW, false); } while (0)
+    if (options && G <= 8) IB_DECODE2(true, true);
+    else if (options) IB_DECODE2(true, false);
+    else if (G <= 8) IB_DECODE2(false, true);
+    else IB_DECODE2(false, false);
+#undef IB_DECODE2
 #undef IB_DECODE
     return ib_launch_status();
 }

@@ -14,9 +14,11 @@ pytestmark = pytest.mark.gpu
 
 
 def cut_in_two(tiles, nkv, min_tiles=8, resident=296):
-    """The requests beyond five quarters of a resident CTA's even share, if both halves have min_tiles."""
-    share = -(-sum(tiles) * nkv // resident)
-    return [4 * t > 5 * share and t >= 2 * min_tiles for t in tiles]
+    """The requests beyond five quarters of a resident CTA's even share, if both halves have min_tiles; none where more than
+    a wave of CTAs has three quarters of the longest one's tiles."""
+    if sum(4 * t > 3 * max(tiles) for t in tiles) * nkv > resident:
+        return [False] * len(tiles)
+    return [4 * resident * t > 5 * sum(tiles) * nkv and t >= 2 * min_tiles for t in tiles]
 
 
 @pytest.mark.parametrize("n,nkv,window", [(2, 2, None), (37, 8, None), (64, 8, 300), (255, 1, None), (256, 2, None)])
@@ -51,7 +53,9 @@ def test_ranked_requests_give_what_the_list_gives(n, nkv, window):
 
 @pytest.mark.parametrize("lens,nkv", [
     ([513, 575, 576, 577, 700, 960, 961, 1023, 1024, 1025] + [40] * 54, 8),      # 9 to 17 tiles: from 16 on in two
-    ([4000] * 14 + [64] * 50, 8), ([300] * 64, 8), ([2000] * 64, 8)])
+    ([2048] * 27 + [1] * 37, 8),                    # nearly as many in two as there can be
+    ([2048] * 37 + [1200] * 27, 8), ([2048] * 38 + [1200] * 26, 8), ([3000] * 38 + [1] * 26, 8),       # a wave of long ones, and one more
+    ([4000] * 14 + [64] * 50, 8), ([1500] * 200 + [3] * 20, 1), ([300] * 64, 8), ([2000] * 64, 8), ([3, 2000], 1)])
 def test_two_slices_are_for_long_requests_beyond_the_even_share_alone(lens, nkv):
     """Every request in one slice has the unranked kernel's bits with one slice, every other one those with two."""
     from inferrs_b200 import kernels as K
