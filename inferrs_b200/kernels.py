@@ -544,7 +544,7 @@ def batched_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act_dtyp
         _check(code, "gemm_tn_simt_batched")
     else:
         code = -1
-        if n <= BATCHED_ROWS and x.dtype == w.dtype == out.dtype == torch.bfloat16:
+        if n <= BATCHED_ROWS and k > 0 and x.dtype == w.dtype == out.dtype == torch.bfloat16:
             # few rows: the library's kernel cannot start before the one ahead has ended, and the one after it waits for it too
             code = _gemm_lib().ib_gemm_tn_rows_batched(_p(x), x.stride(1), x.stride(0), _p(w), _p(out), out.stride(1),
                                                        out.stride(0), n, m, k, b, _stream())

@@ -75,3 +75,11 @@ def test_batch_of_products(n, b, m, k):
         first = torch.empty((b, n, m), dtype=torch.bfloat16, device="cuda")
         K.batched_linear(x, w, first, torch.bfloat16)
         assert torch.equal(first, out.transpose(0, 1))
+
+
+@pytest.mark.parametrize("n", [1, 16, 17])
+def test_batch_of_empty_sums_is_zeros(n):
+    from inferrs_b200 import kernels as K
+    out = torch.full((2, n, 24), float("nan"), dtype=torch.bfloat16, device="cuda")
+    K.batched_linear(rand((2, n, 0), 4), rand((2, 24, 0), 5), out, torch.bfloat16)
+    assert bool((out == 0).all())
