@@ -2,11 +2,19 @@
 // any of the 32 bits.
 //
 // A float32 number has 24 significant bits and bfloat16 has 8, with the same range of exponents: every finite number is exactly
-// the sum of three bfloat16 numbers (its leading eight bits, the next eight of what is left, and the rest).  A product
-// of two numbers is then nine products of their pieces, each exact in float32.  The six largest are taken; the other
-// three are below 2^-22 of the product together, 2^-24 on average.  The tensor cores' float32 accumulators round towards
+// the sum of three bfloat16 numbers (the number rounded to eight bits, what is left rounded again, and the rest: at most 2^-8
+// and 2^-17 of it, of either sign).  A product of two numbers is then nine products of their pieces, each exact in
+// float32.  Eight are taken; the ninth is below 2^-34 of the product.  The tensor cores' float32 accumulators round towards
 // zero, so the one of the largest product is not kept longer than 64 of k: then its value is added to a float32 sum in
-// registers, which rounds to nearest.  The five others have accumulators of their own (two: by size) for a segment of K.
+// registers, which rounds to nearest.  The seven others have accumulators of their own (two: by size) for a segment of K,
+// which are added to each other before they join that sum.
+//
+// Error against 64 bits, of the result's norm, six products of cut pieces / these / a chain of fused multiply-adds: normal x
+// and w, K 512 1.2e-7 / 8.3e-8 / 4.1e-7, K 4,096 1.4e-7 / 1.0e-7 / 1.2e-6; positive ones, K 4,096 1.2e-7 / 7.9e-8 / 8.4e-7; all
+// numbers 1 + 2^-7 - 2^-23, K 512 4.7e-7 / 1.8e-9 / 1.2e-7; sums of a single product 6e-8 / 2.5e-8 / 2.5e-8 (rounded once).  Cutting
+// and leaving out the products of the second and third pieces loses up to 2^-21 of a product, always on one side.  What
+// these cost beside the six: 0 to 1 % up to 64 rows, 2 to 4 % beyond (512 rows, 4,096 features over 1,024: 42.6 -> 43.9 us;
+// 2,048 rows 155 -> 164).
 //
 // The order of the sums depends on K alone, so a row's bits do not depend on how many rows the batch has, where the row
 // stands in it or how the work is cut: the ceil(K / 64) blocks fall into eight segments of equal length (the last may
@@ -24,7 +32,7 @@
 //   warps 8-    the sums: four warps, or beyond 16 tokens eight with half of the tokens each
 //
 // What bounds it (512 rows, 4,096 features over 1,024): 44 us = 98 TFLOP/s, where a chain of multiply-adds took 110 to 160 us
-// (36 TFLOP/s); 2,048 rows 111.  The tensor pipe is busy 30 % of the time, the issue slots 52, memory hands over 0.4 TB/s: the
+// (36 TFLOP/s); 2,048 rows 105.  The tensor pipe is busy 40 % of the time, the issue slots 53, memory hands over 0.4 TB/s: the
 // warps that make the pieces and add up are what a block of 64 of k waits for.  With two warps for x's pieces instead of
 // four 45.8 us, with four summing warps instead of eight 63.5.  Up to 16 rows: a row 7 to 10 us, the way of x
 // and the cluster's exchange; memory takes 1.3 to 4 of them.
@@ -91,16 +99,17 @@ __device__ __forceinline__ void st_cluster(unsigned local_addr, unsigned rank, f
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
 }
 
-// Two neighbouring numbers of K as three pairs of bfloat16, the first in the low half.  Cutting (not rounding) keeps every
-// piece's sign and makes the differences exact.
+// Two neighbouring numbers of K as three pairs of bfloat16, the first in the low half.  Every piece is what is left, rounded
+// to nearest; the differences are exact.  (Beyond 3.39e38 the first piece is an infinity: see `finished`.)
+__device__ __forceinline__ unsigned pack_pair(float a, float b) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const unsigned*>(&v);
+}
 __device__ __forceinline__ void split_pair(float a, float b, unsigned& p0, unsigned& p1, unsigned& p2) {
-    p0 = __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
-    const float a1 = a - __uint_as_float(__float_as_uint(a) & 0xffff0000u);
-    const float b1 = b - __uint_as_float(__float_as_uint(b) & 0xffff0000u);
-    p1 = __byte_perm(__float_as_uint(a1), __float_as_uint(b1), 0x7632);
-    const float a2 = a1 - __uint_as_float(__float_as_uint(a1) & 0xffff0000u);
-    const float b2 = b1 - __uint_as_float(__float_as_uint(b1) & 0xffff0000u);
-    p2 = __byte_perm(__float_as_uint(a2), __float_as_uint(b2), 0x7632);
+    p0 = pack_pair(a, b);
+    const float a1 = a - __uint_as_float(p0 << 16), b1 = b - __uint_as_float(p0 & 0xffff0000u);
+    p1 = pack_pair(a1, b1);
+    p2 = pack_pair(a1 - __uint_as_float(p1 << 16), b1 - __uint_as_float(p1 & 0xffff0000u));
 }
 
 // The result of one row and feature as one chain of fused multiply-adds: what infinities and NaN make of it.
@@ -276,11 +285,14 @@ __global__ void __launch_bounds__(threads_of(BN), (BN <= 16 ? 2 : 1)) split_kern
 #pragma unroll
                 for (int k = 0; k < BK / 16; ++k) {
                     const unsigned a0 = a + k * 8, a1 = a0 + BK / 2, a2 = a1 + BK / 2;
-                    const unsigned long long b0 = b + (unsigned long long)((k * 32) >> 4), b1 = b0 + (unsigned long long)(PIECE >> 4);
+                    const unsigned long long b0 = b + (unsigned long long)((k * 32) >> 4), b1 = b0 + (unsigned long long)(PIECE >> 4),
+                                             b2 = b1 + (unsigned long long)(PIECE >> 4);
                     umma_ts(small, a0, b1, idesc2, (m | k) != 0);
                     umma_ts(d, a0, b0, idesc1, k != 0);
                     umma_ts(small, a1, b0, idesc2, 1);
                     umma_ts(small + BN, a2, b0, idesc1, 1);
+                    umma_ts(small + BN, a1, b2, idesc1, 1);
+                    umma_ts(small, a2, b1, idesc1, 1);
                 }
                 umma_commit(done0 + 8 * s);
                 if (++m == p.blocks_per_segment) { m = 0; ++segment; }
@@ -392,9 +404,15 @@ __global__ void __launch_bounds__(threads_of(BN), (BN <= 16 ? 2 : 1)) split_kern
                 ok = __all_sync(0xffffffffu, ok);            // one answer per warp: the loads below are warp-wide
                 if (!ok) break;
                 fence_after();
-                if (m == p.blocks_per_segment - 1 || i == n_blocks - 1) {   // the segment's last: its small products, smallest first
-                    add(lanes + TMEM_SMALL + BN);
-                    add(lanes + TMEM_SMALL);
+                if (m == p.blocks_per_segment - 1 || i == n_blocks - 1) {   // the segment's last: its small products join once
+#pragma unroll
+                    for (int h = 0; h < C; h += 16) {
+                        float v[16], u[16];
+                        tmem_ld16(lanes + TMEM_SMALL + BN + h, v);
+                        tmem_ld16(lanes + TMEM_SMALL + h, u);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) sum[h + j] += v[j] + u[j];
+                    }
                     fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(small0);

@@ -924,8 +924,8 @@ def gemm_split_supported(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) ->
 
 def gemm_tn_split(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, splits: int = 0, tile_rows: int = 0):
     """out = x @ w.T for float32 tensors on the tensor cores: every number as the exact sum of three bfloat16 pieces,
-    the six largest of the nine products of pieces, sums in float32 (closer to 64 bits than a chain of fused
-    multiply-adds).  ``splits`` CTAs (1, 2, 4, 8) share a tile of ``tile_rows`` rows of w; 0 lets the library choose.
+    eight of the nine products of pieces (the ninth is below 2^-34 of the product), sums in float32 (closer to 64 bits than a
+    chain of fused multiply-adds).  ``splits`` CTAs (1, 2, 4, 8) share a tile of ``tile_rows`` rows of w; 0 lets the library choose.
     Neither changes a bit of the result."""
     for name, t in (("x", x), ("w", w), ("out", out)):
         _need(t, name, (torch.float32,), 2)

@@ -12,11 +12,11 @@ def rand(shape, seed):
 
 
 def bound(x, w):
-    """Of sum |x w|: the three products of pieces that are left out (2^-22); four additions of a block of 64 of k in an
-    accumulator that rounds towards zero (2^-23 each); the small products, 2^-6 of the whole, over a segment of K / 8 in
-    such accumulators (3 K / 128 additions); then up to K / 512 + 6 rounded additions of 2^-24."""
+    """Of sum |x w|: the product of the two smallest pieces, which is left out (2^-34); four additions of a block of 64 of k in
+    an accumulator that rounds towards zero (2^-23 each); the small products, 2^-6 of the whole, over a segment of K / 8 in
+    such accumulators (7 K / 128 additions); then up to K / 512 + 5 rounded additions of 2^-24."""
     k = x.shape[1]
-    return (2.0 ** -22 + 4 * 2.0 ** -23 + (3 * k / 128 + 12) * 2.0 ** -29 + (k / 512 + 6) * 2.0 ** -24) \
+    return (2.0 ** -34 + 4 * 2.0 ** -23 + (7 * k / 128 + 12) * 2.0 ** -29 + (k / 512 + 5) * 2.0 ** -24) \
         * (x.double().abs() @ w.double().abs().t())
 
 
@@ -72,3 +72,58 @@ def test_linear_takes_the_split_product_by_its_width_alone():
         ref = torch.empty((70, 96), device="cuda")
         (K.gemm_tn_split if k >= 512 and k % 4 == 0 else lambda a, b, c: K.gemm_tn_simt(a, b, c, torch.float32))(x, w, ref)
         assert torch.equal(out[0], ref) and torch.equal(out[1], ref[:3])
+
+
+@pytest.mark.parametrize("n,m,k", [(3, 70, 512), (16, 130, 1000), (17, 70, 4096), (64, 130, 1024), (130, 70, 3072)])
+def test_a_sum_of_one_product_is_rounded_once(n, m, k):
+    """One number of a row of x that is not zero, at every place of a block of k and in every segment: the product in 64 bits
+    rounded to 24 (2^-24; the small pieces' products, 2^-6 of it, meet five additions that round towards zero), no worse than the
+    chain of multiply-adds.  And with numbers whose pieces are the largest that there can be."""
+    from inferrs_b200 import kernels as K
+    worst = torch.tensor([1 + 2.0 ** -7 - 2.0 ** -23, 1 + 2.0 ** -8 - 2.0 ** -23, 1 + 2.0 ** -8 + 2.0 ** -16, 2 - 2.0 ** -23], device="cuda")
+    x, w = torch.zeros((n, k), device="cuda"), rand((m, k), 8)
+    w[:4] = worst[:, None]
+    at = torch.arange(n, device="cuda") * 61 % k
+    x[torch.arange(n), at] = torch.cat([worst, rand((n,), 9)])[:n]
+    out, chain = torch.empty((n, m), device="cuda"), torch.empty((n, m), device="cuda")
+    K.gemm_tn_split(x, w, out)
+    K.gemm_tn_simt(x, w, chain, torch.float32)
+    want = x.double() @ w.double().t()
+    err, err_chain = (out.double() - want).abs(), (chain.double() - want).abs()
+    assert bool((err <= (2.0 ** -24 + 5 * 2.0 ** -29) * want.abs()).all())
+    assert float(err.norm()) <= 1.01 * float(err_chain.norm())
+
+
+@pytest.mark.parametrize("kind", ["worst", "positive", "one beyond the others"])
+@pytest.mark.parametrize("n,k", [(8, 512), (70, 2048), (20, 4096)])
+def test_numbers_of_one_sign_and_sums_that_few_products_make(kind, n, k):
+    """No part of a product is left out on one side: where every product would lose the same, and where one makes the sum,
+    the result is within the bound and nearer to 64 bits than the chain's."""
+    from inferrs_b200 import kernels as K
+    if kind == "worst":
+        x, w = torch.full((n, k), 1 + 2.0 ** -7 - 2.0 ** -23, device="cuda"), torch.full((96, k), 1 + 2.0 ** -7 - 2.0 ** -23, device="cuda")
+    elif kind == "positive":
+        x, w = rand((n, k), 10).abs(), rand((96, k), 11).abs()
+    else:
+        x, w = 1e-4 * rand((n, k), 12), rand((96, k), 13)
+        x[:, k // 2] = 1 + rand((n,), 14).abs()
+    out, chain = torch.empty((n, 96), device="cuda"), torch.empty((n, 96), device="cuda")
+    K.gemm_tn_split(x, w, out)
+    K.gemm_tn_simt(x, w, chain, torch.float32)
+    want = x.double() @ w.double().t()
+    err, err_chain = (out.double() - want).abs(), (chain.double() - want).abs()
+    assert bool((err <= bound(x, w)).all()) and float(err.norm()) <= float(err_chain.norm())
+
+
+def test_numbers_whose_first_piece_would_be_an_infinity():
+    """Beyond 3.39e38 a number rounded to bfloat16 is none: such results are made as the chain makes them."""
+    from inferrs_b200 import kernels as K
+    x, w = rand((5, 512), 15), rand((130, 512), 16)
+    x[2], w[7] = 0.0, 0.0
+    x[2, 3], w[7, 5] = 3.4e38, -3.4028234e38
+    w[:, 3] = 0.5
+    out, chain = torch.empty((5, 130), device="cuda"), torch.empty((5, 130), device="cuda")
+    K.gemm_tn_split(x, w, out)
+    K.gemm_tn_simt(x, w, chain, torch.float32)
+    assert torch.equal(out[2], chain[2]) and bool(out[2].isfinite().all())
+    assert torch.equal(out[:, 7].nan_to_num(1.0, 2.0, 3.0), chain[:, 7].nan_to_num(1.0, 2.0, 3.0))
