@@ -38,8 +38,9 @@
 // and the cluster's exchange; memory takes 1.3 to 4 of them.
 //
 // Infinities and NaN: the pieces of an infinity are no numbers, so a result that is not finite is computed again as
-// one chain of fused multiply-adds, by the thread that would store it.  Numbers below 2^-102 have pieces that bfloat16 holds only
-// partly: an absolute error of 2^-133 times the other factor.
+// one chain of fused multiply-adds, by the thread that would store it.  Numbers below 2^-110 have pieces that bfloat16 holds only
+// partly, an absolute error of 2^-134 times the other factor: a result below 2^-90, which may be made of such numbers,
+// is computed again too (but for zeros: rows of zeros are common, and only numbers below 2^-133 vanish).
 //
 // Every wait on an mbarrier is bounded (about two seconds); a wait that runs out records a code in the library's error
 // word, the CTA lets outstanding copies land, frees its tensor memory and returns.
@@ -112,14 +113,16 @@ __device__ __forceinline__ void split_pair(float a, float b, unsigned& p0, unsig
     p2 = pack_pair(a1 - __uint_as_float(p1 << 16), b1 - __uint_as_float(p1 & 0xffff0000u));
 }
 
-// The result of one row and feature as one chain of fused multiply-adds: what infinities and NaN make of it.
+// The result of one row and feature as one chain of fused multiply-adds: what infinities and NaN make of it, and numbers
+// whose pieces are too small for bfloat16.
 __device__ __noinline__ float chain(const float* x, const float* w, int k) {
     float s = 0.0f;
     for (int i = 0; i < k; ++i) s = fmaf(x[i], w[i], s);
     return s;
 }
 __device__ __forceinline__ float finished(const Params& p, float v, int tok, int feature) {
-    return fabsf(v) <= 3.402823466e38f ? v : chain(p.x + (long)tok * p.ldx, p.w + (long)feature * p.ldw, p.k);
+    const float a = fabsf(v);
+    return a <= 3.402823466e38f && (a >= 8.077935669e-28f || a == 0.0f) ? v : chain(p.x + (long)tok * p.ldx, p.w + (long)feature * p.ldw, p.k);
 }
 
 // A segment's sum joins those before it: like the carry of a binary counter, so that equal powers of two of segments

@@ -127,3 +127,21 @@ def test_numbers_whose_first_piece_would_be_an_infinity():
     K.gemm_tn_simt(x, w, chain, torch.float32)
     assert torch.equal(out[2], chain[2]) and bool(out[2].isfinite().all())
     assert torch.equal(out[:, 7].nan_to_num(1.0, 2.0, 3.0), chain[:, 7].nan_to_num(1.0, 2.0, 3.0))
+
+
+@pytest.mark.parametrize("n,k", [(5, 512), (40, 1024), (70, 1024)])
+def test_numbers_whose_pieces_are_too_small_for_bfloat16(n, k):
+    """A result below 2^-90 is the chain's; one row of zeros among them stays zero."""
+    from inferrs_b200 import kernels as K
+    w = rand((96, k), 18)
+    for power in (-96, -110, -120, -126):
+        x = rand((n, k), 17) * 2.0 ** power
+        x[n // 2] = 0.0
+        out, chain = torch.empty((n, 96), device="cuda"), torch.empty((n, 96), device="cuda")
+        K.gemm_tn_split(x, w, out)
+        K.gemm_tn_simt(x, w, chain, torch.float32)
+        small = chain.abs() < 2.0 ** -90
+        assert bool(small.any()) and torch.equal(out[small], chain[small])
+        want = x.double() @ w.double().t()
+        assert bool(((out.double() - want).abs() <= torch.where(small, 2.0 ** -23 * k ** 0.5 * (x.double().abs() @ w.double().abs().t()),
+                                                               bound(x, w)) + 2.0 ** -148).all())
