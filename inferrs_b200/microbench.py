@@ -1,6 +1,7 @@
 """Timing of single kernels at given sizes: the commands behind the summaries in ``profiles/``.
 
     python -m inferrs_b200.microbench gemm --impl tcgen05 --m 8 --n 6144 --k 4096
+    python -m inferrs_b200.microbench gemm --impl split --m 512 --n 4096 --k 1024
     python -m inferrs_b200.microbench attention --form decode --batch 8 --context 2048
     python -m inferrs_b200.microbench attention --form prefill --tokens 2048
     python -m inferrs_b200.microbench chain --impl library --m 8 --layers 8
@@ -62,15 +63,18 @@ def gemm(args) -> dict:
         return {"kernel": "gemm/gated", "m": args.m, "n": 2 * inner, "k": args.k, "us": round(us, 2),
                 "GBps": round(byts / us / 1e3, 1), "TFLOPs": round(4 * args.m * inner * args.k / us / 1e6, 1),
                 "rel_err": err}
-    x = torch.randn(args.m, args.k, device="cuda").to(torch.bfloat16)
-    w = (torch.randn(args.n, args.k, device="cuda") * 0.02).to(torch.bfloat16)
-    out = torch.empty(args.m, args.n, dtype=torch.bfloat16, device="cuda")
+    dtype = torch.float32 if args.impl in ("split", "ffma") else torch.bfloat16
+    x = torch.randn(args.m, args.k, device="cuda").to(dtype)
+    w = (torch.randn(args.n, args.k, device="cuda") * 0.02).to(dtype)
+    out = torch.empty(args.m, args.n, dtype=dtype, device="cuda")
     fn = {"library": lambda: kernels.gemm_tn_bf16(x, w, out),
-          "tcgen05": lambda: kernels.gemm_tn_tcgen05(x, w, out, args.split_k)}[args.impl]
+          "tcgen05": lambda: kernels.gemm_tn_tcgen05(x, w, out, args.split_k),
+          "split": lambda: kernels.gemm_tn_split(x, w, out, max(args.split_k, 0)),
+          "ffma": lambda: kernels.gemm_tn_simt(x, w, out, torch.float32)}[args.impl]
     us = _time(fn, args.iters)
-    ref = x.float() @ w.float().t()
-    err = float((out.float() - ref).abs().max() / ref.abs().max())
-    byts = 2 * (args.n * args.k + args.m * args.k + args.m * args.n)
+    ref = x.double() @ w.double().t() if dtype == torch.float32 else x.float() @ w.float().t()
+    err = float((out.double() - ref).abs().max() / ref.abs().max())
+    byts = x.element_size() * (args.n * args.k + args.m * args.k + args.m * args.n)
     flops = 2 * args.m * args.n * args.k
     return {"kernel": f"gemm/{args.impl}", "m": args.m, "n": args.n, "k": args.k, "us": round(us, 2),
             "GBps": round(byts / us / 1e3, 1), "TFLOPs": round(flops / us / 1e6, 1), "rel_err": err}
@@ -817,8 +821,9 @@ def main(argv=None) -> int:
                          "evenly over the SMs")
     sub = ap.add_subparsers(dest="what", required=True)
     g = sub.add_parser("gemm")
-    g.add_argument("--impl", choices=["library", "tcgen05", "gated"], default="tcgen05",
-                   help="gated: both products of a gated feed-forward and the gate in one tcgen05 kernel")
+    g.add_argument("--impl", choices=["library", "tcgen05", "gated", "split", "ffma"], default="tcgen05",
+                   help="gated: both products of a gated feed-forward and the gate in one tcgen05 kernel; split, ffma: "
+                        "32-bit products in pieces and as chains of multiply-adds")
     g.add_argument("--m", type=int, default=8)
     g.add_argument("--n", type=int, default=6144)
     g.add_argument("--k", type=int, default=4096)
