@@ -38,6 +38,7 @@ def test_streams_update_and_norm(streams, groups, width, dtype):
     res, out = x.cuda(), torch.empty((n, width), dtype=dtype, device="cuda")
     K.stream_add_norm(res, delta.cuda(), mix.cuda(), gain.cuda(), read.cuda(), weight.cuda(), groups, eps, out)
     assert near(res, new) and near(out, normed(torch.einsum("t,ntw->nw", read.double(), new)), 24)
+    among = out
     rows, kept = torch.tensor([4, 0], dtype=torch.int32, device="cuda"), res.clone()
     out = torch.empty((2, width), dtype=dtype, device="cuda")
     K.stream_add_norm(res, None, None, None, None, weight.cuda(), groups, eps, out, rows)
@@ -45,7 +46,7 @@ def test_streams_update_and_norm(streams, groups, width, dtype):
     # one row alone has the bits of the row among others
     one, alone = x[2:3].cuda(), torch.empty((1, width), dtype=dtype, device="cuda")
     K.stream_add_norm(one, delta[2:3].cuda(), mix.cuda(), gain.cuda(), read.cuda(), weight.cuda(), groups, eps, alone)
-    assert torch.equal(one[0], res[2])
+    assert torch.equal(one[0], res[2]) and torch.equal(alone[0], among[2])
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
@@ -68,3 +69,50 @@ def test_heads_normed_and_gated(e_dim, gate_act, normed, shared, dtype):
             K.head_norm_gate(o.cuda(), wide.cuda()[:, offset:offset + heads * e_dim], w.cuda(), normed,
                              K.GATE_SILU if gate_act == 0 else K.GATE_SIGMOID, eps, out)
             assert near(out, want)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width,taps", [(128, 4), (516, 5), (2048, 6), (2052, 3), (4096, 4), (4096, 5), (4100, 2), (8192, 4)])
+def test_kept_rows_of_the_norm_with_a_convolution(width, taps, dtype):
+    """Taps below, at and beyond those that are fetched before the wait, in every number of groups a thread has: three layers
+    a step, each on what the one before left, as a replayed graph with early starts, for three steps."""
+    from inferrs_b200 import kernels as K
+    n, layers, eps = 3, 3, 1e-5
+    delta, weight = rand((layers, n, width), 1).to(dtype).cuda(), (1 + 0.2 * rand((layers, width), 2)).cuda()
+    conv_w, start = 0.3 * rand((layers, taps, width), 3).cuda(), rand((n, width), 4).cuda()
+    keep = (taps - 1) * width
+    first = rand((n + 1, layers * keep), 5).cuda()
+    slots, req = (torch.tensor(t, dtype=torch.int32, device="cuda") for t in ([2, 0, 3], [1, 0, 2]))
+    state, stream, out = first.clone(), torch.empty((n, width), device="cuda"), torch.empty((layers, n, width), dtype=dtype, device="cuda")
+
+    def step():
+        stream.copy_(start)
+        for i in range(layers):
+            K.sandwich_norm(stream, delta[i], None, 0.0, weight[i], eps, out[i], residual=stream,
+                            conv=(conv_w[i], state, i * keep, slots, req))
+
+    step()
+    torch.cuda.synchronize()
+    state.copy_(first)
+    K.set_pdl(True, dtype)
+    graph = torch.cuda.CUDAGraph()
+    try:
+        with torch.cuda.graph(graph):
+            step()
+    finally:
+        K.set_pdl(False, dtype)
+    at = [[2, 0, 3][r] for r in [1, 0, 2]]
+    kept = first[at].double().cpu().reshape(n, layers, taps - 1, width)
+    for _ in range(3):
+        graph.replay()
+        x = start.double().cpu()
+        for i in range(layers):
+            x = x + delta[i].double().cpu()
+            want = x / (x.pow(2).mean(-1, keepdim=True) + eps).sqrt() * weight[i].double().cpu()
+            h = state[at][:, i * keep:(i + 1) * keep].reshape(n, taps - 1, width)[:, -1].double().cpu()      # as it was rounded
+            assert near(h.to(dtype), want, 24)
+            w = conv_w[i].double().cpu()
+            got = h * (1 + w[-1]) + (kept[:, i] * w[None, :-1]).sum(1)
+            assert near(out[i], got, 24)
+            kept[:, i] = torch.cat([kept[:, i, 1:], h[:, None]], 1)
+    assert torch.equal(state[at].double().cpu().reshape(kept.shape), kept) and torch.equal(state[1], first[1])
