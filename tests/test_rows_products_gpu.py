@@ -83,3 +83,50 @@ def test_batch_of_empty_sums_is_zeros(n):
     out = torch.full((2, n, 24), float("nan"), dtype=torch.bfloat16, device="cuda")
     K.batched_linear(rand((2, n, 0), 4), rand((2, 24, 0), 5), out, torch.bfloat16)
     assert bool((out == 0).all())
+
+
+@pytest.mark.parametrize("b,n,k", [(1, 1, 8), (3, 16, 72), (16, 9, 512)])
+def test_batches_run_on_the_kernel_for_few_rows(b, n, k):
+    """The library function itself takes whole rows of either layout, and leaves those that do not start on 16 bytes."""
+    from inferrs_b200 import kernels as K
+    lib, m = K._gemm_lib(), 40
+    w, out = rand((b, m, k), 4, 0.1), torch.empty((b, n, m), dtype=torch.bfloat16, device="cuda")
+
+    def call(x):
+        out.fill_(float("nan"))
+        return lib.ib_gemm_tn_rows_batched(x.data_ptr(), x.stride(1), x.stride(0), w.data_ptr(), out.data_ptr(), out.stride(1),
+                                           out.stride(0), n, m, k, b, torch.cuda.current_stream().cuda_stream)
+
+    for x in (rand((n, b, k + 8), 5)[:, :, :k].transpose(0, 1), rand((b, n, k), 6)):
+        assert call(x) == 0
+        terms = k * 2.0 ** -24 * torch.einsum("bnk,bmk->bnm", x.double().abs(), w.double().abs())
+        assert close(out, torch.einsum("bnk,bmk->bnm", x.double(), w.double()), terms)
+    assert call(rand((b, n, k + 1), 7)[:, :, 1:]) == -1 and bool(out.isnan().all())
+
+
+@pytest.mark.parametrize("m,k", [(m, 72) for m in (8 * 148, 8 * 148 + 1, 32 * 148, 32 * 148 + 1, 32 * 296, 32 * 296 + 1, 48 * 296,
+                                                   48 * 296 + 1, 4 * 48 * 296 - 1, 4 * 48 * 296)]
+                         + [(m, k) for m in (8 * 148, 8 * 148 + 1, 32 * 148, 32 * 148 + 1) for k in (4096, 4104)])
+def test_products_beside_the_lines_of_the_rule(m, k):
+    """`linear` and `gated_linear` on both sides of every size and row count at which another form is chosen."""
+    from inferrs_b200 import kernels as K
+    x, w = rand((17, k), 1), rand((m, k), 2, 0.05)
+    dot, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    for n in (1, 8, 9, 16, 17):
+        for dtype in (torch.bfloat16, torch.float32):
+            out = torch.full((n, m), float("nan"), dtype=dtype, device="cuda")
+            if n <= 16:                                      # (more rows are the library's)
+                K.linear(x[:n], w, out, torch.bfloat16)
+                assert close(out, dot[:n], k * 2.0 ** -24 * size[:n])
+        inner = m // 2
+        out = torch.full((n, inner), float("nan"), dtype=torch.bfloat16, device="cuda")
+        K.gated_linear(x[:n], w[:2 * inner], out, torch.bfloat16)
+        g, u = dot[:n, :inner], dot[:n, inner:2 * inner]
+        want = g / (1 + torch.exp(-g)) * u
+        off = k * 2.0 ** -24 * size[:n]
+        off_g, off_u = off[:, :inner], off[:, inner:2 * inner]
+        # as above, and the gate's fast exponential and division of more rows (2^-20)
+        slack = (2.0 ** -8 * 1.11 + 2.0 ** -20) * g.abs() * u.abs() + 2.0 ** -8 * 2.1 * want.abs() \
+            + 1.2 * (off_g * u.abs() + off_u * g.abs() + off_g * off_u)
+        assert bool(((out.double() - want).abs() <= slack).all())
+    assert K.gemm_tcgen05_error() == 0
