@@ -868,6 +868,12 @@ static int launch_any(int r, const void* w, long n_w, long ldw, const void* x, l
 //              4,096 over 4,096 12.2 / 12.1 / -  / 9.8            gated 12,288 over 4,096  36.4 / 39.8
 //              2,048 over 8,192 12.5 / 18.5 / -  / 12.8           10,240 over 5,120  21.7 / 35.6 / -  / 25.8
 // Boxes of few rows are what a long K does not want; more CTAs than two an SM are a second wave with fetches of its own.
+// 9 to 16 tokens between 4,736 and 9,472 features, tcgen05 / 16 / 32 rows: 6,144 over 4,096 13.2 / 19.8 / 10.2, 8,192 over 2,048
+// 10.2 / 11.8 / 7.1, 9,472 over 5,120 20.2 / 30.0 / 16.5.  Gated, up to 8 tokens, tcgen05 / 16 / 24: 512 over 4,096 22.3 / 5.7 /
+// 6.3, 6,144 over 2,048 14.4 / 11.6 / 8.6, 8,192 over 4,096 27.3 / 22.9 / 24.7, 25,600 over 5,120 92.8 / 79.4 / 76.0.  Of 1, 8, 9 and 16
+// tokens and 4,736 to 151,936 features over 1,024 to 8,192 (gated 512 to 25,600) no product is slower than on tcgen05.  Where
+// the rule leaves tcgen05 its products, others would be faster at some sizes: 8 tokens, 16,384 over 4,096 26.4, in 32 rows 22.2; 16
+// tokens, 151,936 over 1,024 63.6, 57.1; gated, 16 tokens, 8,192 over 4,096 29.3, in 16 rows 24.5 (32,000 over 2,048 to 5,120: equal).
 //
 // With the deep ring (a CTA per SM), 1 / 8 / 16 tokens, 16 rows and 32 rows a CTA, against the best above: 1,024 over 3,072 3.7
 // / 3.8 / 4.4 and 4.1 / 4.1 / 4.8 (4.3 / 4.3 / 4.7); 2,048 over 2,048 3.5 / 4.1 / 5.2 both (4.0 / 4.6 / 6.4); over 8,192 12.0
