@@ -197,8 +197,12 @@ class PortionGraphs:
     the model's attention layers ask for) and is then captured.
     """
 
-    # (beyond a thousand rows a step's time is in proportion to them, padding included: the distances narrow.  1,758 rows of a
-    # 0.6B model 4.32 ms as 2,048, 4.16 as 1,792)
+    # A step's time grows with its rows, padding included, from a few hundred on; beyond a thousand the distances narrow.  ms as
+    # 2,048 rows / as the next of these: 0.6B 1,100 rows 3.42 / 2.50, 1,600 3.44 / 3.09, 1,758 beside 96 single tokens 4.32 / 4.16; eight
+    # layers of 8B 1,100 4.62 / 3.41, 1,600 4.95 / 4.42.  Every captured step costs 0.05 to 0.3 s and its buffers: 44 MB (0.6B), 63 to
+    # 88 MB (8B), up to 185 MB (32B) for each of the three row counts and numbers of requests with tiles that occur, which
+    # is why there are none between 512 and 1,024.  The library's products sum in float32 at all of these (the same bits with
+    # torch's bfloat16 reductions forbidden), but not with one algorithm: a row's last bits follow its step's row count.
     ROW_BUCKETS = (32, 64, 128, 256, 512, 1024, 1280, 1536, 1792, 2048, 4096)
     TILE_PADS = (8,)                 # ... and as many requests as the cache admits
 
