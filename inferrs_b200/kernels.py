@@ -524,7 +524,8 @@ def batched_linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, act_dtyp
     """out[b] = x[b] @ w[b].T for b < B: ``x`` [B, rows, K] (any view with unit last stride, so the heads of a
     [rows, B*K] tensor are multiplied in place), ``w`` [B, M, K] contiguous, ``out`` [B, rows, M] (likewise a view with
     unit last stride: the heads of a [rows, B*M] tensor are written in place).  True 32-bit
-    products with float32 activations or weights, else the tensor cores (the vendor's batched product)."""
+    products with float32 activations or weights, else the tensor cores: up to ``BATCHED_ROWS`` bfloat16 rows that start on 16
+    bytes on the kernel for few rows, everything else as the vendor's batched product."""
     if x.dim() != 3 or w.dim() != 3 or out.dim() != 3 or x.stride(2) != 1:
         raise KernelError("batched_linear: x, w and out must have three dimensions, x with unit last stride")
     _need(w, "w", _W, 3)
