@@ -87,7 +87,8 @@ def uniforms_for(seeds, steps):
 
     from ..cache.manager import host_library
 
-    a, b = (v if hasattr(v, "__len__") else list(v) for v in (seeds, steps))
+    a = seeds if hasattr(seeds, "__len__") else list(seeds)
+    b = steps if hasattr(steps, "__len__") else list(steps)
     if len(a) != len(b):
         if len(a) != 1 and len(b) != 1:
             raise ValueError(f"{len(a)} seeds for {len(b)} steps")
