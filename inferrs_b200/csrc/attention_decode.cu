@@ -365,7 +365,7 @@ __device__ __forceinline__ void store_row(const Params& P, __nv_bfloat16* out_ro
 
 // OPTIONS: a factor, a slope and a sink per head, a cap on the scores, a sequence's first keys beside the window, a
 // gate per head.
-// RANKED is a form of its own: with both in one, either pays for what the other keeps in registers.
+// RANKED: see the head of this file; a form of its own, so that the others run through none of its instructions.
 template <bool OPTIONS, bool FEW, bool RANKED>
 __global__ void __launch_bounds__(THREADS, 2) decode_kernel(const __grid_constant__ CUtensorMap map_k,
                                                             const __grid_constant__ CUtensorMap map_v, const Params P) {
